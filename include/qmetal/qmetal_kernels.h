@@ -125,6 +125,27 @@ int qmk_pauli_expect(const float *state, uint32_t n, uint64_t flip,
                      const uint32_t *ny, double *d_out, void *workspace,
                      size_t workspace_bytes, void *stream);
 
+/* Z strings (masks of any weight inside n bits), up to 32 per call, n >= 10:
+ * d_out[t] = sum_i (-1)^popcount(i & masks[t]) |a_i|^2 in one read of the
+ * state. qmk_pauli_expect serves flip = 0 through it. */
+int qmk_z_expect(const float *state, uint32_t n, uint32_t num_terms,
+                 const uint64_t *masks, double *d_out, void *workspace,
+                 size_t workspace_bytes, void *stream);
+
+/* Single X terms on distinct wires, any of wires 0..5 and at most seven wires
+ * >= 6, n >= 10, in one read of the state: d_out[k] = <psi|X_w|psi> / 2 for
+ * w = wires[k] (each pair of amplitudes once, as qmk_pauli_expect). */
+int qmk_x_expect(const float *state, uint32_t n, uint32_t num_wires,
+                 const uint32_t *wires, double *d_out, void *workspace,
+                 size_t workspace_bytes, void *stream);
+
+/* Up to 64 Pauli strings of any flip and sign masks on a state of at most 14
+ * qubits, one block each in one launch. d_out[t] as qmk_pauli_expect gives it
+ * (half of <psi|P_t|psi> up to sign where flip is not 0). */
+int qmk_expect_small(const float *state, uint32_t n, uint32_t num_terms,
+                     const uint64_t *flips, const uint64_t *sign_masks,
+                     const uint32_t *ny, double *d_out, void *stream);
+
 /* lambda (=|+=) sum_t coeff_t * i^ny_t * P_t psi over terms sharing one flip
  * mask, up to 16 per call; coeffs real. overwrite != 0 stores instead of
  * accumulating. Replaces pauli_accum + zero_state (kernels.metal:313-327,

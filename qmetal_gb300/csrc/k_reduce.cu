@@ -74,65 +74,54 @@ struct PauliArgs {
   uint64_t sign[kMaxT];
 };
 
-// flip == 0: sum_i s_t(i) |psi_i|^2, two amplitudes per float4.
-template <int T>
+// flip != 0: over pairs (i, j = i ^ flip) with bit hbit of i clear,
+// sum s_t(i) * (Re or Im of conj(psi_i) psi_j); the host applies +-2. Two
+// pairs a vector: j's vector is v ^ (flip >> 1), its halves traded when bit 0
+// is flipped too. INV: flip is bit 0 alone, the pair is one vector's halves.
+template <int T, bool INV>
 __global__ void __launch_bounds__(kThreads)
-k_pauli_z(const float4 *__restrict__ st, uint64_t nvec, PauliArgs p, Area a, double *out) {
+k_pauli_x(const float4 *__restrict__ st, uint64_t nsites, PauliArgs p, Area a, double *out) {
   double acc[T];
 #pragma unroll
   for (int t = 0; t < T; t++) acc[t] = 0.0;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kThreads;
-  for (uint64_t v0 = static_cast<uint64_t>(blockIdx.x) * kThreads + threadIdx.x; v0 < nvec;
-       v0 += stride * kChunk) {
+  const uint64_t vflip = p.flip >> 1;
+  for (uint64_t s0 = static_cast<uint64_t>(blockIdx.x) * kThreads + threadIdx.x; s0 < nsites;
+       s0 += stride * kChunk) {
+    float4 x[kChunk], y[kChunk];
+    uint64_t v[kChunk];
+#pragma unroll
+    for (int k = 0; k < kChunk; k++) {
+      const uint64_t s = s0 + k * stride;
+      v[k] = INV ? s : ins0(s, p.hbit - 1);
+      x[k] = (s < nsites) ? st[v[k]] : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (!INV) y[k] = (s < nsites) ? st[v[k] ^ vflip] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     float part[T];
 #pragma unroll
     for (int t = 0; t < T; t++) part[t] = 0.0f;
 #pragma unroll
     for (int k = 0; k < kChunk; k++) {
-      const uint64_t v = v0 + k * stride;
-      if (v >= nvec) break;
-      const float4 x = st[v];
-      const float p0 = x.x * x.x + x.y * x.y, p1 = x.z * x.z + x.w * x.w;
-      const uint64_t i0 = 2 * v;
+      const float2 i0 = lo2(x[k]), i1 = hi2(x[k]);
+      if (INV) {
+        const float re = i0.x * i1.x + i0.y * i1.y, im = i0.x * i1.y - i0.y * i1.x;
 #pragma unroll
-      for (int t = 0; t < T; t++) {
-        const int s0 = parity64(i0 & p.sign[t]);
-        const int s1 = s0 ^ static_cast<int>(p.sign[t] & 1);
-        part[t] += (s0 ? -p0 : p0) + (s1 ? -p1 : p1);
-      }
-    }
+        for (int t = 0; t < T; t++) {
+          const float w = (p.useim >> t & 1) ? im : re;
+          part[t] += parity64((v[k] << 1) & p.sign[t]) ? -w : w;
+        }
+      } else {
+        const bool odd = p.flip & 1ull;
+        const float2 j0 = odd ? hi2(y[k]) : lo2(y[k]), j1 = odd ? lo2(y[k]) : hi2(y[k]);
+        const float re0 = i0.x * j0.x + i0.y * j0.y, im0 = i0.x * j0.y - i0.y * j0.x;
+        const float re1 = i1.x * j1.x + i1.y * j1.y, im1 = i1.x * j1.y - i1.y * j1.x;
 #pragma unroll
-    for (int t = 0; t < T; t++) acc[t] += part[t];
-  }
-  finish<T>(acc, p.nt, a, OutContig{out, false});
-}
-
-// flip != 0: over pairs (i, j = i ^ flip) with bit hbit of i clear,
-// sum s_t(i) * (Re or Im of conj(psi_i) psi_j); the host applies +-2.
-template <int T>
-__global__ void __launch_bounds__(kThreads)
-k_pauli_x(const float2 *__restrict__ st, uint64_t npairs, PauliArgs p, Area a, double *out) {
-  double acc[T];
-#pragma unroll
-  for (int t = 0; t < T; t++) acc[t] = 0.0;
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kThreads;
-  constexpr int C = 2 * kChunk;
-  for (uint64_t u0 = static_cast<uint64_t>(blockIdx.x) * kThreads + threadIdx.x; u0 < npairs;
-       u0 += stride * C) {
-    float part[T];
-#pragma unroll
-    for (int t = 0; t < T; t++) part[t] = 0.0f;
-#pragma unroll
-    for (int k = 0; k < C; k++) {
-      const uint64_t u = u0 + k * stride;
-      if (u >= npairs) break;
-      const uint64_t i = ins0(u, p.hbit), j = i ^ p.flip;
-      const float2 x = st[i], y = st[j];
-      const float re = x.x * y.x + x.y * y.y, im = x.x * y.y - x.y * y.x;
-#pragma unroll
-      for (int t = 0; t < T; t++) {
-        const float v = (p.useim >> t & 1) ? im : re;
-        part[t] += parity64(i & p.sign[t]) ? -v : v;
+        for (int t = 0; t < T; t++) {
+          const bool im = p.useim >> t & 1;
+          const float w0 = im ? im0 : re0, w1 = im ? im1 : re1;
+          const float w = (p.sign[t] & 1ull) ? w0 - w1 : w0 + w1;
+          part[t] += parity64((v[k] << 1) & p.sign[t]) ? -w : w;
+        }
       }
     }
 #pragma unroll
@@ -234,14 +223,11 @@ k_adj1q(float4 *__restrict__ psi, float4 *__restrict__ lam, uint64_t nsites, uin
 template <int T>
 void launch_pauli(const float *state, uint32_t n, const PauliArgs &p, Area a,
                   double *out, cudaStream_t s) {
-  const unsigned g = reduce_grid();
-  if (p.flip == 0) {
-    k_pauli_z<T><<<g, kThreads, 0, s>>>(reinterpret_cast<const float4 *>(state),
-                                        1ull << (n - 1), p, a, out);
-  } else {
-    k_pauli_x<T><<<g, kThreads, 0, s>>>(reinterpret_cast<const float2 *>(state),
-                                        1ull << (n - 1), p, a, out);
-  }
+  const float4 *st = reinterpret_cast<const float4 *>(state);
+  const uint64_t nsites = p.flip == 1 ? 1ull << (n - 1) : 1ull << (n - 2);
+  const unsigned g = std::min<unsigned>(reduce_grid(), grid_for(nsites, kThreads * kChunk));
+  if (p.flip == 1) k_pauli_x<T, true><<<g, kThreads, 0, s>>>(st, nsites, p, a, out);
+  else k_pauli_x<T, false><<<g, kThreads, 0, s>>>(st, nsites, p, a, out);
 }
 
 template <int T>
@@ -358,17 +344,21 @@ k_accum_local(float4 *__restrict__ lam, const float4 *__restrict__ psi, uint64_t
 extern "C" int qmk_abs2sum(const float *state, uint32_t n, double *d_out,
                            void *ws, size_t ws_bytes, void *stream) {
   if (!state || !d_out || n < 1 || n > 40 || !ok_ws(ws, ws_bytes, n)) return -1;
-  k_abs2<<<reduce_grid(), kThreads, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const float4 *>(state), 1ull << (n - 1), area_of(ws), d_out);
+  const uint64_t nvec = 1ull << (n - 1);
+  const unsigned g = std::min<unsigned>(reduce_grid(), grid_for(nvec, kThreads * kChunk));
+  k_abs2<<<g, kThreads, 0, (cudaStream_t)stream>>>(reinterpret_cast<const float4 *>(state), nvec,
+                                                   area_of(ws), d_out);
   return launch_status();
 }
 
 extern "C" int qmk_dot_re(const float *x, const float *y, uint32_t n, double *d_out,
                           void *ws, size_t ws_bytes, void *stream) {
   if (!x || !y || !d_out || n < 1 || n > 40 || !ok_ws(ws, ws_bytes, n)) return -1;
-  k_dot_re<<<reduce_grid(), kThreads, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const float4 *>(x), reinterpret_cast<const float4 *>(y),
-      1ull << (n - 1), area_of(ws), d_out);
+  const uint64_t nvec = 1ull << (n - 1);
+  const unsigned g = std::min<unsigned>(reduce_grid(), grid_for(nvec, kThreads * kChunk));
+  k_dot_re<<<g, kThreads, 0, (cudaStream_t)stream>>>(reinterpret_cast<const float4 *>(x),
+                                                     reinterpret_cast<const float4 *>(y), nvec,
+                                                     area_of(ws), d_out);
   return launch_status();
 }
 
@@ -380,9 +370,18 @@ extern "C" int qmk_pauli_expect(const float *state, uint32_t n, uint64_t flip,
       !ok_ws(ws, ws_bytes, n))
     return -1;
   if (n < 64 && (flip >> n)) return -1;
+  if (reinterpret_cast<uintptr_t>(state) & 15u) return -1;
+  if (flip == 0) {
+    const uint64_t none[kMaxT] = {};
+    const uint32_t even[kMaxT] = {};
+    uint64_t masks[kMaxT];
+    for (uint32_t t = 0; t < nt; t++) masks[t] = signs[t] & ((1ull << n) - 1);
+    return n >= 10 ? qmk_z_expect(state, n, nt, masks, d_out, ws, ws_bytes, stream)
+                   : qmk_expect_small(state, n, nt, none, masks, even, d_out, stream);
+  }
   PauliArgs p{};
   p.flip = flip;
-  p.hbit = flip ? 63 - __builtin_clzll(flip) : 0;
+  p.hbit = 63 - __builtin_clzll(flip);
   p.nt = nt;
   for (uint32_t t = 0; t < nt; t++) {
     p.sign[t] = signs[t];

@@ -26,6 +26,9 @@ namespace {
 constexpr size_t kResultSlots = 4096;
 constexpr uint32_t kMaxGroup = 5;    // wires per register-group launch
 constexpr uint32_t kTermsPerPass = 16;
+constexpr uint32_t kSmallExpect = 14;    // widest state whose strings go a block each
+constexpr size_t kSmallTerms = 64;       // strings per such launch
+constexpr size_t kZTermsPerPass = 32;
 
 cudaStream_t S(void *p) { return static_cast<cudaStream_t>(p); }
 
@@ -758,10 +761,13 @@ double Simulator::abs2sum() {
 
 double Simulator::norm() { return std::sqrt(abs2sum()); }
 
-// <P_t> for every term, grouped so terms that share a flip mask share a pass.
+// <P_t> for every term, in as few reads of the state as its strings allow.
+// Up to kSmallExpect qubits every string is a block of one launch (the state
+// is in cache and a launch costs more than a read). Above, Z strings go up to
+// 32 a read, single X terms up to seven wires >= 6 with wires 0..5 a read, and
+// other strings that share a flip mask up to 16 a read.
 void Simulator::pauli_values(const float *st, const Hamiltonian &h, std::vector<double> &vals) {
   vals.assign(h.terms.size(), 0.0);
-  const auto groups = group_by_flip(h);
   struct Slot { size_t term; size_t slot; };
   std::vector<Slot> pending;
   size_t used = 0;
@@ -779,17 +785,91 @@ void Simulator::pauli_values(const float *st, const Hamiltonian &h, std::vector<
     pending.clear();
     used = 0;
   };
-  for (const FlipGroup &g : groups) {
+  // Room for `count` more results.
+  auto room = [&](size_t count) {
+    if (used + count > kResultSlots) drain();
+  };
+  if (n_ <= kSmallExpect) {
+    for (size_t b = 0; b < h.terms.size(); b += kSmallTerms) {
+      const size_t take = std::min(kSmallTerms, h.terms.size() - b);
+      room(take);
+      uint64_t flips[kSmallTerms], signs[kSmallTerms];
+      uint32_t nys[kSmallTerms];
+      for (size_t j = 0; j < take; j++) {
+        const PauliString &p = h.terms[b + j].pauli;
+        flips[j] = p.x_mask | p.y_mask;
+        signs[j] = p.y_mask | p.z_mask;
+        nys[j] = popc(p.y_mask);
+        pending.push_back({b + j, used + j});
+      }
+      check(qmk_expect_small(st, n_, static_cast<uint32_t>(take), flips, signs, nys,
+                             d_results_ + used, stream_),
+            "expectation");
+      dispatches_++;
+      used += take;
+    }
+    drain();
+    return;
+  }
+  std::vector<size_t> zs;                     // Z strings
+  std::map<uint32_t, std::vector<size_t>> xs; // single X terms by wire
+  Hamiltonian rest;
+  std::vector<size_t> rest_of;
+  for (size_t t = 0; t < h.terms.size(); t++) {
+    const PauliString &p = h.terms[t].pauli;
+    if (!(p.x_mask | p.y_mask)) {
+      zs.push_back(t);
+    } else if (!p.y_mask && !p.z_mask && popc(p.x_mask) == 1) {
+      xs[static_cast<uint32_t>(__builtin_ctzll(p.x_mask))].push_back(t);
+    } else {
+      rest.terms.push_back(h.terms[t]);
+      rest_of.push_back(t);
+    }
+  }
+  for (size_t b = 0; b < zs.size(); b += kZTermsPerPass) {
+    const size_t take = std::min(kZTermsPerPass, zs.size() - b);
+    room(take);
+    uint64_t masks[kZTermsPerPass];
+    for (size_t j = 0; j < take; j++) {
+      masks[j] = h.terms[zs[b + j]].pauli.z_mask;
+      pending.push_back({zs[b + j], used + j});
+    }
+    check(qmk_z_expect(st, n_, static_cast<uint32_t>(take), masks, d_results_ + used, ws_,
+                       ws_bytes_, stream_),
+          "expectation");
+    dispatches_++;
+    used += take;
+  }
+  // Wires 0..5 go with the last pass; wires >= 6 evenly over their passes.
+  std::vector<uint32_t> low, high;
+  for (const auto &kv : xs) (kv.first < 6 ? low : high).push_back(kv.first);
+  const size_t passes = std::max<size_t>((high.size() + 6) / 7, low.empty() ? 0 : 1);
+  for (size_t k = 0, at = 0; k < passes; k++) {
+    std::vector<uint32_t> wires;
+    const size_t left = passes - k, take = (high.size() - at + left - 1) / left;
+    wires.insert(wires.end(), high.begin() + at, high.begin() + at + take);
+    at += take;
+    if (left == 1) wires.insert(wires.end(), low.begin(), low.end());
+    room(wires.size());
+    for (size_t j = 0; j < wires.size(); j++)
+      for (size_t t : xs[wires[j]]) pending.push_back({t, used + j});
+    check(qmk_x_expect(st, n_, static_cast<uint32_t>(wires.size()), wires.data(),
+                       d_results_ + used, ws_, ws_bytes_, stream_),
+          "expectation");
+    dispatches_++;
+    used += wires.size();
+  }
+  for (const FlipGroup &g : group_by_flip(rest)) {
     for (size_t b = 0; b < g.terms.size(); b += kTermsPerPass) {
       const uint32_t take = static_cast<uint32_t>(std::min<size_t>(kTermsPerPass, g.terms.size() - b));
-      if (used + take > kResultSlots) drain();
+      room(take);
       uint64_t signs[kTermsPerPass];
       uint32_t nys[kTermsPerPass];
       for (uint32_t j = 0; j < take; j++) {
-        const PauliString &p = h.terms[g.terms[b + j]].pauli;
+        const PauliString &p = rest.terms[g.terms[b + j]].pauli;
         signs[j] = p.y_mask | p.z_mask;
         nys[j] = popc(p.y_mask);
-        pending.push_back({g.terms[b + j], used + j});
+        pending.push_back({rest_of[g.terms[b + j]], used + j});
       }
       check(qmk_pauli_expect(st, n_, g.flip, take, signs, nys, d_results_ + used, ws_, ws_bytes_,
                              stream_),
