@@ -36,6 +36,10 @@ int qmk_apply_1q(float *state, uint32_t n, uint32_t q, const float m[8],
 int qmk_apply_phase(float *state, uint32_t n, uint64_t mask, float re,
                     float im, void *stream);
 
+/* The same with the factor in FP64, applied as FP32 high and low parts. */
+int qmk_apply_phase64(float *state, uint32_t n, uint64_t mask, double re,
+                      double im, void *stream);
+
 /* k commuting 2x2s on distinct ascending wires in one pass: wire 0 pairs the
  * lanes of each vector, wires 1..5 exchange with partner lanes by warp
  * shuffle, wires >= 6 pair registers. One launch takes wire 0 plus up to five

@@ -439,7 +439,7 @@ extern "C" int qmk_zdiag_costate(float *lam, const float *psi, uint32_t n, uint3
   uint8_t *base = static_cast<uint8_t *>(ws);
   DiagDesc *dd = reinterpret_cast<DiagDesc *>(base);
   float *table = reinterpret_cast<float *>(base + kDescBytes);
-  k_quad_prep<false><<<grid_for(1u << d.W, kThreads), kThreads, 0, s>>>(d, dd, table);
+  k_quad_prep<false><<<grid_for(1u << d.W, kPrepThreads), kPrepThreads, 0, s>>>(d, dd, table);
   int rc = launch_status();
   if (rc) return rc;
   const uint64_t ntiles = 1ull << (n - d.W);
@@ -469,7 +469,7 @@ extern "C" int qmk_adjoint_diagonal(float *psi, float *lam, uint32_t n, uint32_t
   DiagDesc *dd = reinterpret_cast<DiagDesc *>(base);
   float2 *table = reinterpret_cast<float2 *>(base + kDescBytes);
   if (undo) {
-    k_quad_prep<true><<<grid_for(1u << d.W, kThreads), kThreads, 0, s>>>(d, dd, table);
+    k_quad_prep<true><<<grid_for(1u << d.W, kPrepThreads), kPrepThreads, 0, s>>>(d, dd, table);
     int rc = launch_status();
     if (rc) return rc;
   } else {

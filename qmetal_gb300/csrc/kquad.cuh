@@ -92,15 +92,18 @@ inline int build_quad_desc(uint32_t n, uint32_t nt, const uint64_t *masks, const
 }
 
 // Copy the descriptor into the workspace and tabulate f_L over the 2^W low
-// indices: e^{i f_L} (PHASE) as float2, or f_L itself as float.
+// indices: e^{i f_L} (PHASE) as float2, or f_L itself as float. Bound by its
+// FP64 sums and sincos at this part's FP64 rate (a warp instruction holds a
+// multiprocessor's FP64 unit for 16 cycles), so its blocks are two warps: the
+// 2^13 entries then spread over 128 multiprocessors instead of 32.
+constexpr unsigned kPrepThreads = 64;
+
 template <bool PHASE>
 __global__ void k_quad_prep(const DiagDesc d, DiagDesc *__restrict__ out, void *__restrict__ table) {
-  if (blockIdx.x == 0) {
-    const uint64_t *src = reinterpret_cast<const uint64_t *>(&d);
-    uint64_t *dst = reinterpret_cast<uint64_t *>(out);
-    for (uint32_t k = threadIdx.x; k < sizeof(DiagDesc) / 8; k += blockDim.x) dst[k] = src[k];
-  }
   const uint32_t lo = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t *src = reinterpret_cast<const uint64_t *>(&d);
+  uint64_t *dst = reinterpret_cast<uint64_t *>(out);
+  for (uint32_t k = lo; k < sizeof(DiagDesc) / 8; k += gridDim.x * blockDim.x) dst[k] = src[k];
   if (lo >= (1u << d.W)) return;
   double f = 0.0;
   for (uint32_t r = 0; r < d.W; r++)

@@ -346,7 +346,8 @@ void Simulator::apply_gate_to(float *st, const Gate &g) {
     float f[8];
     narrow(m, f);
     if (unit_diag(f))
-      check(qmk_apply_phase(st, n_, 1ull << g.qubits[0], f[6], f[7], stream_), "apply");
+      check(qmk_apply_phase64(st, n_, 1ull << g.qubits[0], m[3].real(), m[3].imag(), stream_),
+            "apply");
     else
       check(qmk_apply_1q(st, n_, g.qubits[0], f, stream_), "apply");
     dispatches_++;
@@ -369,8 +370,7 @@ void Simulator::apply_gate_to(float *st, const Gate &g) {
       case G_CZ:
       case G_CP: {
         const cdouble ph = g.kind == G_CZ ? cdouble(-1, 0) : std::polar(1.0, g.params[0]);
-        check(qmk_apply_phase(st, n_, (1ull << a) | (1ull << b), float(ph.real()),
-                              float(ph.imag()), stream_),
+        check(qmk_apply_phase64(st, n_, (1ull << a) | (1ull << b), ph.real(), ph.imag(), stream_),
               "apply");
         dispatches_++;
         return;
@@ -581,7 +581,9 @@ void Simulator::apply_op_to(float *st, const PlanOp &op) {
       float f[8];
       narrow(op.matrix, f);
       if (unit_diag(f))
-        check(qmk_apply_phase(st, n_, 1ull << op.qubits[0], f[6], f[7], stream_), "dense1q");
+        check(qmk_apply_phase64(st, n_, 1ull << op.qubits[0], op.matrix[3].real(),
+                                op.matrix[3].imag(), stream_),
+              "dense1q");
       else
         check(qmk_apply_1q(st, n_, op.qubits[0], f, stream_), "dense1q");
       dispatches_++;
@@ -643,7 +645,9 @@ void Simulator::apply_op_to(float *st, const PlanOp &op) {
       check(qmk_apply_diagonal(st, n_, static_cast<uint32_t>(nt), op.masks.data(),
                                op.angles.data(), op.global_phase, ws_, ws_bytes_, stream_),
             "diagonal layer");
-      dispatches_ += 2 + (wide + 63) / 64;
+      // one term is a masked phase, one launch
+      const bool phase = nt == 1 && op.global_phase == 0.0 && op.masks[0] && popc(op.masks[0]) <= 3;
+      dispatches_ += phase ? 1 : 2 + (wide + 63) / 64;
       return;
     }
     case PlanOp::Kind::Swap: {
