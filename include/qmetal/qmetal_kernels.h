@@ -57,6 +57,17 @@ int qmk_apply_blocked(float *state, uint32_t n, uint32_t block_bits,
                       uint32_t count, const uint32_t *qubits,
                       const float *matrices, void *stream);
 
+/* One in-place pass, n >= 13: one 2x2 per wire of `qubits` (distinct, any
+ * order; k may be 0), then CX and SWAP gates, three words each: 0 for
+ * CX(a, b) or 1 for SWAP(a, b), then a and b. The pass holds the 2x2s' and the
+ * gates' wires: any of wires 0..5 with up to four wires >= 6, or up to seven
+ * wires >= 6. Serves apply_1q and apply_controlled_1q / apply_swap dispatches
+ * (simulator.mm:453-547). Returns -1 for any other wires without launching. */
+int qmk_apply_group_moves(float *state, uint32_t n, uint32_t k,
+                          const uint32_t *qubits, const float *mats,
+                          uint32_t num_moves, const uint32_t *moves,
+                          void *stream);
+
 /* 2x2 on `target` where every control bit is set; 1 or 2 controls (CX, CY,
  * CCX). Replaces apply_controlled_1q (kernels.metal:148-163;
  * simulator.mm:526-537) and apply_ccx (kernels.metal:392-408). */

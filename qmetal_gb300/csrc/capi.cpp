@@ -401,7 +401,8 @@ size_t qm_schedule_export(qm_circuit c, const qm_hamiltonian *h, int which, uint
       case 0: serialise_schedule(merged_schedule(build_plan(c->c, FusionOptions{})), n, v); break;
       case 1: serialise_schedule(backward_schedule(c->c, tile_high), n, v); break;
       case 2: serialise_schedule(costate_schedule(hamiltonian_of(h), n), v); break;
-      default: throw std::runtime_error("schedule: which must be 0, 1 or 2");
+      case 3: serialise_schedule(inplace_schedule(build_plan(c->c, FusionOptions{})), n, v); break;
+      default: throw std::runtime_error("schedule: which must be 0, 1, 2 or 3");
     }
     if (out && cap) std::memcpy(out, v.data(), sizeof(double) * std::min(cap, v.size()));
     return v.size();

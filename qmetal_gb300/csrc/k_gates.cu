@@ -282,8 +282,14 @@ k_group5_pair(float4 *__restrict__ st, uint64_t nsites, GroupArgs g) {
 // the last WB wires run in registers too. One shared-memory round trip per
 // site instead of a pair exchange per wire; every load and store is a
 // 512-byte warp row.
+//
+// CX and SWAP gates among the wires may follow: a linear map of a site's row
+// number, carried by the store addresses, so the pass takes no longer.
 struct BlkGroupArgs {
   uint32_t pos[7];   // the wires' vector bits (wire - 1), ascending, all >= 5
+  uint32_t act;      // bit j: wire j of the site has a 2x2
+  uint32_t moved;    // rows move after the 2x2s:
+  uint8_t img[7];    //   the image of each row bit
   M2 m[7];
   M2 m0;             // wire 0 when W0
 };
@@ -328,7 +334,14 @@ k_group_blk(float4 *__restrict__ st, uint64_t nsites, BlkGroupArgs g) {
   __shared__ uint64_t row_off[kThreads / 32][2][NV];
   {
     const int l = lane & (NV - 1);
-    const uint32_t row = lane < NV ? row_a(l) : row_b(l);
+    uint32_t row = lane < NV ? row_a(l) : row_b(l);
+    if (lane >= NV && g.moved) {
+      uint32_t to = 0;
+#pragma unroll
+      for (int j = 0; j < KB; j++)
+        if ((row >> j) & 1u) to ^= g.img[j];
+      row = to;
+    }
     uint64_t v = 0;
 #pragma unroll
     for (int j = 0; j < KB; j++)
@@ -362,7 +375,9 @@ k_group_blk(float4 *__restrict__ st, uint64_t nsites, BlkGroupArgs g) {
     }
     cp_async_commit();
   };
-  auto reg_wire = [&](float4 (&r)[NV], int j, const M2 &m) {
+  auto reg_wire = [&](float4 (&r)[NV], int j, int wire) {
+    if (!((g.act >> wire) & 1u)) return;
+    const M2 &m = g.m[wire];
 #pragma unroll
     for (int l = 0; l < NV; l++) {
       if ((l >> j) & 1) continue;
@@ -392,7 +407,7 @@ k_group_blk(float4 *__restrict__ st, uint64_t nsites, BlkGroupArgs g) {
         }
       }
 #pragma unroll
-      for (int j = 0; j < 4; j++) reg_wire(r, j, g.m[j]);
+      for (int j = 0; j < 4; j++) reg_wire(r, j, j);
 #pragma unroll
       for (int l = 0; l < NV; l++) site[row_a(l) * 32 + lane] = r[l];
     }
@@ -405,7 +420,7 @@ k_group_blk(float4 *__restrict__ st, uint64_t nsites, BlkGroupArgs g) {
     prefetch(rd + 1);
     if (active) {
 #pragma unroll
-      for (int j = 0; j < WB; j++) reg_wire(r, j, g.m[4 + j]);
+      for (int j = 0; j < WB; j++) reg_wire(r, j, 4 + j);
       const uint64_t base = base_of(sidx);
 #pragma unroll
       for (int l = 0; l < NV; l++) st[base | row_off[warp][1][l]] = r[l];
@@ -503,6 +518,90 @@ k_group_warp(float4 *__restrict__ st, uint64_t nwsites, WarpGroupArgs g) {
       st[v] = join2(r[u][l]);
     }
   }
+}
+
+// The warp tile of wires 0..5 and four wires >= 6, with CX and SWAP gates
+// among them after the 2x2s: a linear map of the tile's ten index bits. Each
+// warp scatters its 1024 amplitudes by that map into 8 KiB of shared memory of
+// its own and reads them back in order, so the stores stay whole rows and no
+// block barrier is needed.
+struct WarpMovesArgs {
+  uint32_t lact, hact;   // bit j: wire j / the j-th wire >= 6 has a 2x2
+  uint32_t hpos[4];      // site-number bits (wire - 6), ascending
+  M2 lm[6];
+  MX hm[4];
+  uint16_t img[10];      // the image of each index bit: wires 0..5, then the four
+};
+
+template <int CLS>
+__global__ void __launch_bounds__(kThreads, 2)
+k_group_moves(float4 *__restrict__ st, uint64_t nwsites, WarpMovesArgs g) {
+  constexpr int NV = 16;
+  extern __shared__ __align__(16) float4 xw[];   // [warp][NV][32 lanes]
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t ws = (static_cast<uint64_t>(blockIdx.x) * kThreads + threadIdx.x) >> 5;
+  if (ws >= nwsites) return;   // uniform over the warp, and no block barrier follows
+  uint64_t b = ws;
+#pragma unroll
+  for (int j = 0; j < 4; j++) b = ins0(b, g.hpos[j]);
+  const uint64_t base = (b << 5) | lane;
+  auto vec_of = [&](int l) {
+    uint64_t v = base;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if ((l >> j) & 1) v |= 1ull << (g.hpos[j] + 5);
+    return v;
+  };
+  Cx2 r[NV];
+#pragma unroll
+  for (int l = 0; l < NV; l++) r[l] = split2(st[vec_of(l)]);
+  if (g.lact & 1u) {
+#pragma unroll
+    for (int l = 0; l < NV; l++) apply_w0x<CLS>(g.lm[0], r[l]);
+  }
+#pragma unroll
+  for (int q = 1; q < 6; q++) {
+    if (!((g.lact >> q) & 1u)) continue;
+    const bool one = (lane >> (q - 1)) & 1;
+    const M2 m = g.lm[q];
+    // own' = s own + t other: (a, b) on the wire's 0 side, (d, c) on its 1 side
+    const float2 cs = one ? m.d : m.a, ct = one ? m.c : m.b;
+#pragma unroll
+    for (int l = 0; l < NV; l++) {
+      const Cx2 mine = r[l];
+      Cx2 other;
+      other.re.x = __shfl_xor_sync(0xffffffffu, mine.re.x, 1 << (q - 1));
+      other.re.y = __shfl_xor_sync(0xffffffffu, mine.re.y, 1 << (q - 1));
+      other.im.x = __shfl_xor_sync(0xffffffffu, mine.im.x, 1 << (q - 1));
+      other.im.y = __shfl_xor_sync(0xffffffffu, mine.im.y, 1 << (q - 1));
+      r[l] = cmacx<CLS>(cs, mine, ct, other);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    if (!((g.hact >> j) & 1u)) continue;
+#pragma unroll
+    for (int l = 0; l < NV; l++)
+      if (!((l >> j) & 1)) applyx<CLS>(g.hm[j], r[l], r[l | (1 << j)]);
+  }
+  float4 *mine = xw + (threadIdx.x >> 5) * NV * 32;
+  float2 *amp = reinterpret_cast<float2 *>(mine);
+  uint32_t at = 0;
+#pragma unroll
+  for (int k = 0; k < 5; k++)
+    if ((lane >> k) & 1u) at ^= g.img[1 + k];
+#pragma unroll
+  for (int l = 0; l < NV; l++) {
+    uint32_t to = at;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if ((l >> j) & 1) to ^= g.img[6 + j];
+    amp[to] = make_float2(r[l].re.x, r[l].im.x);
+    amp[to ^ g.img[0]] = make_float2(r[l].re.y, r[l].im.y);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int l = 0; l < NV; l++) st[vec_of(l)] = mine[l * 32 + lane];
 }
 
 constexpr int kMaxBlockedGates = 96;
@@ -946,6 +1045,7 @@ extern "C" int qmk_apply_group(float *state, uint32_t n, uint32_t k,
           bg.m0 = m;
         } else {
           bg.pos[kb] = qubits[j] - 1;
+          bg.act |= 1u << kb;
           bg.m[kb] = m;
           kb++;
         }
@@ -997,6 +1097,109 @@ extern "C" int qmk_apply_group(float *state, uint32_t n, uint32_t k,
     default: return -1;
   }
   return launch_status();
+}
+
+template <int CLS>
+static int launch_group_moves(float4 *st, uint64_t nw, const WarpMovesArgs &g, cudaStream_t s) {
+  constexpr size_t smem = static_cast<size_t>(kThreads / 32) * 16 * 32 * sizeof(float4);
+  static std::atomic<bool> opted[64];   // zero-initialised: false
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
+  if (!opted[dev]) {   // the opt-in above 48 KiB is per device
+    const cudaError_t e = cudaFuncSetAttribute(
+        k_group_moves<CLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return static_cast<int>(e);
+    opted[dev] = true;
+  }
+  k_group_moves<CLS><<<grid_for(nw, kThreads / 32), kThreads, smem, s>>>(st, nw, g);
+  return launch_status();
+}
+
+extern "C" int qmk_apply_group_moves(float *state, uint32_t n, uint32_t k, const uint32_t *qubits,
+                                     const float *mats, uint32_t num_moves, const uint32_t *moves,
+                                     void *stream) {
+  if (!valid_state(state, n) || n < 13 || (k && (!qubits || !mats)) || !num_moves || !moves)
+    return -1;
+  uint64_t held = 0, tile = 0;
+  for (uint32_t j = 0; j < k; j++) {
+    if (qubits[j] >= n || ((held >> qubits[j]) & 1ull)) return -1;
+    held |= 1ull << qubits[j];
+  }
+  tile = held;
+  for (uint32_t j = 0; j < num_moves; j++) {
+    const uint32_t a = moves[3 * j + 1], b = moves[3 * j + 2];
+    if (moves[3 * j] > 1 || a >= n || b >= n || a == b) return -1;
+    tile |= (1ull << a) | (1ull << b);
+  }
+  const bool low = (tile & 63ull) != 0;
+  uint64_t high = tile & ~63ull;
+  const uint32_t nh = static_cast<uint32_t>(__builtin_popcountll(high));
+  if (nh > (low ? 4u : 7u)) return -1;
+  // Fill up with the lowest free wires >= 6.
+  const uint32_t fill = low ? 4u : nh > 6 ? 7u : 6u;
+  for (uint32_t w = 6; static_cast<uint32_t>(__builtin_popcountll(high)) < fill; w++)
+    high |= 1ull << w;
+  // Each wire's bit of the site index: wires 0..5 of a warp tile, then the high ones.
+  uint32_t bit_of[40], pos[7], at = 0;
+  for (uint32_t w = 0; w < 6; w++) bit_of[w] = w;
+  for (uint32_t w = 6; w < n; w++) {
+    if (!((high >> w) & 1ull)) continue;
+    pos[at] = w;
+    bit_of[w] = (low ? 6 : 0) + at++;
+  }
+  uint16_t img[10];
+  for (uint32_t j = 0; j < (low ? 10u : fill); j++) {
+    uint32_t x = 1u << j;
+    for (uint32_t m = 0; m < num_moves; m++) {
+      const uint32_t a = bit_of[moves[3 * m + 1]], b = bit_of[moves[3 * m + 2]];
+      if (moves[3 * m]) {
+        const uint32_t d = ((x >> a) ^ (x >> b)) & 1u;
+        x ^= (d << a) | (d << b);
+      } else {
+        x ^= ((x >> a) & 1u) << b;
+      }
+    }
+    img[j] = static_cast<uint16_t>(x);
+  }
+  std::vector<M2> all;
+  for (uint32_t j = 0; j < k; j++) all.push_back(m2_from(mats + 8 * j));
+  const int cls = k ? common_class(all.data(), static_cast<int>(k)) : kMatReal;
+  float4 *st = reinterpret_cast<float4 *>(state);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (low) {
+    WarpMovesArgs g{};
+    for (uint32_t j = 0; j < 4; j++) g.hpos[j] = pos[j] - 6;
+    for (uint32_t j = 0; j < k; j++) {
+      const uint32_t b = bit_of[qubits[j]];
+      if (b < 6) {
+        g.lact |= 1u << b;
+        g.lm[b] = all[j];
+      } else {
+        g.hact |= 1u << (b - 6);
+        g.hm[b - 6] = mx_from(all[j]);
+      }
+    }
+    std::copy(img, img + 10, g.img);
+    const uint64_t nw = 1ull << (n - 10);
+    switch (cls) {
+      case kMatRx: return launch_group_moves<kMatRx>(st, nw, g, s);
+      case kMatReal: return launch_group_moves<kMatReal>(st, nw, g, s);
+      default: return launch_group_moves<kMatGeneral>(st, nw, g, s);
+    }
+  }
+  BlkGroupArgs g{};
+  for (uint32_t j = 0; j < fill; j++) {
+    g.pos[j] = pos[j] - 1;
+    g.img[j] = static_cast<uint8_t>(img[j]);
+  }
+  g.moved = 1;
+  for (uint32_t j = 0; j < k; j++) {
+    g.act |= 1u << bit_of[qubits[j]];
+    g.m[bit_of[qubits[j]]] = all[j];
+  }
+  const uint64_t nsites = 1ull << (n - 6 - fill);
+  return fill == 6 ? launch_group_blk<2, false>(st, nsites, g, cls, s)
+                   : launch_group_blk<3, false>(st, nsites, g, cls, s);
 }
 
 extern "C" int qmk_apply_blocked(float *state, uint32_t n, uint32_t b,

@@ -122,88 +122,122 @@ int generator_of(const Gate &g) {
 
 // ---------------------------------------------------------------------------
 
+namespace {
+
+// Wires 0..5 (wire 0 apart), and wires >= 6, that one group pass may hold.
+bool group_fits(uint32_t n, bool zero, size_t lane, size_t high) {
+  (void)zero;
+  if (lane >= 1 && high <= 4 && n >= 6 + high) return true;
+  if (lane == 0 && high >= 6 && high <= 7 && n >= 6 + high) return true;   // block groups
+  return lane + high <= 5;
+}
+
+// Most wires >= 6 one pass of such wires alone may hold.
+uint32_t high_cap(uint32_t n) { return n >= 13 ? 7 : n >= 12 ? 6 : 5; }
+
+// One-wire ops on distinct wires, not yet issued.
+struct WireRun {
+  std::vector<uint32_t> wires;
+  std::vector<cdouble> mats;
+  bool holds(uint32_t q) const { return std::find(wires.begin(), wires.end(), q) != wires.end(); }
+  void add(uint32_t q, const cdouble *m) {
+    wires.push_back(q);
+    mats.insert(mats.end(), m, m + 4);
+  }
+  void clear() {
+    wires.clear();
+    mats.clear();
+  }
+};
+
+// The run's ops (they all commute) as the fewest group passes: wires 0..5
+// take k wires >= 6 along, the rest go up to seven a pass in order. Where a
+// lane wire's matrix is general, the pass of the lane wires is bound by its
+// multiply-adds: of the k that give the fewest passes the least is kept, but
+// at least one where there is one (a pass of the lane wires alone has too
+// little work per thread to hide its loads), so an HEA layer at 28 qubits
+// goes as 6 + 1, 7, 7, 7 wires instead of 6 + 4, 7, 7, 4. Narrow matrices
+// (real, RX-like, diagonal) halve the lane pass's multiply-adds: it then
+// keeps as many wires >= 6 as fit. Returns each pass's entries of the run.
+std::vector<std::vector<size_t>> split_run(uint32_t n, const WireRun &run) {
+  std::vector<size_t> low, high;
+  for (size_t i = 0; i < run.wires.size(); i++) (run.wires[i] < 6 ? low : high).push_back(i);
+  size_t lane = 0;
+  bool zero = false, general = false;
+  for (size_t i : low) {
+    if (run.wires[i] == 0) zero = true;
+    else lane++;
+    general = general || narrowed_class(&run.mats[4 * i]) == 0;
+  }
+  const size_t cap = high_cap(n);
+  size_t best_k = 0, best = SIZE_MAX;
+  for (size_t k = low.empty() ? 0 : std::min<size_t>(1, high.size()); k <= high.size(); k++) {
+    const bool some = !low.empty() || k > 0;
+    if (some && !group_fits(n, zero, lane, k)) break;
+    const size_t passes = (some ? 1 : 0) + (high.size() - k + cap - 1) / cap;
+    if (passes < best || (!general && passes == best)) {
+      best = passes;
+      best_k = k;
+    }
+  }
+  std::vector<std::vector<size_t>> out;
+  std::vector<size_t> first = low;
+  first.insert(first.end(), high.begin(), high.begin() + best_k);
+  if (!first.empty()) out.push_back(std::move(first));
+  for (size_t j = best_k; j < high.size(); j += cap)
+    out.emplace_back(high.begin() + j, high.begin() + std::min(high.size(), j + cap));
+  for (auto &pass : out)
+    std::sort(pass.begin(), pass.end(),
+              [&](size_t a, size_t b) { return run.wires[a] < run.wires[b]; });
+  return out;
+}
+
+ForwardStep group_step(const WireRun &run, const std::vector<size_t> &idx) {
+  ForwardStep s;
+  s.kind = ForwardStep::Group;
+  for (size_t i : idx) s.wires.push_back(run.wires[i]);
+  s.mats.reserve(4 * idx.size());
+  for (size_t i : idx)
+    s.mats.insert(s.mats.end(), run.mats.begin() + 4 * i, run.mats.begin() + 4 * i + 4);
+  return s;
+}
+
+// A plan op that only moves amplitudes between two wires.
+bool is_wire_move(const PlanOp &op, uint32_t n) {
+  const bool cx = op.kind == PlanOp::Kind::Controlled1q && op.matrix[0] == 0.0 &&
+                  op.matrix[1] == 1.0 && op.matrix[2] == 1.0 && op.matrix[3] == 0.0;
+  return (cx || op.kind == PlanOp::Kind::Swap) && op.qubits[0] < n && op.qubits[1] < n &&
+         op.qubits[0] != op.qubits[1];
+}
+
+// The wires and matrices of a one-qubit plan op; false for any other op.
+bool one_wire_op(const PlanOp &op, uint32_t n, const uint32_t *&wires, const cdouble *&mats,
+                 size_t &count) {
+  if (op.kind == PlanOp::Kind::Dense1q) {
+    wires = op.qubits;
+    mats = op.matrix;
+    count = 1;
+  } else if (op.kind == PlanOp::Kind::Dense1qGroup) {
+    wires = op.group_qubits.data();
+    mats = op.group_matrices.data();
+    count = op.group_qubits.size();
+  } else {
+    return false;
+  }
+  for (size_t j = 0; j < count; j++)
+    if (wires[j] >= n) throw std::runtime_error("qubit index out of range");
+  return true;
+}
+
+}  // namespace
+
 std::vector<ForwardStep> merged_schedule(const Plan &p) {
   const uint32_t n = p.num_qubits;
   std::vector<ForwardStep> out;
-  std::vector<uint32_t> wires;
-  std::vector<cdouble> mats;
-  auto fits = [&](const std::vector<uint32_t> &w) {
-    uint32_t lane = 0, high = 0, zero = 0;
-    for (uint32_t q : w) {
-      if (q == 0) zero++;
-      else if (q <= 5) lane++;
-      else high++;
-    }
-    if (zero > 1) return false;
-    if (lane >= 1 && lane <= 5 && high <= 4 && n >= 6 + high) return true;
-    if (lane == 0 && high >= 6 && high <= 7 && n >= 6 + high) return true;   // block groups
-    return lane + high <= 5;
-  };
-  // One pass for the given entries of the pending run, wires ascending.
-  auto emit = [&](std::vector<size_t> idx) {
-    if (idx.empty()) return;
-    std::sort(idx.begin(), idx.end(), [&](size_t a, size_t b) { return wires[a] < wires[b]; });
-    ForwardStep s;
-    s.kind = ForwardStep::Group;
-    for (size_t i : idx) {
-      s.wires.push_back(wires[i]);
-      s.mats.insert(s.mats.end(), mats.begin() + 4 * i, mats.begin() + 4 * i + 4);
-    }
-    out.push_back(std::move(s));
-  };
-  // A run of one-wire ops on distinct wires (they all commute) in the fewest
-  // passes: wires 0..5 take k wires >= 6 along, the rest go up to seven a
-  // pass in order. Where a lane wire's matrix is general, the pass of the
-  // lane wires is bound by its multiply-adds: of the k that give the fewest
-  // passes the least is kept, but at least one where there is one (a pass of
-  // the lane wires alone has too little work per thread to hide its loads),
-  // so an HEA layer at 28 qubits goes as 6 + 1, 7, 7, 7 wires instead of
-  // 6 + 4, 7, 7, 4. Otherwise the greatest is kept.
+  WireRun held;
   auto flush = [&]() {
-    if (wires.empty()) return;
-    std::vector<size_t> low, high;
-    for (size_t i = 0; i < wires.size(); i++) (wires[i] < 6 ? low : high).push_back(i);
-    auto wires_of = [&](const std::vector<size_t> &idx) {
-      std::vector<uint32_t> w;
-      for (size_t i : idx) w.push_back(wires[i]);
-      return w;
-    };
-    // Wires >= 6 in passes of their own, greedily in order.
-    auto chunks = [&](size_t from) {
-      std::vector<std::vector<size_t>> c;
-      for (size_t j = from; j < high.size(); j++) {
-        if (c.empty()) {
-          c.push_back({high[j]});
-          continue;
-        }
-        std::vector<uint32_t> trial = wires_of(c.back());
-        trial.push_back(wires[high[j]]);
-        if (fits(trial)) c.back().push_back(high[j]);
-        else c.push_back({high[j]});
-      }
-      return c;
-    };
-    // Narrow matrices (real, RX-like, diagonal) halve the lane pass's
-    // multiply-adds: it then keeps as many wires >= 6 as fit.
-    bool general = false;
-    for (size_t i : low) general = general || narrowed_class(&mats[4 * i]) == 0;
-    size_t best_k = 0, best = SIZE_MAX;
-    for (size_t k = low.empty() ? 0 : std::min<size_t>(1, high.size()); k <= high.size(); k++) {
-      std::vector<size_t> first = low;
-      first.insert(first.end(), high.begin(), high.begin() + k);
-      if (!first.empty() && !fits(wires_of(first))) break;
-      const size_t passes = (first.empty() ? 0 : 1) + chunks(k).size();
-      if (passes < best || (!general && passes == best)) {
-        best = passes;
-        best_k = k;
-      }
-    }
-    std::vector<size_t> first = low;
-    first.insert(first.end(), high.begin(), high.begin() + best_k);
-    emit(first);
-    for (const auto &c : chunks(best_k)) emit(c);
-    wires.clear();
-    mats.clear();
+    for (const auto &pass : split_run(n, held)) out.push_back(group_step(held, pass));
+    held.clear();
   };
   std::vector<PermGate> run;
   std::vector<size_t> run_ops;
@@ -229,46 +263,152 @@ std::vector<ForwardStep> merged_schedule(const Plan &p) {
   };
   for (size_t i = 0; i < p.ops.size(); i++) {
     const PlanOp &op = p.ops[i];
-    const bool cx = op.kind == PlanOp::Kind::Controlled1q && op.matrix[0] == 0.0 &&
-                    op.matrix[1] == 1.0 && op.matrix[2] == 1.0 && op.matrix[3] == 0.0;
-    if ((cx || op.kind == PlanOp::Kind::Swap) && op.qubits[0] < n && op.qubits[1] < n &&
-        op.qubits[0] != op.qubits[1]) {
+    if (is_wire_move(op, n)) {
       flush();
       run.push_back({op.kind == PlanOp::Kind::Swap, op.qubits[0], op.qubits[1]});
       run_ops.push_back(i);
       continue;
     }
     flush_run();
-    std::vector<uint32_t> w;
-    std::vector<cdouble> m;
-    if (op.kind == PlanOp::Kind::Dense1q) {
-      w.push_back(op.qubits[0]);
-      m.assign(op.matrix, op.matrix + 4);
-    } else if (op.kind == PlanOp::Kind::Dense1qGroup) {
-      w = op.group_qubits;
-      m = op.group_matrices;
-    } else {
+    const uint32_t *w = nullptr;
+    const cdouble *m = nullptr;
+    size_t count = 0;
+    if (!one_wire_op(op, n, w, m, count)) {
       flush();
       ForwardStep s;
       s.ops = {i};
       out.push_back(std::move(s));
       continue;
     }
-    for (uint32_t q : w)
-      if (q >= n) throw std::runtime_error("qubit index out of range");
     bool overlap = false;
-    for (uint32_t q : w)
-      if (std::find(wires.begin(), wires.end(), q) != wires.end()) overlap = true;
+    for (size_t j = 0; j < count; j++) overlap = overlap || held.holds(w[j]);
     if (overlap) flush();
     // The group's wires commute with each other and with the pending ones:
     // they join the pending run, which is split into passes when it ends.
-    for (size_t j = 0; j < w.size(); j++) {
-      wires.push_back(w[j]);
-      mats.insert(mats.end(), m.begin() + 4 * j, m.begin() + 4 * j + 4);
-    }
+    for (size_t j = 0; j < count; j++) held.add(w[j], m + 4 * j);
   }
   flush();
   flush_run();
+  return out;
+}
+
+// ---------------------------------------------------------------------------
+
+namespace {
+
+// One way to issue a pending run of one-wire ops and the CX / SWAP gates that
+// follow it: passes of at most `cap` wires >= 6 each (at most four beside
+// wires 0..5), every pass with the gates, in order, that it holds both wires
+// of and that no gate left for later has a wire of.
+std::vector<ForwardStep> move_passes(const WireRun &held, const std::vector<PermGate> &run,
+                                     const std::vector<size_t> &run_ops, uint32_t cap) {
+  std::vector<ForwardStep> out;
+  std::vector<bool> gate_done(run.size(), false), wire_done(held.wires.size(), false);
+  size_t left = run.size() + held.wires.size();
+  while (left) {
+    uint64_t tile = 0, blocked = 0;
+    uint32_t high = 0;
+    bool low = false;
+    auto admit = [&](uint64_t wires) {
+      uint32_t add = 0;
+      bool lo = low;
+      for (uint64_t m = wires & ~tile; m; m &= m - 1) {
+        if (__builtin_ctzll(m) < 6) lo = true;
+        else add++;
+      }
+      if (high + add > (lo ? std::min(cap, 4u) : cap)) return false;
+      tile |= wires;
+      high += add;
+      low = lo;
+      return true;
+    };
+    ForwardStep s;
+    s.kind = ForwardStep::Moves;
+    for (size_t k = 0; k < run.size(); k++) {
+      if (gate_done[k]) continue;
+      const uint64_t w = (1ull << run[k].a) | (1ull << run[k].b);
+      if ((w & blocked) || !admit(w)) {
+        blocked |= w;
+        continue;
+      }
+      s.moves.push_back(run[k]);
+      s.ops.push_back(run_ops[k]);
+      gate_done[k] = true;
+      left--;
+    }
+    std::vector<size_t> idx;
+    for (size_t i = 0; i < held.wires.size(); i++) {
+      if (wire_done[i] || !admit(1ull << held.wires[i])) continue;
+      wire_done[i] = true;
+      idx.push_back(i);
+      left--;
+    }
+    std::sort(idx.begin(), idx.end(),
+              [&](size_t a, size_t b) { return held.wires[a] < held.wires[b]; });
+    ForwardStep g = group_step(held, idx);
+    s.wires = std::move(g.wires);
+    s.mats = std::move(g.mats);
+    if (s.moves.empty()) s.kind = ForwardStep::Group;
+    out.push_back(std::move(s));
+  }
+  return out;
+}
+
+}  // namespace
+
+std::vector<ForwardStep> inplace_schedule(const Plan &p) {
+  const uint32_t n = p.num_qubits;
+  std::vector<ForwardStep> out;
+  WireRun held;
+  std::vector<PermGate> run;
+  std::vector<size_t> run_ops;
+  auto flush = [&]() {
+    const auto groups = split_run(n, held);
+    std::vector<ForwardStep> best;
+    if (!run.empty() && n >= kMovesMinQubits) {
+      for (uint32_t cap = 4; cap <= 7; cap++) {
+        std::vector<ForwardStep> t = move_passes(held, run, run_ops, cap);
+        if (best.empty() || t.size() < best.size()) best = std::move(t);
+      }
+    }
+    // A pass reads and writes the state (2 S); a CX or SWAP of its own moves S.
+    if (!best.empty() && 2 * best.size() <= 2 * groups.size() + run.size()) {
+      for (ForwardStep &s : best) out.push_back(std::move(s));
+    } else {
+      for (const auto &pass : groups) out.push_back(group_step(held, pass));
+      for (size_t i : run_ops) {
+        ForwardStep s;
+        s.ops = {i};
+        out.push_back(std::move(s));
+      }
+    }
+    held.clear();
+    run.clear();
+    run_ops.clear();
+  };
+  for (size_t i = 0; i < p.ops.size(); i++) {
+    const PlanOp &op = p.ops[i];
+    if (is_wire_move(op, n)) {
+      run.push_back({op.kind == PlanOp::Kind::Swap, op.qubits[0], op.qubits[1]});
+      run_ops.push_back(i);
+      continue;
+    }
+    const uint32_t *w = nullptr;
+    const cdouble *m = nullptr;
+    size_t count = 0;
+    if (!one_wire_op(op, n, w, m, count)) {
+      flush();
+      ForwardStep s;
+      s.ops = {i};
+      out.push_back(std::move(s));
+      continue;
+    }
+    bool later = !run.empty();
+    for (size_t j = 0; j < count; j++) later = later || held.holds(w[j]);
+    if (later) flush();
+    for (size_t j = 0; j < count; j++) held.add(w[j], m + 4 * j);
+  }
+  flush();
   return out;
 }
 
@@ -780,11 +920,19 @@ void serialise_schedule(const std::vector<ForwardStep> &s, uint32_t n, std::vect
   v.push_back(static_cast<double>(s.size()));
   for (const ForwardStep &st : s) {
     v.push_back(st.kind);
-    if (st.kind == ForwardStep::Group) {
+    if (st.kind == ForwardStep::Group || st.kind == ForwardStep::Moves) {
       v.push_back(static_cast<double>(st.wires.size()));
       for (size_t i = 0; i < st.wires.size(); i++) {
         v.push_back(st.wires[i]);
         put_mat(v, &st.mats[4 * i]);
+      }
+      if (st.kind == ForwardStep::Moves) {
+        v.push_back(static_cast<double>(st.moves.size()));
+        for (const PermGate &m : st.moves) {
+          v.push_back(m.swap ? 1.0 : 0.0);
+          v.push_back(m.a);
+          v.push_back(m.b);
+        }
       }
     } else if (st.kind == ForwardStep::Permute) {
       put_map(v, n, st.cols, st.off);

@@ -44,14 +44,16 @@ bool permutation_pays(const Affine &m, size_t gates);
 // --- merged forward --------------------------------------------------------
 
 struct ForwardStep {
-  enum Kind : uint8_t { Group, Permute, Op };
+  enum Kind : uint8_t { Group, Permute, Op, Moves };
   Kind kind = Op;
-  std::vector<uint32_t> wires;   // Group: ascending, distinct
-  std::vector<cdouble> mats;     // Group: one row-major 2x2 per wire
+  std::vector<uint32_t> wires;   // Group / Moves: ascending, distinct
+  std::vector<cdouble> mats;     // Group / Moves: one row-major 2x2 per wire
+  std::vector<PermGate> moves;   // Moves: CX / SWAP gates after the 2x2s, in order
   std::vector<uint64_t> cols;    // Permute: gather map
   uint64_t off = 0;
   // Op: the one plan op to apply. Permute: the run's plan ops, applied one
-  // by one when there is no room for the gather's second buffer.
+  // by one when there is no room for the gather's second buffer. Moves: the
+  // plan ops of `moves`.
   std::vector<size_t> ops;
 };
 
@@ -61,6 +63,16 @@ struct ForwardStep {
 // turned into one gather pass where that moves fewer bytes. Every other op
 // passes through. Same unitary as the plan.
 std::vector<ForwardStep> merged_schedule(const Plan &p);
+
+// The plan without a second buffer: its one-qubit ops merged as above, and a
+// run of CX / SWAP ops shared out among passes that hold their wires (the
+// passes' 2x2s run first), where that moves fewer bytes than the run's gates
+// one by one. A pass with moves holds any of wires 0..5 and up to four wires
+// >= 6, or up to seven wires >= 6; it needs kMovesMinQubits. An HEA layer of
+// 30 wires and its ladder go as five passes (10 S) instead of eight groups
+// and 29 CX (45 S): three layers and the 60 terms of their Hamiltonian 187 -> 57 ms.
+constexpr uint32_t kMovesMinQubits = 13;
+std::vector<ForwardStep> inplace_schedule(const Plan &p);
 
 // --- co-state lambda = H psi and the energy ---------------------------------
 
@@ -149,6 +161,7 @@ int generator_of(const Gate &g);
 //     0 (Group)   nw, (wire, m00.re, m00.im, m01.re, m01.im, m10.., m11..) x nw
 //     1 (Permute) n, cols[n], off, nops, ops[nops]
 //     2 (Op)      op
+//     3 (Moves)   nw, (wire, m00.re, ..) x nw, ngates, (swap, a, b) x ngates
 //   co-state: [steps] then per step
 //     0 (ZDiag)   nt, (zmask, coeff) x nt
 //     1 (Local)   overwrite, nt, (wire, sign, ny, coeff) x nt

@@ -398,7 +398,52 @@ void Simulator::apply_gate_to(float *st, const Gate &g) {
   throw std::runtime_error(std::string("unsupported gate: ") + gate_name(g.kind));
 }
 
-void Simulator::run(const Circuit &c) { run(c, FusionOptions{}); }
+// The default plan through inplace_schedule(): its passes merged further, in
+// the state's own buffer. Explicit options and plans run op for op.
+void Simulator::run(const Circuit &c) {
+  if (c.num_qubits != n_) throw std::runtime_error("circuit/simulator size mismatch");
+  activate();
+  run_inplace(build_plan(c, FusionOptions{}));
+}
+
+void Simulator::run_inplace(const Plan &p) {
+  for (const ForwardStep &st : inplace_schedule(p)) {
+    if (st.kind == ForwardStep::Op) apply_op_to(state_, p.ops[st.ops[0]]);
+    else apply_group_step(st);
+  }
+}
+
+// One 2x2 per wire, then the step's moves, in one launch.
+void Simulator::apply_group_step(const ForwardStep &st) {
+  const uint32_t k = static_cast<uint32_t>(st.wires.size());
+  if (k == 1 && st.moves.empty()) {
+    apply_dense_1q(state_, st.wires[0], st.mats.data());
+    return;
+  }
+  std::vector<float> fm(8 * k);
+  for (uint32_t i = 0; i < k; i++) narrow(&st.mats[4 * i], &fm[8 * i]);
+  if (st.moves.empty()) {
+    check(qmk_apply_group(state_, n_, k, st.wires.data(), fm.data(), stream_), "merged group");
+  } else {
+    std::vector<uint32_t> moves;
+    for (const PermGate &m : st.moves) moves.insert(moves.end(), {m.swap ? 1u : 0u, m.a, m.b});
+    check(qmk_apply_group_moves(state_, n_, k, st.wires.data(), fm.data(),
+                                static_cast<uint32_t>(st.moves.size()), moves.data(), stream_),
+          "merged group");
+  }
+  dispatches_++;
+}
+
+void Simulator::apply_dense_1q(float *st, uint32_t q, const cdouble *m) {
+  if (q >= n_) throw std::runtime_error("qubit index out of range");
+  float f[8];
+  narrow(m, f);
+  if (unit_diag(f))
+    check(qmk_apply_phase64(st, n_, 1ull << q, m[3].real(), m[3].imag(), stream_), "dense1q");
+  else
+    check(qmk_apply_1q(st, n_, q, f, stream_), "dense1q");
+  dispatches_++;
+}
 
 void Simulator::run(const Circuit &c, const FusionOptions &opts) {
   if (c.num_qubits != n_) throw std::runtime_error("circuit/simulator size mismatch");
@@ -463,7 +508,7 @@ void Simulator::run_cached(const Circuit &c) {
   cuda_check(cudaStreamBeginCapture(S(stream_), cudaStreamCaptureModeThreadLocal), "graph capture");
   cudaGraph_t graph = nullptr;
   try {
-    for (const PlanOp &op : plan.ops) apply_op_to(state_, op);
+    run_inplace(plan);
   } catch (...) {
     cudaStreamEndCapture(S(stream_), &graph);
     if (graph) cudaGraphDestroy(graph);
@@ -492,15 +537,10 @@ void Simulator::run_merged(const Plan &p) {
   activate();
   for (const ForwardStep &st : merged_schedule(p)) {
     switch (st.kind) {
-      case ForwardStep::Group: {
-        std::vector<float> fm(2 * st.mats.size());
-        for (size_t i = 0; i < st.wires.size(); i++) narrow(&st.mats[4 * i], &fm[8 * i]);
-        check(qmk_apply_group(state_, n_, static_cast<uint32_t>(st.wires.size()), st.wires.data(),
-                              fm.data(), stream_),
-              "merged group");
-        dispatches_++;
+      case ForwardStep::Group:
+      case ForwardStep::Moves:
+        apply_group_step(st);
         break;
-      }
       case ForwardStep::Permute: {
         if (keep_ckpts_ && ensure_scratch()) {
           if (float *dst = take_buffer()) {
@@ -576,19 +616,9 @@ void Simulator::run_profiled(const Plan &p, std::vector<double> &seconds) {
 
 void Simulator::apply_op_to(float *st, const PlanOp &op) {
   switch (op.kind) {
-    case PlanOp::Kind::Dense1q: {
-      if (op.qubits[0] >= n_) throw std::runtime_error("qubit index out of range");
-      float f[8];
-      narrow(op.matrix, f);
-      if (unit_diag(f))
-        check(qmk_apply_phase64(st, n_, 1ull << op.qubits[0], op.matrix[3].real(),
-                                op.matrix[3].imag(), stream_),
-              "dense1q");
-      else
-        check(qmk_apply_1q(st, n_, op.qubits[0], f, stream_), "dense1q");
-      dispatches_++;
+    case PlanOp::Kind::Dense1q:
+      apply_dense_1q(st, op.qubits[0], op.matrix);
       return;
-    }
     case PlanOp::Kind::Dense1qGroup: {
       const size_t k = op.group_qubits.size();
       if (k < 2) throw std::runtime_error("group size must be at least 2");

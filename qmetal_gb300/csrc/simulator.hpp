@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "circuit.hpp"
+#include "schedule.hpp"
 
 namespace qmetal {
 
@@ -27,6 +28,8 @@ class Simulator {
 
   void reset();
   void apply(const Gate &g);
+  // The default plan, its passes merged further in place; with options, and
+  // for a plan, one launch group per plan op.
   void run(const Circuit &c);
   void run(const Circuit &c, const FusionOptions &opts);
   void run(const Plan &p);
@@ -118,6 +121,9 @@ class Simulator {
   void activate() const;
   void apply_gate_to(float *state, const Gate &g);
   void apply_op_to(float *state, const PlanOp &op);
+  void apply_dense_1q(float *state, uint32_t q, const cdouble *m);
+  void apply_group_step(const ForwardStep &st);
+  void run_inplace(const Plan &p);
   void pauli_values(const float *state, const Hamiltonian &h, std::vector<double> &vals);
   void costate(const Hamiltonian &h);
   void prepare_adjoint(const Circuit &c, const Hamiltonian &h);

@@ -1,0 +1,96 @@
+"""The in-place schedule of Simulator.run, replayed in complex128 on the CPU
+against the oracle's gate-by-gate run, with the limits its kernels rely on: a
+pass with moves holds any of wires 0..5 and up to four wires >= 6, or up to
+seven wires >= 6, and exists from 13 qubits."""
+import numpy as np
+import pytest
+
+import oracle
+import qmetal_gb300 as qm  # noqa: F401
+from qmetal_gb300 import workloads as W
+from test_schedules import Reader, apply_1q, plan_op
+
+CX, CZ, SWAP, CP = W.CX, W.CZ, W.SWAP, W.CP
+
+
+def _steps(c):
+    v = c.schedule_export("inplace")
+    r, out = Reader(v), []
+    for _ in range(r.i()):
+        kind = r.i()
+        assert kind in (0, 2, 3)
+        if kind == 2:
+            out.append(("op", r.i()))
+            continue
+        mats = [(r.i(), r.mat()) for _ in range(r.i())]
+        moves = [(r.i(), r.i(), r.i()) for _ in range(r.i())] if kind == 3 else []
+        out.append(("moves" if kind == 3 else "group", mats, moves))
+    assert r.p == len(v)
+    return out
+
+
+def _move(st, swap, a, b):
+    i = np.arange(st.size)
+    d = ((i >> a) ^ (i >> b)) & 1 if swap else (i >> a) & 1
+    out = np.empty_like(st)
+    out[i ^ (d << b) ^ ((d << a) if swap else 0)] = st
+    return out
+
+
+def _replay(n, gates):
+    c = W.to_circuit(n, gates)
+    plan = np.array(c.plan_export())
+    st = np.zeros(1 << n, dtype=complex)
+    st[0] = 1.0
+    steps = _steps(c)
+    for s in steps:
+        if s[0] == "op":
+            st = oracle.run_plan(n, plan_op(plan, s[1]), init=st)
+            continue
+        wires = [w for w, _ in s[1]]
+        assert wires == sorted(set(wires))
+        for w, m in s[1]:
+            st = apply_1q(st, n, w, m)
+        if s[0] == "moves":
+            assert n >= 13 and s[2]
+            held = set(wires) | {q for _, a, b in s[2] for q in (a, b)}
+            assert sum(q >= 6 for q in held) <= (4 if min(held) < 6 else 7)
+            for swap, a, b in s[2]:
+                assert a != b
+                st = _move(st, swap, a, b)
+    return st, steps
+
+
+def _random(n, count, rng):
+    gates = []
+    for _ in range(count):
+        a, b = (int(q) for q in rng.choice(n, 2, replace=False))
+        kind = int(rng.choice([CX, CX, CX, SWAP, CZ, CP, W.RY, W.RZ, W.H]))
+        if kind == CP:
+            gates.append((kind, (a, b), (0.4,)))
+        elif kind in (CX, SWAP, CZ):
+            gates.append((kind, (a, b), ()))
+        else:
+            gates.append((kind, (a,), (0.7,) if kind in (W.RY, W.RZ) else ()))
+    return gates
+
+
+@pytest.mark.parametrize("n", [5, 11, 12, 13, 14])
+def test_inplace_schedule(n):
+    rng = np.random.default_rng(40 + n)
+    reverse = [(CX, (q + 1, q), ()) for q in reversed(range(n - 1))]
+    swaps = [(SWAP, (q, n - 1 - q), ()) for q in range(n // 2)]
+    layer = [(W.RY, (q,), (0.1 + q,)) for q in range(n)]
+    for gates in (W.ghz(n), W.hea(n, 2), W.qft_swap(n), W.tfim_chain(n, 2), W.random_u3(n, 2),
+                  W.qaoa_ring_seeded(n, 2), layer + reverse + layer + swaps, layer + swaps + reverse,
+                  _random(n, 60, rng), _random(n, 60, rng)):
+        got, _ = _replay(n, gates)
+        assert np.abs(got - oracle.run(n, gates)).max() <= 1e-12
+
+
+@pytest.mark.parametrize("n, passes", [(28, 4), (30, 5), (13, 2)])
+def test_hea_layer_passes(n, passes):
+    steps = _steps(W.to_circuit(n, W.hea(n, 1)))
+    assert len(steps) == passes
+    assert sum(len(s[2]) for s in steps) == n - 1
+    assert sorted(w for s in steps for w, _ in s[1]) == list(range(n))
