@@ -85,7 +85,9 @@ int qm_synchronize(qm_simulator s);
 
 uint32_t qm_num_qubits(qm_simulator s);
 uint64_t qm_dim(qm_simulator s);
-uint64_t qm_dispatch_count(qm_simulator s);       /* kernels launched */
+/* Kernels launched; up to 13 qubits, where qm_run and its variants run a
+ * circuit's plan in one launch, the plan's ops count as one each. */
+uint64_t qm_dispatch_count(qm_simulator s);
 
 /* View of the interleaved state, 2 * qm_dim() floats, valid until the next
  * mutation. Here the state lives in device memory; the returned pointer is a
@@ -166,7 +168,9 @@ size_t qm_circuit_plan_export(qm_circuit c, int collapse_1q_windows,
  *   which = 1: the block-wise backward sweep (qm_energy_and_gradient) with
  *              `tile_high` wires >= 6 per window pass (1..6);
  *   which = 2: the co-state lambda = H psi of `h` for the circuit's width;
- *   which = 3: the default plan as qm_run launches it, in place.
+ *   which = 3: the default plan as qm_run launches it, in place;
+ *   which = 4: the default plan as one launch runs it, up to 13 qubits (its
+ *              groups hold up to three wires).
  * Forward steps: 0 group (nw, then wire and a row-major 2x2 as re/im pairs per
  * wire), 1 gather (n, cols[n], off, nops, plan op indices), 2 plan op (index),
  * 3 group with CX / SWAP gates after it (nw and its matrices as 0, then ngates

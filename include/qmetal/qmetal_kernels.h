@@ -108,6 +108,46 @@ int qmk_apply_diagonal(float *state, uint32_t n, uint32_t num_terms,
                        double global_phase, void *workspace,
                        size_t workspace_bytes, void *stream);
 
+/* A whole circuit on a state of up to QMK_SMALL_MAX_QUBITS qubits, in one
+ * launch (more where the ops outgrow a launch's arguments), the ops in order:
+ *   GROUP       2x2s on `count` (1..3) ascending wires q; mats, 8 floats each
+ *   PHASE       amplitudes with every bit of `mask` set times phase (re, im)
+ *   CONTROLLED  2x2 `mats` on wire q[0] where every bit of `mask` is set
+ *   MAP         amplitude y from XOR of cols[j] over y's bits (n entries, an
+ *               invertible map: a run of CX / SWAP gates)
+ *   LAYER       a diagonal layer (masks of any weight), as qmk_apply_diagonal
+ * Bad arguments return -1 before anything is launched. The workspace (of at
+ * least qmk_small_workspace_bytes(n)) holds the layers' phase tables. Serves
+ * the reference's dispatches gate by gate (kernels.metal:48-218, 392-408). */
+#define QMK_SMALL_MAX_QUBITS 13
+#define QMK_SMALL_MAX_TERMS 3000   /* per layer */
+enum {
+  QMK_SMALL_GROUP = 0,
+  QMK_SMALL_PHASE = 1,
+  QMK_SMALL_CONTROLLED = 2,
+  QMK_SMALL_MAP = 3,
+  QMK_SMALL_LAYER = 4
+};
+typedef struct {
+  uint32_t num_terms;
+  const uint64_t *masks;
+  const double *angles;
+  double global_phase;
+} qmk_phase_layer;
+typedef struct {
+  uint32_t kind, count;
+  uint32_t q[3];
+  const float *mats;
+  uint64_t mask;
+  double phase[2];
+  const uint64_t *cols;
+  qmk_phase_layer layer;
+} qmk_small_op;
+size_t qmk_small_workspace_bytes(uint32_t n);
+int qmk_run_small(float *state, uint32_t n, size_t num_ops,
+                  const qmk_small_op *ops, void *workspace,
+                  size_t workspace_bytes, void *stream);
+
 /* Returned when a size exceeds a fixed capacity (nothing is launched). */
 #define QMK_ERR_TOO_LARGE (-2)
 

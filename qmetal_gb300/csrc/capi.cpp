@@ -402,7 +402,8 @@ size_t qm_schedule_export(qm_circuit c, const qm_hamiltonian *h, int which, uint
       case 1: serialise_schedule(backward_schedule(c->c, tile_high), n, v); break;
       case 2: serialise_schedule(costate_schedule(hamiltonian_of(h), n), v); break;
       case 3: serialise_schedule(inplace_schedule(build_plan(c->c, FusionOptions{})), n, v); break;
-      default: throw std::runtime_error("schedule: which must be 0, 1, 2 or 3");
+      case 4: serialise_schedule(small_schedule(build_plan(c->c, FusionOptions{})), n, v); break;
+      default: throw std::runtime_error("schedule: which must be 0..4");
     }
     if (out && cap) std::memcpy(out, v.data(), sizeof(double) * std::min(cap, v.size()));
     return v.size();

@@ -414,6 +414,55 @@ std::vector<ForwardStep> inplace_schedule(const Plan &p) {
 
 // ---------------------------------------------------------------------------
 
+std::vector<ForwardStep> small_schedule(const Plan &p) {
+  const uint32_t n = p.num_qubits;
+  std::vector<ForwardStep> out;
+  WireRun held;
+  std::vector<PermGate> run;
+  auto flush = [&]() {
+    std::vector<size_t> idx(held.wires.size());
+    for (size_t i = 0; i < idx.size(); i++) idx[i] = i;
+    std::sort(idx.begin(), idx.end(),
+              [&](size_t a, size_t b) { return held.wires[a] < held.wires[b]; });
+    for (size_t b = 0; b < idx.size(); b += 3)
+      out.push_back(group_step(held, {idx.begin() + b, idx.begin() + std::min(idx.size(), b + 3)}));
+    held.clear();
+    if (run.empty()) return;
+    const Affine map = run_map(n, run, false);
+    ForwardStep s;
+    s.kind = ForwardStep::Permute;
+    s.cols = map.cols;
+    s.off = map.off;
+    out.push_back(std::move(s));
+    run.clear();
+  };
+  for (size_t i = 0; i < p.ops.size(); i++) {
+    const PlanOp &op = p.ops[i];
+    if (is_wire_move(op, n)) {
+      run.push_back({op.kind == PlanOp::Kind::Swap, op.qubits[0], op.qubits[1]});
+      continue;
+    }
+    const uint32_t *w = nullptr;
+    const cdouble *m = nullptr;
+    size_t count = 0;
+    if (!one_wire_op(op, n, w, m, count)) {
+      flush();
+      ForwardStep s;
+      s.ops = {i};
+      out.push_back(std::move(s));
+      continue;
+    }
+    bool later = !run.empty();
+    for (size_t j = 0; j < count; j++) later = later || held.holds(w[j]);
+    if (later) flush();
+    for (size_t j = 0; j < count; j++) held.add(w[j], m + 4 * j);
+  }
+  flush();
+  return out;
+}
+
+// ---------------------------------------------------------------------------
+
 namespace {
 
 struct FlipGroup {

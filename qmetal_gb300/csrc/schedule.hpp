@@ -74,6 +74,10 @@ std::vector<ForwardStep> merged_schedule(const Plan &p);
 constexpr uint32_t kMovesMinQubits = 13;
 std::vector<ForwardStep> inplace_schedule(const Plan &p);
 
+// The plan for a state that one block holds: one-qubit ops three wires a
+// step, every run of CX / SWAP ops as one gather, other ops as they are.
+std::vector<ForwardStep> small_schedule(const Plan &p);
+
 // --- co-state lambda = H psi and the energy ---------------------------------
 
 struct CostateStep {

@@ -119,6 +119,7 @@ Simulator::Simulator(uint32_t n) : n_(n) {
   cuda_check(cudaGetDevice(&device_), "cudaGetDevice");
   const uint64_t bytes = (uint64_t(1) << n) * 8ull;
   ws_bytes_ = qmk_workspace_bytes(n);
+  small_ws_bytes_ = qmk_small_workspace_bytes(n);   // behind ws_
   size_t free_b = 0, total_b = 0;
   cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
   if (bytes + ws_bytes_ > free_b)
@@ -129,7 +130,8 @@ Simulator::Simulator(uint32_t n) : n_(n) {
   stream_ = s;
   try {
     cuda_check(cudaMalloc(&state_, bytes), "Simulator: state allocation failed");
-    cuda_check(cudaMalloc(&ws_, ws_bytes_), "Simulator: workspace allocation failed");
+    cuda_check(cudaMalloc(&ws_, ws_bytes_ + small_ws_bytes_),
+               "Simulator: workspace allocation failed");
     cuda_check(cudaMalloc(&d_results_, kResultSlots * sizeof(double)), "cudaMalloc results");
     cuda_check(cudaMallocHost(&h_results_, (kResultSlots + 1) * sizeof(double)), "cudaMallocHost");
     h_waits_ = reinterpret_cast<unsigned *>(h_results_ + kResultSlots);
@@ -407,6 +409,10 @@ void Simulator::run(const Circuit &c) {
 }
 
 void Simulator::run_inplace(const Plan &p) {
+  if (small()) {
+    run_small(p);
+    return;
+  }
   for (const ForwardStep &st : inplace_schedule(p)) {
     if (st.kind == ForwardStep::Op) apply_op_to(state_, p.ops[st.ops[0]]);
     else apply_group_step(st);
@@ -434,6 +440,106 @@ void Simulator::apply_group_step(const ForwardStep &st) {
   dispatches_++;
 }
 
+// The plan on a narrow state, its ops in one launch. A dispatch is counted for
+// each plan op. An op the launch cannot take (malformed, or a layer of too
+// many terms) runs, or is refused, by itself in its place.
+void Simulator::run_small(const Plan &p) {
+  std::vector<qmk_small_op> ops;
+  std::vector<std::vector<float>> mats;
+  const auto steps = small_schedule(p);
+  mats.reserve(steps.size() + p.ops.size() * 2);   // ops point into it
+  uint64_t before = 0;
+  auto launch = [&]() {
+    if (!ops.empty())
+      check(qmk_run_small(state_, n_, ops.size(), ops.data(),
+                          static_cast<uint8_t *>(ws_) + ws_bytes_, small_ws_bytes_, stream_),
+            "circuit");
+    ops.clear();
+  };
+  auto matrices = [&](const cdouble *m, size_t count) {
+    mats.emplace_back(8 * count);
+    for (size_t j = 0; j < count; j++) narrow(m + 4 * j, mats.back().data() + 8 * j);
+    return mats.back().data();
+  };
+  auto phase = [&](uint64_t mask, double re, double im) {
+    qmk_small_op o{};
+    o.kind = QMK_SMALL_PHASE;
+    o.mask = mask;
+    o.phase[0] = re;
+    o.phase[1] = im;
+    ops.push_back(o);
+  };
+  auto controlled = [&](uint64_t ctrl, uint32_t q, const cdouble *m) {
+    qmk_small_op o{};
+    o.kind = QMK_SMALL_CONTROLLED;
+    o.mask = ctrl;
+    o.q[0] = q;
+    o.mats = matrices(m, 1);
+    ops.push_back(o);
+  };
+  // False where the op goes its own way.
+  auto plan_op = [&](const PlanOp &op) {
+    const uint32_t *q = op.qubits;
+    if (op.kind == PlanOp::Kind::Controlled1q) {
+      if (q[0] >= n_ || q[1] >= n_ || q[0] == q[1]) return false;
+      controlled(1ull << q[0], q[1], op.matrix);
+    } else if (op.kind == PlanOp::Kind::CCX) {
+      if (q[0] >= n_ || q[1] >= n_ || q[2] >= n_ || q[0] == q[1] || q[0] == q[2] || q[1] == q[2])
+        return false;
+      cdouble x[4];
+      gate_matrix_1q(G_X, nullptr, x);
+      controlled((1ull << q[0]) | (1ull << q[1]), q[2], x);
+    } else if (op.kind == PlanOp::Kind::DiagonalLayer) {
+      const size_t nt = op.masks.size();
+      if (op.angles.size() != nt || nt > QMK_SMALL_MAX_TERMS) return false;
+      for (uint64_t m : op.masks)
+        if (m >> n_) return false;
+      if (nt == 0) return true;
+      if (nt == 1 && op.global_phase == 0.0 && op.masks[0] && popc(op.masks[0]) <= 3) {
+        phase(op.masks[0], std::cos(op.angles[0]), std::sin(op.angles[0]));
+        return true;
+      }
+      qmk_small_op o{};
+      o.kind = QMK_SMALL_LAYER;
+      o.layer = {static_cast<uint32_t>(nt), op.masks.data(), op.angles.data(), op.global_phase};
+      ops.push_back(o);
+    } else {
+      return false;
+    }
+    return true;
+  };
+  for (const ForwardStep &st : steps) {
+    qmk_small_op o{};
+    if (st.kind == ForwardStep::Group) {
+      if (st.wires.size() == 1) {
+        float f[8];
+        narrow(st.mats.data(), f);
+        if (unit_diag(f)) {
+          phase(1ull << st.wires[0], st.mats[3].real(), st.mats[3].imag());
+          continue;
+        }
+      }
+      o.kind = QMK_SMALL_GROUP;
+      o.count = static_cast<uint32_t>(st.wires.size());
+      std::copy(st.wires.begin(), st.wires.end(), o.q);
+      o.mats = matrices(st.mats.data(), st.wires.size());
+      ops.push_back(o);
+    } else if (st.kind == ForwardStep::Permute) {
+      o.kind = QMK_SMALL_MAP;
+      o.cols = st.cols.data();
+      ops.push_back(o);
+    } else if (!plan_op(p.ops[st.ops[0]])) {
+      launch();
+      const uint64_t own = dispatches_;
+      apply_op_to(state_, p.ops[st.ops[0]]);
+      before += dispatches_ - own - 1;   // counted with the plan's ops below
+      dispatches_ = own;
+    }
+  }
+  launch();
+  dispatches_ += p.ops.size() + before;
+}
+
 void Simulator::apply_dense_1q(float *st, uint32_t q, const cdouble *m) {
   if (q >= n_) throw std::runtime_error("qubit index out of range");
   float f[8];
@@ -453,6 +559,10 @@ void Simulator::run(const Circuit &c, const FusionOptions &opts) {
 void Simulator::run(const Plan &p) {
   if (p.num_qubits != n_) throw std::runtime_error("plan/simulator size mismatch");
   activate();
+  if (small()) {
+    run_small(p);
+    return;
+  }
   for (const PlanOp &op : p.ops) apply_op_to(state_, op);
 }
 
@@ -535,6 +645,12 @@ void Simulator::run_cached(const Circuit &c) {
 void Simulator::run_merged(const Plan &p) {
   if (p.num_qubits != n_) throw std::runtime_error("plan/simulator size mismatch");
   activate();
+  if (small() && !keep_ckpts_) {
+    const uint64_t own = dispatches_;
+    run_small(p);
+    dispatches_ = own + 1;
+    return;
+  }
   for (const ForwardStep &st : merged_schedule(p)) {
     switch (st.kind) {
       case ForwardStep::Group:

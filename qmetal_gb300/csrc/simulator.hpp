@@ -124,6 +124,9 @@ class Simulator {
   void apply_dense_1q(float *state, uint32_t q, const cdouble *m);
   void apply_group_step(const ForwardStep &st);
   void run_inplace(const Plan &p);
+  void run_small(const Plan &p);
+  // The state fits one block: circuits run in one launch.
+  bool small() const { return small_ws_bytes_ != 0; }
   void pauli_values(const float *state, const Hamiltonian &h, std::vector<double> &vals);
   void costate(const Hamiltonian &h);
   void prepare_adjoint(const Circuit &c, const Hamiltonian &h);
@@ -171,6 +174,7 @@ class Simulator {
   bool scratch_failed_ = false;
   void *ws_ = nullptr;
   size_t ws_bytes_ = 0;
+  size_t small_ws_bytes_ = 0;           // behind ws_bytes_ in ws_ (0: the state is too wide)
   void *sample_ws_ = nullptr;
   size_t sample_ws_bytes_ = 0;
   uint64_t *d_shots_ = nullptr;

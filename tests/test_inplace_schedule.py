@@ -1,14 +1,15 @@
-"""The in-place schedule of Simulator.run, replayed in complex128 on the CPU
-against the oracle's gate-by-gate run, with the limits its kernels rely on: a
-pass with moves holds any of wires 0..5 and up to four wires >= 6, or up to
-seven wires >= 6, and exists from 13 qubits."""
+"""The schedules of Simulator.run, replayed in complex128 on the CPU against
+the oracle's gate-by-gate run, with the limits their kernels rely on. In place:
+a pass with moves holds any of wires 0..5 and up to four wires >= 6, or up to
+seven wires >= 6, and exists from 13 qubits. In one launch (up to 13 qubits):
+groups of up to three ascending wires, gathers without an offset."""
 import numpy as np
 import pytest
 
 import oracle
 import qmetal_gb300 as qm  # noqa: F401
 from qmetal_gb300 import workloads as W
-from test_schedules import Reader, apply_1q, plan_op
+from test_schedules import Reader, apply_1q, decode_forward, gather, plan_op
 
 CX, CZ, SWAP, CP = W.CX, W.CZ, W.SWAP, W.CP
 
@@ -94,3 +95,31 @@ def test_hea_layer_passes(n, passes):
     assert len(steps) == passes
     assert sum(len(s[2]) for s in steps) == n - 1
     assert sorted(w for s in steps for w, _ in s[1]) == list(range(n))
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 6, 9, 13])
+def test_small_schedule(n):
+    rng = np.random.default_rng(70 + n)
+    circuits = [[(W.RY, (q,), (0.3 + q,)) for q in range(n)] * 2]
+    if n > 1:
+        circuits += [W.hea(n, 2), W.random_u3(n, 2), _random(n, 80, rng)]
+    if n > 2:
+        circuits += [W.ghz(n), W.qft_swap(n), W.qaoa_ring_seeded(n, 2),
+                     [(W.CCX, (0, 1, 2), ()), (W.CY, (2, 0), ())] * 2]
+    for gates in circuits:
+        c = W.to_circuit(n, gates)
+        plan = np.array(c.plan_export())
+        st = np.zeros(1 << n, dtype=complex)
+        st[0] = 1.0
+        for s in decode_forward(c.schedule_export("small")):
+            if s[0] == "group":
+                wires = [w for w, _ in s[1]]
+                assert wires == sorted(set(wires)) and 1 <= len(wires) <= 3
+                for w, m in s[1]:
+                    st = apply_1q(st, n, w, m)
+            elif s[0] == "permute":
+                assert s[2] == 0
+                st = gather(st, n, s[1], s[2])
+            else:
+                st = oracle.run_plan(n, plan_op(plan, s[1]), init=st)
+        assert np.abs(st - oracle.run(n, gates)).max() <= 1e-12
