@@ -115,18 +115,37 @@ int qmk_apply_diagonal(float *state, uint32_t n, uint32_t num_terms,
  *   CONTROLLED  2x2 `mats` on wire q[0] where every bit of `mask` is set
  *   MAP         amplitude y from XOR of cols[j] over y's bits (n entries, an
  *               invertible map: a run of CX / SWAP gates)
- *   LAYER       a diagonal layer (masks of any weight), as qmk_apply_diagonal
+ *   LAYER       a diagonal layer (masks of any weight), as qmk_apply_diagonal;
+ *               conj: its conjugate
+ * and with `adjoint` also
+ *   both        the op on the state and the co-state
+ *   save k      MAP: keep the state from before it as number k (from 1, up to
+ *               QMK_SMALL_MAX_SAVES); with `both`: the state comes from number
+ *               k, and only the co-state through the map
+ *   COSTATE     lambda = H psi and the energy: layer's Z strings with their
+ *               coefficients as angles, then num_items strings of (x|y, y|z, Y
+ *               count) with coefficients `mats`
+ *   WINDOW      num_items (up to QMK_SMALL_MAX_WINDOW, of which twelve with a
+ *               generator) of (index into q, generator 0..3, gradient slot),
+ *               each its gradient, then its 2x2 of `mats` on both states
+ *   DIAG_GRAD   num_items of (Z mask, gradient slot), the gradient of each
  * Bad arguments return -1 before anything is launched. The workspace (of at
- * least qmk_small_workspace_bytes(n)) holds the layers' phase tables. Serves
- * the reference's dispatches gate by gate (kernels.metal:48-218, 392-408). */
+ * least qmk_small_workspace_bytes(n)) holds the layers' phase tables and the
+ * kept states. Serves the reference's dispatches gate by gate
+ * (kernels.metal:48-218, 313-408). */
 #define QMK_SMALL_MAX_QUBITS 13
-#define QMK_SMALL_MAX_TERMS 3000   /* per layer */
+#define QMK_SMALL_MAX_TERMS 3000   /* per op */
+#define QMK_SMALL_MAX_SAVES 32
+#define QMK_SMALL_MAX_WINDOW 24
 enum {
   QMK_SMALL_GROUP = 0,
   QMK_SMALL_PHASE = 1,
   QMK_SMALL_CONTROLLED = 2,
   QMK_SMALL_MAP = 3,
-  QMK_SMALL_LAYER = 4
+  QMK_SMALL_LAYER = 4,
+  QMK_SMALL_WINDOW = 5,
+  QMK_SMALL_COSTATE = 6,
+  QMK_SMALL_DIAG_GRAD = 7
 };
 typedef struct {
   uint32_t num_terms;
@@ -137,16 +156,25 @@ typedef struct {
 typedef struct {
   uint32_t kind, count;
   uint32_t q[3];
+  uint32_t both, conj, save;
   const float *mats;
   uint64_t mask;
   double phase[2];
   const uint64_t *cols;
   qmk_phase_layer layer;
+  uint32_t num_items;
+  const uint32_t *items;
 } qmk_small_op;
+typedef struct {
+  float *costate;       /* 2^n amplitudes */
+  double *grad;         /* device, num_grad slots */
+  size_t num_grad;
+  double *energy;       /* device */
+} qmk_small_adjoint;
 size_t qmk_small_workspace_bytes(uint32_t n);
 int qmk_run_small(float *state, uint32_t n, size_t num_ops,
-                  const qmk_small_op *ops, void *workspace,
-                  size_t workspace_bytes, void *stream);
+                  const qmk_small_op *ops, const qmk_small_adjoint *adjoint,
+                  void *workspace, size_t workspace_bytes, void *stream);
 
 /* Returned when a size exceeds a fixed capacity (nothing is launched). */
 #define QMK_ERR_TOO_LARGE (-2)

@@ -14,6 +14,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <deque>
 #include <map>
 #include <stdexcept>
 
@@ -440,45 +441,75 @@ void Simulator::apply_group_step(const ForwardStep &st) {
   dispatches_++;
 }
 
-// The plan on a narrow state, its ops in one launch. A dispatch is counted for
-// each plan op. An op the launch cannot take (malformed, or a layer of too
-// many terms) runs, or is refused, by itself in its place.
-void Simulator::run_small(const Plan &p) {
+namespace {
+
+// The op list of one narrow-state launch, and what its ops point to.
+class SmallProgram {
+ public:
+  explicit SmallProgram(uint32_t n) : n_(n) {}
+
   std::vector<qmk_small_op> ops;
-  std::vector<std::vector<float>> mats;
-  const auto steps = small_schedule(p);
-  mats.reserve(steps.size() + p.ops.size() * 2);   // ops point into it
-  uint64_t before = 0;
-  auto launch = [&]() {
-    if (!ops.empty())
-      check(qmk_run_small(state_, n_, ops.size(), ops.data(),
-                          static_cast<uint8_t *>(ws_) + ws_bytes_, small_ws_bytes_, stream_),
-            "circuit");
-    ops.clear();
-  };
-  auto matrices = [&](const cdouble *m, size_t count) {
-    mats.emplace_back(8 * count);
-    for (size_t j = 0; j < count; j++) narrow(m + 4 * j, mats.back().data() + 8 * j);
-    return mats.back().data();
-  };
-  auto phase = [&](uint64_t mask, double re, double im) {
-    qmk_small_op o{};
-    o.kind = QMK_SMALL_PHASE;
+
+  void clear() { ops.clear(); }
+
+  void phase(uint64_t mask, double re, double im, bool both = false) {
+    qmk_small_op &o = add(QMK_SMALL_PHASE, both);
     o.mask = mask;
     o.phase[0] = re;
     o.phase[1] = im;
-    ops.push_back(o);
-  };
-  auto controlled = [&](uint64_t ctrl, uint32_t q, const cdouble *m) {
-    qmk_small_op o{};
-    o.kind = QMK_SMALL_CONTROLLED;
+  }
+
+  // 2x2s on up to three ascending wires.
+  void group(const uint32_t *wires, uint32_t count, const cdouble *m, bool both = false) {
+    float f[8];
+    narrow(m, f);
+    if (count == 1 && unit_diag(f)) {
+      phase(1ull << wires[0], m[3].real(), m[3].imag(), both);
+      return;
+    }
+    qmk_small_op &o = add(QMK_SMALL_GROUP, both);
+    o.count = count;
+    std::copy(wires, wires + count, o.q);
+    o.mats = matrices(m, count);
+  }
+
+  void controlled(uint64_t ctrl, uint32_t q, const cdouble *m, bool both = false) {
+    qmk_small_op &o = add(QMK_SMALL_CONTROLLED, both);
     o.mask = ctrl;
     o.q[0] = q;
     o.mats = matrices(m, 1);
-    ops.push_back(o);
-  };
-  // False where the op goes its own way.
-  auto plan_op = [&](const PlanOp &op) {
+  }
+
+  void map(const std::vector<uint64_t> &cols, uint32_t save, bool both = false) {
+    maps_.push_back(cols);
+    qmk_small_op &o = add(QMK_SMALL_MAP, both);
+    o.cols = maps_.back().data();
+    o.save = save;
+  }
+
+  // A diagonal layer, or its conjugate. The terms stay the caller's.
+  void layer(const std::vector<uint64_t> &masks, const std::vector<double> &angles, double gphase,
+             bool conj = false, bool both = false) {
+    if (masks.empty() && gphase == 0.0) return;
+    if (masks.size() == 1 && gphase == 0.0 && masks[0] && popc(masks[0]) <= 3) {
+      phase(masks[0], std::cos(angles[0]), conj ? -std::sin(angles[0]) : std::sin(angles[0]), both);
+      return;
+    }
+    qmk_small_op &o = add(QMK_SMALL_LAYER, both);
+    o.conj = conj;
+    o.layer = {static_cast<uint32_t>(masks.size()), masks.data(), angles.data(), gphase};
+  }
+
+  bool layer_fits(const std::vector<uint64_t> &masks, size_t angles) const {
+    if (angles != masks.size() || masks.size() > QMK_SMALL_MAX_TERMS) return false;
+    for (uint64_t m : masks)
+      if (m >> n_) return false;
+    return true;
+  }
+
+  // A plan op that small_schedule leaves as it is; false if it is malformed
+  // or of a kind that runs by itself.
+  bool plan_op(const PlanOp &op) {
     const uint32_t *q = op.qubits;
     if (op.kind == PlanOp::Kind::Controlled1q) {
       if (q[0] >= n_ || q[1] >= n_ || q[0] == q[1]) return false;
@@ -490,54 +521,270 @@ void Simulator::run_small(const Plan &p) {
       gate_matrix_1q(G_X, nullptr, x);
       controlled((1ull << q[0]) | (1ull << q[1]), q[2], x);
     } else if (op.kind == PlanOp::Kind::DiagonalLayer) {
-      const size_t nt = op.masks.size();
-      if (op.angles.size() != nt || nt > QMK_SMALL_MAX_TERMS) return false;
-      for (uint64_t m : op.masks)
-        if (m >> n_) return false;
-      if (nt == 0) return true;
-      if (nt == 1 && op.global_phase == 0.0 && op.masks[0] && popc(op.masks[0]) <= 3) {
-        phase(op.masks[0], std::cos(op.angles[0]), std::sin(op.angles[0]));
-        return true;
-      }
-      qmk_small_op o{};
-      o.kind = QMK_SMALL_LAYER;
-      o.layer = {static_cast<uint32_t>(nt), op.masks.data(), op.angles.data(), op.global_phase};
-      ops.push_back(o);
+      if (!layer_fits(op.masks, op.angles.size())) return false;
+      if (!op.masks.empty()) layer(op.masks, op.angles, op.global_phase);
     } else {
       return false;
     }
     return true;
-  };
-  for (const ForwardStep &st : steps) {
-    qmk_small_op o{};
-    if (st.kind == ForwardStep::Group) {
-      if (st.wires.size() == 1) {
-        float f[8];
-        narrow(st.mats.data(), f);
-        if (unit_diag(f)) {
-          phase(1ull << st.wires[0], st.mats[3].real(), st.mats[3].imag());
-          continue;
-        }
+  }
+
+  // A gate on both states, other than CX and SWAP.
+  bool gate_on_both(const Gate &g) {
+    const uint32_t *q = g.qubits;
+    for (int k = 0; k < g.num_qubits; k++) {
+      if (q[k] >= n_) return false;
+      for (int j = 0; j < k; j++)
+        if (q[j] == q[k]) return false;
+    }
+    cdouble m[4];
+    if (g.num_qubits == 1) {
+      gate_matrix_1q(g.kind, g.params, m);
+      group(q, 1, m, true);
+    } else if (g.kind == G_CY) {
+      gate_matrix_1q(G_Y, nullptr, m);
+      controlled(1ull << q[0], q[1], m, true);
+    } else if (g.kind == G_CZ || g.kind == G_CP) {
+      const cdouble ph = g.kind == G_CZ ? cdouble(-1, 0) : std::polar(1.0, g.params[0]);
+      phase((1ull << q[0]) | (1ull << q[1]), ph.real(), ph.imag(), true);
+    } else if (g.kind == G_CCX) {
+      gate_matrix_1q(G_X, nullptr, m);
+      controlled((1ull << q[0]) | (1ull << q[1]), q[2], m, true);
+    } else {
+      return false;
+    }
+    return true;
+  }
+
+  // lambda = H psi and the energy: Z strings by their table, the rest one by one.
+  bool costate(const Hamiltonian &h) {
+    std::vector<uint64_t> masks;
+    std::vector<double> coeffs;
+    std::vector<uint32_t> items;
+    std::vector<float> rest;
+    for (const PauliTerm &t : h.terms) {
+      const PauliString &p = t.pauli;
+      if (p.x_mask | p.y_mask) {
+        items.insert(items.end(), {static_cast<uint32_t>(p.x_mask | p.y_mask),
+                                   static_cast<uint32_t>(p.y_mask | p.z_mask), popc(p.y_mask)});
+        rest.push_back(static_cast<float>(t.coefficient));
+      } else {
+        masks.push_back(p.z_mask);
+        coeffs.push_back(t.coefficient);
       }
-      o.kind = QMK_SMALL_GROUP;
-      o.count = static_cast<uint32_t>(st.wires.size());
-      std::copy(st.wires.begin(), st.wires.end(), o.q);
-      o.mats = matrices(st.mats.data(), st.wires.size());
-      ops.push_back(o);
+    }
+    if (masks.size() > QMK_SMALL_MAX_TERMS || rest.size() > QMK_SMALL_MAX_TERMS) return false;
+    maps_.push_back(std::move(masks));
+    angles_.push_back(std::move(coeffs));
+    words_.push_back(std::move(items));
+    floats_.push_back(std::move(rest));
+    qmk_small_op &o = add(QMK_SMALL_COSTATE, false);
+    o.layer = {static_cast<uint32_t>(maps_.back().size()), maps_.back().data(),
+               angles_.back().data(), 0.0};
+    o.num_items = static_cast<uint32_t>(floats_.back().size());
+    o.items = words_.back().data();
+    o.mats = floats_.back().data();
+    return true;
+  }
+
+  // A window tile, up to three of its wires a step.
+  void window(const std::vector<WireOp> &tile) {
+    std::map<uint32_t, std::vector<const WireOp *>> by_wire;
+    for (const WireOp &o : tile) by_wire[o.wire].push_back(&o);
+    std::vector<uint32_t> wires, items;
+    std::vector<float> mats;
+    uint32_t grads = 0;
+    auto flush = [&]() {
+      if (items.empty()) return;
+      words_.push_back(std::move(items));
+      floats_.push_back(std::move(mats));
+      items.clear();
+      mats.clear();
+      qmk_small_op &o = add(QMK_SMALL_WINDOW, false);
+      o.count = static_cast<uint32_t>(wires.size());
+      std::copy(wires.begin(), wires.end(), o.q);
+      o.num_items = static_cast<uint32_t>(words_.back().size() / 3);
+      o.items = words_.back().data();
+      o.mats = floats_.back().data();
+      wires.clear();
+      grads = 0;
+    };
+    constexpr size_t kMost = 12;   // gradients per step
+    for (const auto &kv : by_wire) {
+      const size_t held = items.size() / 3, more = kv.second.size();
+      if (wires.size() == 3 || held + more > QMK_SMALL_MAX_WINDOW || grads + more > kMost) flush();
+      wires.push_back(kv.first);
+      size_t in_step = 0;
+      for (const WireOp *o : kv.second) {
+        if (in_step == kMost) {   // a long wire goes on in steps of its own
+          flush();
+          wires.push_back(kv.first);
+          in_step = 0;
+        }
+        in_step++;
+        items.insert(items.end(), {static_cast<uint32_t>(wires.size() - 1),
+                                   static_cast<uint32_t>(o->gen), o->gen ? o->slot : 0u});
+        mats.resize(mats.size() + 8);
+        narrow(o->minv, mats.data() + mats.size() - 8);
+        grads += o->gen != 0;
+      }
+    }
+    flush();
+  }
+
+  void diag_grad(const std::vector<uint64_t> &gens, const std::vector<uint32_t> &slots) {
+    std::vector<uint32_t> items;
+    for (size_t g = 0; g < gens.size(); g++)
+      items.insert(items.end(), {static_cast<uint32_t>(gens[g]), slots[g]});
+    words_.push_back(std::move(items));
+    qmk_small_op &o = add(QMK_SMALL_DIAG_GRAD, false);
+    o.num_items = static_cast<uint32_t>(gens.size());
+    o.items = words_.back().data();
+  }
+
+ private:
+  qmk_small_op &add(uint32_t kind, bool both) {
+    ops.push_back(qmk_small_op{});
+    ops.back().kind = kind;
+    ops.back().both = both;
+    return ops.back();
+  }
+  const float *matrices(const cdouble *m, size_t count) {
+    floats_.emplace_back(8 * count);
+    for (size_t j = 0; j < count; j++) narrow(m + 4 * j, floats_.back().data() + 8 * j);
+    return floats_.back().data();
+  }
+
+  uint32_t n_;
+  std::deque<std::vector<float>> floats_;   // deques: what an op points to stays in place
+  std::deque<std::vector<uint32_t>> words_;
+  std::deque<std::vector<uint64_t>> maps_;
+  std::deque<std::vector<double>> angles_;
+};
+
+}  // namespace
+
+void Simulator::launch_program(const std::vector<qmk_small_op> &ops, const qmk_small_adjoint *adj) {
+  if (ops.empty()) return;
+  check(qmk_run_small(state_, n_, ops.size(), ops.data(), adj,
+                      static_cast<uint8_t *>(ws_) + ws_bytes_, small_ws_bytes_, stream_),
+        "circuit");
+}
+
+// The plan on a narrow state, its ops in one launch. A dispatch is counted for
+// each plan op. An op the launch cannot take (malformed, or a layer of too
+// many terms) runs, or is refused, by itself in its place.
+void Simulator::run_small(const Plan &p) {
+  SmallProgram prog(n_);
+  const uint64_t start = dispatches_;
+  uint64_t extra = 0;   // launches of an op beyond one
+  const auto steps = small_schedule(p);
+  for (const ForwardStep &st : steps) {
+    if (st.kind == ForwardStep::Group) {
+      prog.group(st.wires.data(), static_cast<uint32_t>(st.wires.size()), st.mats.data());
     } else if (st.kind == ForwardStep::Permute) {
-      o.kind = QMK_SMALL_MAP;
-      o.cols = st.cols.data();
-      ops.push_back(o);
-    } else if (!plan_op(p.ops[st.ops[0]])) {
-      launch();
+      prog.map(st.cols, 0);
+    } else if (!prog.plan_op(p.ops[st.ops[0]])) {
+      launch_program(prog.ops, nullptr);
+      prog.clear();
       const uint64_t own = dispatches_;
       apply_op_to(state_, p.ops[st.ops[0]]);
-      before += dispatches_ - own - 1;   // counted with the plan's ops below
-      dispatches_ = own;
+      if (dispatches_ > own) extra += dispatches_ - own - 1;
     }
   }
-  launch();
-  dispatches_ += p.ops.size() + before;
+  launch_program(prog.ops, nullptr);
+  dispatches_ = start + p.ops.size() + extra;
+}
+
+// Forward pass, samples, co-state and backward sweep of a gradient on a narrow
+// state: one launch (two with samples), through small_schedule and
+// backward_schedule. Every map of the forward pass keeps the state from before
+// it, which the sweep takes back instead of undoing the map on it, where the
+// two schedules' maps pair up one to one. False, with nothing launched, for a
+// circuit that the launch cannot take.
+bool Simulator::small_gradient(const Circuit &c, const Hamiltonian &h, const Plan &plan,
+                               size_t shots, uint64_t seed) {
+  const auto fwd = small_schedule(plan);
+  const auto bwd = backward_schedule(c, tile_high_);
+  // The sweep's steps with every run of CX / SWAP undos as one map.
+  struct Undo {
+    const BackwardStep *step = nullptr;   // null: a map
+    std::vector<uint64_t> cols;
+  };
+  std::vector<Undo> undos;
+  std::vector<PermGate> run;   // in undo order
+  auto end_run = [&]() {
+    if (run.empty()) return;
+    std::reverse(run.begin(), run.end());
+    undos.push_back({nullptr, run_map(n_, run, true).cols});
+    run.clear();
+  };
+  for (const BackwardStep &st : bwd) {
+    if (st.kind == BackwardStep::GateUndo || st.kind == BackwardStep::PermuteUndo) {
+      bool moves = true;
+      for (size_t k : st.gates) {
+        const Gate &g = c.ops[k];
+        moves = moves && (g.kind == G_CX || g.kind == G_SWAP) && g.qubits[0] != g.qubits[1];
+      }
+      if (moves) {
+        for (size_t k : st.gates)
+          run.push_back({c.ops[k].kind == G_SWAP, c.ops[k].qubits[0], c.ops[k].qubits[1]});
+        continue;
+      }
+    }
+    end_run();
+    undos.push_back({&st, {}});
+  }
+  end_run();
+  std::vector<const std::vector<uint64_t> *> kept, undone;
+  for (const ForwardStep &st : fwd)
+    if (st.kind == ForwardStep::Permute) kept.push_back(&st.cols);
+  for (const Undo &u : undos)
+    if (!u.step) undone.push_back(&u.cols);
+  bool pair = kept.size() == undone.size() && kept.size() <= QMK_SMALL_MAX_SAVES;
+  for (size_t i = 0; pair && i < kept.size(); i++)
+    pair = inverts(n_, *kept[kept.size() - 1 - i], 0, *undone[i], 0);
+
+  SmallProgram prog(n_);
+  uint32_t saves = 0;
+  for (const ForwardStep &st : fwd) {
+    if (st.kind == ForwardStep::Group)
+      prog.group(st.wires.data(), static_cast<uint32_t>(st.wires.size()), st.mats.data());
+    else if (st.kind == ForwardStep::Permute)
+      prog.map(st.cols, pair ? ++saves : 0);
+    else if (!prog.plan_op(plan.ops[st.ops[0]]))
+      return false;
+  }
+  const size_t forward_ops = prog.ops.size();
+  if (!prog.costate(h)) return false;
+  for (const Undo &u : undos) {
+    if (!u.step) {
+      prog.map(u.cols, pair ? saves-- : 0, true);
+      continue;
+    }
+    const BackwardStep &st = *u.step;
+    if (st.kind == BackwardStep::Window) {
+      prog.window(st.tile);
+    } else if (st.kind == BackwardStep::Diag) {
+      if (!prog.layer_fits(st.masks, st.angles.size())) return false;
+      if (!st.gens.empty()) prog.diag_grad(st.gens, st.slots);
+      if (st.undo) prog.layer(st.masks, st.angles, st.gphase, true, true);
+    } else {
+      for (size_t k : st.gates)
+        if (!prog.gate_on_both(invert(c.ops[k]))) return false;
+    }
+  }
+  const qmk_small_adjoint adj{costate_, d_grad_, d_grad_cap_, d_results_};
+  if (shots) {
+    std::vector<qmk_small_op> head(prog.ops.begin(), prog.ops.begin() + forward_ops);
+    launch_program(head, &adj);
+    launch_sample(shots, seed);
+    prog.ops.erase(prog.ops.begin(), prog.ops.begin() + forward_ops);
+    dispatches_++;
+  }
+  launch_program(prog.ops, &adj);
+  dispatches_++;
+  return true;
 }
 
 void Simulator::apply_dense_1q(float *st, uint32_t q, const cdouble *m) {
@@ -1298,6 +1545,20 @@ void Simulator::sweep_fused(const Circuit &c) {
   }
 }
 
+// From |0...0>: forward pass, samples, co-state with the energy, block-wise sweep.
+void Simulator::fused_gradient(const Circuit &c, const Hamiltonian &h, size_t shots,
+                               uint64_t seed) {
+  const Plan plan = build_plan(c, FusionOptions{});
+  if (small() && small_gradient(c, h, plan, shots, seed)) return;
+  keep_ckpts_ = checkpoints_pair(c, plan);
+  run_merged(plan);
+  keep_ckpts_ = false;
+  if (shots) launch_sample(shots, seed);
+  energy_and_costate(h);
+  sweep_fused(c);
+  drop_checkpoints();
+}
+
 std::pair<double, std::vector<double>> Simulator::energy_and_gradient(const Circuit &c,
                                                                       const Hamiltonian &h,
                                                                       bool fused) {
@@ -1312,18 +1573,9 @@ std::pair<double, std::vector<double>> Simulator::energy_and_gradient(const Circ
     reset();
     drop_checkpoints();
     if (fused) {
-      const Plan plan = build_plan(c, FusionOptions{});
-      keep_ckpts_ = checkpoints_pair(c, plan);
-      run_merged(plan);
-      keep_ckpts_ = false;
+      fused_gradient(c, h, 0, 0);
     } else {
       run(build_plan(c, FusionOptions::none()));
-    }
-    if (fused) {
-      energy_and_costate(h);
-      sweep_fused(c);
-      drop_checkpoints();
-    } else {
       // The reference's co-state: one pass per flip mask, then the energy.
       costate(h);
       check(qmk_dot_re(state_, costate_, n_, d_results_, ws_, ws_bytes_, stream_), "energy");
@@ -1356,14 +1608,7 @@ void Simulator::serve(const Circuit &c, const Hamiltonian &h, size_t shots, uint
   try {
     reset();
     drop_checkpoints();
-    const Plan plan = build_plan(c, FusionOptions{});
-    keep_ckpts_ = checkpoints_pair(c, plan);
-    run_merged(plan);
-    keep_ckpts_ = false;
-    if (shots) launch_sample(shots, seed);
-    energy_and_costate(h);
-    sweep_fused(c);
-    drop_checkpoints();
+    fused_gradient(c, h, shots, seed);
     if (!c.ops.empty() && grad)
       cuda_check(cudaMemcpyAsync(grad, d_grad_, c.ops.size() * sizeof(double),
                                  cudaMemcpyDeviceToHost, S(stream_)),
@@ -1420,10 +1665,13 @@ void Simulator::serve_enqueue(const Circuit &c, const Hamiltonian &h, size_t sho
     throw std::runtime_error("serve_enqueue: buffers not reserved for this request");
   prepare_adjoint(c, h);
   reset();
-  run_merged(build_plan(c, FusionOptions{}));
-  if (shots) launch_sample(shots, seed);
-  energy_and_costate(h);
-  sweep_fused(c);
+  const Plan plan = build_plan(c, FusionOptions{});
+  if (!small() || !small_gradient(c, h, plan, shots, seed)) {
+    run_merged(plan);
+    if (shots) launch_sample(shots, seed);
+    energy_and_costate(h);
+    sweep_fused(c);
+  }
   if (!c.ops.empty() && pinned_grad)
     cuda_check(cudaMemcpyAsync(pinned_grad, d_grad_, c.ops.size() * sizeof(double),
                                cudaMemcpyDeviceToHost, S(stream_)),

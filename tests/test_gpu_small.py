@@ -81,3 +81,62 @@ def test_norm_and_layers_repeat():
     sim.run(W.to_circuit(n, gates))
     want = oracle.run(n, gates)
     assert np.abs(sim.get_state() - want).max() <= 8 * len(gates) * 2.0 ** -24
+
+
+def _terms(n, rng):
+    full = (1 << n) - 1
+    out = [(0.5, 0, 0, 0), (-1.0, 0, 0, 1), (0.7, 1 << (n - 1), 0, 0), (0.3, 0, 1, 0)]
+    for _ in range(6):
+        x = int(rng.integers(0, full + 1))
+        y = int(rng.integers(0, full + 1)) & ~x
+        z = int(rng.integers(0, full + 1)) & ~(x | y)
+        out.append((float(rng.uniform(-1, 1)), x, y, z))
+    return out
+
+
+def _check_gradient(n, gates, terms):
+    e0, g0 = oracle.energy_and_gradient(n, gates, terms)
+    c, h = W.to_circuit(n, gates), W.to_hamiltonian(terms)
+    # both states carry the gates' roundings, forward and back, and H's norm
+    tol = 4 * 8 * max(1, len(gates)) * 2.0 ** -24 * sum(abs(t[0]) for t in terms)
+    sim = qm.Simulator(n)
+    for _ in range(2):
+        e, g = sim.energy_and_gradient(c, h)
+        assert abs(e - e0) <= tol
+        assert len(g) == len(gates) and np.abs(np.array(g) - g0).max(initial=0.0) <= tol
+    (eb, gb, sb), = qm.batch_serve([(c, h, 50, 3)], lanes=1)
+    assert abs(eb - e0) <= tol and np.abs(np.array(gb) - g0).max(initial=0.0) <= tol
+    ref = qm.Simulator(n)
+    ref.run_merged(c)
+    assert sb == ref.sample(50, seed=3)
+
+
+@pytest.mark.parametrize("n", range(1, 15))
+def test_gradient(n):
+    rng = np.random.default_rng(360 + n)
+    terms = _terms(n, rng)
+    rotations = [(int(k), (int(q),), (float(rng.uniform(-3, 3)),))
+                 for k, q in zip(rng.choice([W.RX, W.RY, W.RZ], 60), rng.integers(0, n, 60))]
+    _check_gradient(n, rotations, terms)
+    _check_gradient(n, [(W.RX, (0,), (0.1 * k,)) for k in range(40)], terms)
+    if n == 1:
+        return
+    free = [g for g in (_gate(n, rng) for _ in range(150)) if g[0] not in (W.P, W.CP)]
+    _check_gradient(n, free, terms)
+    _check_gradient(n, W.hea(n, 4), W.ring_tfim_hamiltonian(n, 0.7) if n > 2 else terms)
+    if n > 2:
+        _check_gradient(n, W.qaoa_ring_seeded(n, 3), W.maxcut_hamiltonian(
+            [(i, (i + 1) % n) for i in range(n)]))
+        _check_gradient(n, W.tfim_chain(n, 4), W.ring_tfim_hamiltonian(n, 0.7))
+        coupled = []
+        for _ in range(2):   # more couplings than one step's sums
+            for a in range(n):
+                for b in range(a):
+                    coupled += [(W.CX, (a, b), ()), (W.RZ, (b,), (0.2 + a,)), (W.CX, (a, b), ())]
+            coupled += [(W.RX, (q,), (0.5,)) for q in range(n)]
+        _check_gradient(n, coupled, terms)
+
+
+@pytest.mark.parametrize("n, depth", [(4, 40), (10, 20), (13, 12)])
+def test_gradient_long(n, depth):
+    _check_gradient(n, W.hea(n, depth), W.ring_tfim_hamiltonian(n, 0.7))   # several launches
