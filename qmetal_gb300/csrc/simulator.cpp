@@ -108,7 +108,7 @@ uint64_t Simulator::recommended_working_set() {
   return total_b;
 }
 
-Simulator::Simulator(uint32_t n) : n_(n) {
+Simulator::Simulator(uint32_t n) : n_(n), capacity_(n) {
   if (n == 0 || n > kMaxQubits)
     throw std::runtime_error("Simulator: num_qubits must be 1.." + std::to_string(kMaxQubits));
   const char *fault = std::getenv("QMETAL_FAULT");
@@ -156,26 +156,103 @@ Simulator::Simulator(uint32_t n) : n_(n) {
   }
 }
 
+namespace {
+
+size_t padded(size_t bytes) { return (bytes + 255) & ~size_t(255); }
+
+// The widest workspace for narrow states that a simulator of up to n qubits needs.
+size_t small_bytes_up_to(uint32_t n) {
+  return qmk_small_workspace_bytes(std::min<uint32_t>(n, QMK_SMALL_MAX_QUBITS));
+}
+
+}  // namespace
+
+size_t Simulator::lane_device_bytes(uint32_t n, size_t max_gates, size_t max_shots) {
+  return 2 * padded((size_t(8) << n)) + padded(qmk_workspace_bytes(n) + small_bytes_up_to(n)) +
+         padded(kResultSlots * sizeof(double)) +
+         padded(std::max<size_t>(max_gates, 1) * sizeof(double)) +
+         (max_shots ? padded(qmk_sample_workspace_bytes(n)) + padded(max_shots * sizeof(uint64_t))
+                    : 0);
+}
+
+size_t Simulator::lane_pinned_bytes() { return (kResultSlots + 1) * sizeof(double); }
+
+// A batch lane's simulator of up to n qubits: everything but its stream comes
+// from the batch's memory, so a lane allocates nothing and frees nothing.
+Simulator::Simulator(uint32_t n, const LaneMemory &m) : n_(n), capacity_(n), lane_(m) {
+  if (n == 0 || n > kMaxQubits)
+    throw std::runtime_error("Simulator: num_qubits must be 1.." + std::to_string(kMaxQubits));
+  cuda_check(cudaGetDevice(&device_), "cudaGetDevice");
+  ws_bytes_ = qmk_workspace_bytes(n);
+  small_ws_bytes_ = qmk_small_workspace_bytes(n);
+  uint8_t *at = static_cast<uint8_t *>(m.device);
+  auto take = [&](size_t bytes) {
+    uint8_t *p = at;
+    at += padded(bytes);
+    return p;
+  };
+  state_ = reinterpret_cast<float *>(take(size_t(8) << n));
+  costate_ = reinterpret_cast<float *>(take(size_t(8) << n));
+  ws_ = take(ws_bytes_ + small_bytes_up_to(n));
+  d_results_ = reinterpret_cast<double *>(take(kResultSlots * sizeof(double)));
+  d_grad_cap_ = std::max<size_t>(m.max_gates, 1);
+  d_grad_ = reinterpret_cast<double *>(take(d_grad_cap_ * sizeof(double)));
+  if (m.max_shots) {
+    sample_ws_bytes_ = qmk_sample_workspace_bytes(n);
+    sample_ws_ = take(sample_ws_bytes_);
+    d_shots_cap_ = m.max_shots;
+    d_shots_ = reinterpret_cast<uint64_t *>(take(m.max_shots * sizeof(uint64_t)));
+  }
+  h_results_ = static_cast<double *>(m.pinned);
+  h_waits_ = reinterpret_cast<unsigned *>(h_results_ + kResultSlots);
+  cudaStream_t s;
+  cuda_check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");
+  stream_ = s;
+  try {
+    check(qmk_workspace_init(ws_, ws_bytes_, stream_), "workspace init");
+    const char *fault = std::getenv("QMETAL_FAULT");
+    fault_launch_ = fault && std::strcmp(fault, "launch") == 0;
+    if (const char *cap = std::getenv("QMETAL_MAX_CHECKPOINTS"))
+      ck_limit_ = static_cast<size_t>(std::strtoul(cap, nullptr, 10));
+  } catch (...) {
+    release();
+    throw;
+  }
+}
+
+void Simulator::narrow_to(uint32_t n) {
+  if (n == 0 || n > capacity_) throw std::runtime_error("Simulator: wider than its memory");
+  n_ = n;
+  small_ws_bytes_ = qmk_small_workspace_bytes(n);
+  invalidate_graphs();
+}
+
+void Simulator::free_device(void *p) {
+  const uint8_t *b = static_cast<const uint8_t *>(lane_.device);
+  const uint8_t *q = static_cast<const uint8_t *>(p);
+  if (!b || q < b || q >= b + lane_.device_bytes) cudaFree(p);
+}
+
 Simulator::~Simulator() { release(); }
 
 void Simulator::release() {
   if (stream_) cudaStreamSynchronize(S(stream_));
   for (const GraphEntry &e : graphs_) cudaGraphExecDestroy(static_cast<cudaGraphExec_t>(e.exec));
   graphs_.clear();
-  cudaFree(state_);
-  cudaFree(costate_);
-  cudaFree(scratch_);
+  free_device(state_);
+  free_device(costate_);
+  free_device(scratch_);
   scratch_ = nullptr;
-  for (const Checkpoint &c : ckpts_) cudaFree(c.buf);
+  for (const Checkpoint &c : ckpts_) free_device(c.buf);
   ckpts_.clear();
-  for (float *b : ck_free_) cudaFree(b);
+  for (float *b : ck_free_) free_device(b);
   ck_free_.clear();
-  cudaFree(ws_);
-  cudaFree(sample_ws_);
-  cudaFree(d_shots_);
-  cudaFree(d_results_);
-  cudaFree(d_grad_);
-  if (h_results_) cudaFreeHost(h_results_);
+  free_device(ws_);
+  free_device(sample_ws_);
+  free_device(d_shots_);
+  free_device(d_results_);
+  free_device(d_grad_);
+  if (h_results_ && !lane_.pinned) cudaFreeHost(h_results_);
   if (mirror_) {
     if (mirror_pinned_) cudaFreeHost(mirror_);
     else std::free(mirror_);
@@ -214,7 +291,7 @@ void Simulator::synchronize() {
 bool Simulator::ensure_scratch() {
   if (scratch_) return true;
   if (scratch_failed_) return false;
-  const size_t bytes = dim() * 8;
+  const size_t bytes = size_t(8) << capacity_;
   size_t free_b = 0, total_b = 0;
   // Keep 2 GiB of headroom for other simulators and the runtime.
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < bytes + (2ull << 30) ||
@@ -241,7 +318,7 @@ float *Simulator::take_buffer() {
   size_t held = 0;
   for (const Checkpoint &c : ckpts_) held += c.buf != nullptr;
   if (held >= ck_limit_) return nullptr;
-  const size_t bytes = dim() * 8;
+  const size_t bytes = size_t(8) << capacity_;
   size_t free_b = 0, total_b = 0;
   float *b = nullptr;
   // Keep 4 GiB of headroom for other simulators and the runtime.
@@ -1321,7 +1398,7 @@ void Simulator::launch_sample(size_t shots, uint64_t seed) {
     sample_ws_bytes_ = need;
   }
   if (d_shots_cap_ < shots) {
-    cudaFree(d_shots_);
+    free_device(d_shots_);
     d_shots_ = nullptr;
     d_shots_cap_ = 0;
     cuda_check(cudaMalloc(&d_shots_, shots * sizeof(uint64_t)), "sampling output");
@@ -1411,7 +1488,7 @@ void Simulator::prepare_adjoint(const Circuit &c, const Hamiltonian &h) {
   }
   const size_t G = std::max<size_t>(c.ops.size(), 1);
   if (d_grad_cap_ < G) {
-    cudaFree(d_grad_);
+    free_device(d_grad_);
     d_grad_ = nullptr;
     d_grad_cap_ = 0;
     cuda_check(cudaMalloc(&d_grad_, G * sizeof(double)), "gradient buffer");
@@ -1637,7 +1714,7 @@ void Simulator::reserve(size_t max_gates, size_t max_shots) {
   }
   const size_t G = std::max<size_t>(max_gates, 1);
   if (d_grad_cap_ < G) {
-    cudaFree(d_grad_);
+    free_device(d_grad_);
     d_grad_ = nullptr;
     d_grad_cap_ = 0;
     cuda_check(cudaMalloc(&d_grad_, G * sizeof(double)), "gradient buffer");
@@ -1648,7 +1725,7 @@ void Simulator::reserve(size_t max_gates, size_t max_shots) {
     cuda_check(cudaMalloc(&sample_ws_, sample_ws_bytes_), "sampling workspace");
   }
   if (max_shots && d_shots_cap_ < max_shots) {
-    cudaFree(d_shots_);
+    free_device(d_shots_);
     d_shots_ = nullptr;
     d_shots_cap_ = 0;
     cuda_check(cudaMalloc(&d_shots_, max_shots * sizeof(uint64_t)), "sampling output");

@@ -23,6 +23,21 @@ constexpr uint32_t kMaxQubits = 34;
 class Simulator {
  public:
   explicit Simulator(uint32_t num_qubits);
+  // For a batch lane: a simulator of up to num_qubits in memory the batch
+  // holds (lane_device_bytes() device bytes, 256-byte aligned, and
+  // lane_pinned_bytes() of pinned host memory), which outlives it.
+  struct LaneMemory {
+    void *device = nullptr;
+    size_t device_bytes = 0;
+    void *pinned = nullptr;
+    size_t max_gates = 0, max_shots = 0;
+  };
+  Simulator(uint32_t num_qubits, const LaneMemory &memory);
+  static size_t lane_device_bytes(uint32_t num_qubits, size_t max_gates, size_t max_shots);
+  static size_t lane_pinned_bytes();
+  // The next circuits have n qubits, at most the simulator's own number. The
+  // state is undefined until it is reset or set.
+  void narrow_to(uint32_t n);
   ~Simulator();
   Simulator(const Simulator &) = delete;
   Simulator &operator=(const Simulator &) = delete;
@@ -118,6 +133,7 @@ class Simulator {
 
  private:
   void release();
+  void free_device(void *p);   // unless it is lane memory
   void check(int rc, const char *what);
   void activate() const;
   void apply_gate_to(float *state, const Gate &g);
@@ -171,6 +187,8 @@ class Simulator {
   void invalidate_graphs();
 
   uint32_t n_ = 0;
+  uint32_t capacity_ = 0;               // qubits its buffers hold
+  LaneMemory lane_;
   int device_ = 0;
   void *stream_ = nullptr;
   float *state_ = nullptr;
