@@ -187,6 +187,14 @@ size_t qm_circuit_plan_export(qm_circuit c, int collapse_1q_windows,
 size_t qm_schedule_export(qm_circuit c, const qm_hamiltonian *h, int which,
                           uint32_t tile_high, double *out, size_t cap);
 
+/* qm_circuit_add for `count` gates in one call: gate k takes the next
+ * num_qubits[k] entries of qubits and num_params[k] of params. The first gate
+ * that qm_circuit_add would refuse ends the call with its error; the gates
+ * before it stay. */
+int qm_circuit_add_many(qm_circuit c, size_t count, const int *kinds,
+                        const uint32_t *num_qubits, const uint32_t *qubits,
+                        const uint32_t *num_params, const double *params);
+
 /* Per-term expectation values <P_t> (without the coefficients), one entry
  * per Hamiltonian term, computed in grouped passes over the state. */
 int qm_expectation_terms(qm_simulator s, const qm_hamiltonian *h,

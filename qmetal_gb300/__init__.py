@@ -91,6 +91,8 @@ _circuit_create = _decl("qm_circuit_create", c_void_p, c_uint32)
 _circuit_destroy = _decl("qm_circuit_destroy", None, c_void_p)
 _circuit_add = _decl("qm_circuit_add", c_int, c_void_p, c_int, _u32p, c_uint32,
                      _f64p, c_uint32)
+_circuit_add_many = _decl("qm_circuit_add_many", c_int, c_void_p, c_size_t, POINTER(c_int), _u32p,
+                          _u32p, _u32p, _f64p)
 _circuit_size = _decl("qm_circuit_size", c_size_t, c_void_p)
 _plan_size = _decl("qm_circuit_plan_size", c_size_t, c_void_p, c_int)
 _plan_export = _decl("qm_circuit_plan_export", c_size_t, c_void_p, c_int, c_int,
@@ -255,6 +257,22 @@ class Circuit:
         """Append a gate by its qm_gate_kind code."""
         return self._add(int(kind), tuple(int(q) for q in qubits),
                          tuple(float(p) for p in params))
+
+    def extend(self, gates):
+        """Append (kind, qubits, params) gates in one call (116 gates: 230 us
+        one at a time, most of it the crossings)."""
+        kinds, nqs, qubits, nps, params = [], [], [], [], []
+        for kind, qs, ps in gates:
+            kinds.append(int(kind))
+            nqs.append(len(qs))
+            qubits.extend(map(int, qs))
+            nps.append(len(ps))
+            params.extend(map(float, ps))
+        n = len(kinds)
+        _check(_circuit_add_many(self._h, n, (c_int * n)(*kinds), (c_uint32 * n)(*nqs),
+                                 (c_uint32 * max(1, len(qubits)))(*qubits), (c_uint32 * n)(*nps),
+                                 (c_double * max(1, len(params)))(*params)))
+        return self
 
     # single-qubit
     def x(self, q): return self._add(X, (q,))

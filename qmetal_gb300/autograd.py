@@ -39,11 +39,9 @@ class Template:
         a = [float(x) for x in angles]
         if len(a) != self.num_params:
             raise ValueError(f"expected {self.num_params} angles, got {len(a)}")
-        c = Circuit(self.num_qubits)
         it = iter(a)
-        for k, qs, ps in self.gates:
-            c.add(k, qs, (next(it),) if ps else ())
-        return c
+        return Circuit(self.num_qubits).extend(
+            (k, qs, (next(it),) if ps else ()) for k, qs, ps in self.gates)
 
 
 def _ham(h):

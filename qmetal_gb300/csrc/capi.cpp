@@ -167,6 +167,23 @@ int qm_circuit_add(qm_circuit c, qm_gate_kind kind, const uint32_t *qubits, uint
   return guarded([&] { c->c.add(gate_of(c->c.num_qubits, kind, qubits, nq, params, np)); });
 }
 
+int qm_circuit_add_many(qm_circuit c, size_t count, const int *kinds, const uint32_t *num_qubits,
+                        const uint32_t *qubits, const uint32_t *num_params, const double *params) {
+  if (!c || (count && (!kinds || !num_qubits || !num_params))) {
+    set_error(c ? "null argument" : "null circuit");
+    return -1;
+  }
+  return guarded([&] {
+    c->c.ops.reserve(c->c.ops.size() + count);
+    for (size_t k = 0; k < count; k++) {
+      const uint32_t nq = num_qubits[k], np = num_params[k];
+      c->c.add(gate_of(c->c.num_qubits, static_cast<qm_gate_kind>(kinds[k]), qubits, nq, params, np));
+      qubits += nq;
+      if (params) params += np;
+    }
+  });
+}
+
 size_t qm_circuit_size(qm_circuit c) { return c ? c->c.size() : 0; }
 
 size_t qm_circuit_plan_size(qm_circuit c, int fuse) {

@@ -26,10 +26,7 @@ CX, CY, CZ, SWAP, CP, CCX = 12, 13, 14, 15, 16, 17
 
 def to_circuit(n, gates):
     from . import Circuit
-    c = Circuit(n)
-    for k, qs, ps in gates:
-        c.add(k, qs, ps)
-    return c
+    return Circuit(n).extend(gates)
 
 
 def hot_wires_first(n, gates):
