@@ -227,10 +227,7 @@ __device__ __forceinline__ void adj_diag_body(float4 *__restrict__ psi, float4 *
     }
     __syncthreads();
   }
-  double acc[T > 0 ? T : 1];
-#pragma unroll
-  for (int t = 0; t < (T > 0 ? T : 1); t++) acc[t] = accf[t];
-  if constexpr (T > 0) finish<T>(acc, g.ngen, a, out);
+  if constexpr (T > 0) finish<T>(accf, g.ngen, a, out);
 }
 
 template <int T>

@@ -68,7 +68,7 @@ k_adj_warp(float4 *__restrict__ psi, float4 *__restrict__ lam, uint64_t nwsites,
     }
   }
   if constexpr (NG > 0) {
-    double acc[NA];
+    float acc[NA];
 #pragma unroll
     for (int t = 0; t < NA; t++) acc[t] = sacc[t][threadIdx.x];
     finish<NG>(acc, static_cast<int>(g.ngrad), a, out);
@@ -167,7 +167,7 @@ k_adj_pair(float4 *__restrict__ psi, float4 *__restrict__ lam, uint64_t nwsites,
     }
   }
   if constexpr (NG > 0) {
-    double acc[NA];
+    float acc[NA];
 #pragma unroll
     for (int t = 0; t < NA; t++) acc[t] = sacc[t][tid];
     finish<NG>(acc, static_cast<int>(g.ngrad), a, out);

@@ -398,10 +398,7 @@ k_adj_pair_uni(float4 *__restrict__ psi, float4 *__restrict__ lam, uint64_t nwsi
       accf[LANE0 + M * k] += ((lane >> g.lbit[k]) & 1) ? -sl : sl;
     accf[REG0 + 3 * M] += half ? -sl : sl;
   }
-  double acc[NOPS];
-#pragma unroll
-  for (int t = 0; t < NOPS; t++) acc[t] = accf[t];
-  finish<NOPS>(acc, NOPS, a, out);
+  finish<NOPS>(accf, NOPS, a, out);
 }
 
 // KH <= 3 register wires on one warp, optionally with wire 0 and the five
@@ -482,10 +479,7 @@ k_adj_warp_uni(float4 *__restrict__ psi, float4 *__restrict__ lam, uint64_t nwsi
     for (int k = 0; k < NL; k++)
       accf[LANE0 + M * k + RZ] += ((lane >> g.lbit[k]) & 1) ? -sl : sl;
   }
-  double acc[NOPS];
-#pragma unroll
-  for (int t = 0; t < NOPS; t++) acc[t] = accf[t];
-  finish<NOPS>(acc, NOPS, a, out);
+  finish<NOPS>(accf, NOPS, a, out);
 }
 
 // Five or six wires >= 6 per pass on a block tile: a site is 2^(3 + WB)
@@ -656,10 +650,7 @@ k_adj_blk_uni(float4 *__restrict__ psi, float4 *__restrict__ lam, uint64_t nsite
   }
   if (stalled && !__all_sync(0xffffffffu, mbar_wait(&mbar[warp], stalled_parity)) && lane == 0)
     atomicAdd(a.waits, 1u);
-  double acc[NOPS];
-#pragma unroll
-  for (int t = 0; t < NOPS; t++) acc[t] = accf[t];
-  finish<NOPS>(acc, NOPS, a, out);
+  finish<NOPS>(accf, NOPS, a, out);
 }
 
 template <int WB, int M, int C0, int G0, int C1, int G1>

@@ -26,7 +26,6 @@
 #include <vector>
 
 #include "kadjoint.cuh"
-#include "kcommon.cuh"
 #include "../../include/qmetal/qmetal_kernels.h"
 
 using namespace qmk;
@@ -161,33 +160,14 @@ __device__ __forceinline__ void group_cls(float2 *amp, uint32_t n, const uint32_
   }
 }
 
-// A sum as FP32 high and low parts: exact to about 2^-46, on the FP32 pipe (an
-// FP64 add holds a multiprocessor's FP64 unit for 16 cycles a warp).
-struct Two {
-  float hi, lo;
-};
-__device__ __forceinline__ Two two_add(Two a, Two b) {
-  const float s = __fadd_rn(a.hi, b.hi), t = __fadd_rn(s, -a.hi);
-  const float e = __fadd_rn(__fadd_rn(a.hi, -__fadd_rn(s, -t)), __fadd_rn(b.hi, -t));
-  const float lo = __fadd_rn(e, __fadd_rn(a.lo, b.lo));
-  const float hi = __fadd_rn(s, lo);
-  return {hi, __fadd_rn(lo, -__fadd_rn(hi, -s))};
-}
-
 // The threads' partial sums of one result, added by one warp in a fixed order.
 __device__ __forceinline__ double row_sum(const float *row, uint32_t count) {
   const uint32_t lane = threadIdx.x & 31;
   Two v = {0.0f, 0.0f};
-  for (uint32_t t = lane; t < count; t += 32) v = two_add(v, {row[t], 0.0f});
+  for (uint32_t t = lane; t < count; t += 32) v = add(v, Two{row[t], 0.0f});
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-    v = two_add(v, {__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)});
-  if (__any_sync(0xffffffffu, v.hi != v.hi)) {   // infinities: their plain sum
-    double d = 0.0;
-    for (uint32_t t = lane; t < count; t += 32) d += row[t];
-    return warp_sum(d);
-  }
-  return static_cast<double>(v.hi) + static_cast<double>(v.lo);
+  for (int o = 16; o > 0; o >>= 1) v = add(v, shfl_xor(v, o));
+  return widen(v);
 }
 
 // Im(conj(lambda) P psi) over the register pairs of wire bit J.
