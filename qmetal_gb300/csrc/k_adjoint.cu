@@ -44,14 +44,18 @@ namespace {
 
 __global__ void __launch_bounds__(kThreads)
 k_zdiag(float4 *__restrict__ lam, const float4 *__restrict__ psi, const DiagDesc *__restrict__ d,
-        const float2 *__restrict__ table2, uint64_t ntiles, Area a, double *out) {
+        const float2 *__restrict__ table2, uint64_t nparts, uint32_t part_bits, Area a,
+        double *out) {
   __shared__ float cr[kWMax];
   __shared__ float hr;
   __shared__ __align__(16) float Y1[64];
   __shared__ float Y2[1 << (kWMax - 6)];
-  const uint32_t W = d->W, tid = threadIdx.x, nv = 1u << (W - 1);
+  // A block takes one of the 2^part_bits equal parts of a tile's vectors.
+  const uint32_t W = d->W, tid = threadIdx.x, nv = 1u << (W - 1 - part_bits);
   double acc[1] = {0.0};
-  for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+  for (uint64_t kp = blockIdx.x; kp < nparts; kp += gridDim.x) {
+    const uint64_t tile = kp >> part_bits;
+    const uint32_t first = (static_cast<uint32_t>(kp) & ((1u << part_bits) - 1u)) * nv;
     tile_coeffs<false>(d, tile, nullptr, nullptr, cr, &hr, false);
     __syncthreads();
     tile_real_tables(W, cr, hr, Y1, Y2);
@@ -66,20 +70,20 @@ k_zdiag(float4 *__restrict__ lam, const float4 *__restrict__ psi, const DiagDesc
       for (int k = 0; k < UU; k++) {
         const uint32_t e = e0 + k * kThreads;
         if (e < nv) {
-          x[k] = psi[base + e];
-          t[k] = table2[e];   // table of floats read two at a time
+          x[k] = psi[base + first + e];
+          t[k] = table2[first + e];   // table of floats read two at a time
         }
       }
 #pragma unroll
       for (int k = 0; k < UU; k++) {
         const uint32_t e = e0 + k * kThreads;
         if (e >= nv) continue;
-        const uint32_t lo = 2 * e;
+        const uint32_t lo = 2 * (first + e);
         const float2 y1 = *reinterpret_cast<const float2 *>(&Y1[lo & 63]);
         const float y2 = Y2[lo >> 6];
         const float d0 = t[k].x + (y1.x + y2), d1 = t[k].y + (y1.y + y2);
         const float4 v = x[k];
-        lam[base + e] = make_float4(d0 * v.x, d0 * v.y, d1 * v.z, d1 * v.w);
+        lam[base + first + e] = make_float4(d0 * v.x, d0 * v.y, d1 * v.z, d1 * v.w);
         part += d0 * (v.x * v.x + v.y * v.y) + d1 * (v.z * v.z + v.w * v.w);
       }
     }
@@ -440,11 +444,13 @@ extern "C" int qmk_zdiag_costate(float *lam, const float *psi, uint32_t n, uint3
   int rc = launch_status();
   if (rc) return rc;
   const uint64_t ntiles = 1ull << (n - d.W);
-  const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(ntiles, reduce_grid()));
+  const uint32_t part_bits = tile_part_bits(ntiles, d.W - 1);
+  const uint64_t nparts = ntiles << part_bits;
+  const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(nparts, reduce_grid()));
   k_zdiag<<<grid, kThreads, 0, s>>>(reinterpret_cast<float4 *>(lam),
                                     reinterpret_cast<const float4 *>(psi), dd,
-                                    reinterpret_cast<const float2 *>(table), ntiles, area_of(ws),
-                                    d_energy);
+                                    reinterpret_cast<const float2 *>(table), nparts, part_bits,
+                                    area_of(ws), d_energy);
   return launch_status();
 }
 

@@ -43,19 +43,23 @@ namespace {
 
 __global__ void __launch_bounds__(kThreads)
 k_diag(float4 *__restrict__ st, const DiagDesc *__restrict__ d,
-       const float4 *__restrict__ table4, uint64_t ntiles, int tile_bit, int vec_bit) {
+       const float4 *__restrict__ table4, uint64_t nparts, uint32_t part_bits, int tile_bit,
+       int vec_bit) {
   __shared__ float2 f[kWMax];
   __shared__ float2 eH;
   __shared__ __align__(16) float2 Y1[64];
   __shared__ float2 Y2[1 << (kWMax - 6)];
   const uint32_t W = d->W;
   const uint32_t tid = threadIdx.x;
-  // tile_bit / vec_bit >= 0: only tiles / vectors with that bit set.
-  const uint32_t nv = 1u << (vec_bit < 0 ? W - 1 : W - 2);
+  // tile_bit / vec_bit >= 0: only tiles / vectors with that bit set. A block
+  // takes one of the 2^part_bits equal parts of a tile's vectors.
+  const uint32_t nv = 1u << ((vec_bit < 0 ? W - 1 : W - 2) - part_bits);
   auto vec = [&](uint32_t e) {
     return vec_bit < 0 ? e : static_cast<uint32_t>(ins0(e, vec_bit)) | (1u << vec_bit);
   };
-  for (uint64_t k = blockIdx.x; k < ntiles; k += gridDim.x) {
+  for (uint64_t kp = blockIdx.x; kp < nparts; kp += gridDim.x) {
+    const uint64_t k = kp >> part_bits;
+    const uint32_t first = (static_cast<uint32_t>(kp) & ((1u << part_bits) - 1u)) * nv;
     const uint64_t tile = tile_bit < 0 ? k : ins0(k, tile_bit) | (1ull << tile_bit);
     tile_coeffs<true>(d, tile, f, &eH, nullptr, nullptr, false);
     __syncthreads();
@@ -69,20 +73,20 @@ k_diag(float4 *__restrict__ st, const DiagDesc *__restrict__ d,
       for (int k = 0; k < UU; k++) {
         const uint32_t e = e0 + k * kThreads;
         if (e < nv) {
-          x[k] = st[base + vec(e)];
-          t[k] = table4[vec(e)];
+          x[k] = st[base + vec(first + e)];
+          t[k] = table4[vec(first + e)];
         }
       }
 #pragma unroll
       for (int k = 0; k < UU; k++) {
         const uint32_t e = e0 + k * kThreads;
         if (e >= nv) continue;
-        const uint32_t lo = 2 * vec(e);
+        const uint32_t lo = 2 * vec(first + e);
         const float4 y1 = *reinterpret_cast<const float4 *>(&Y1[lo & 63]);
         const float2 y2 = Y2[lo >> 6];
         const float2 f0 = cmul(cmul(lo2(t[k]), lo2(y1)), y2);
         const float2 f1 = cmul(cmul(hi2(t[k]), hi2(y1)), y2);
-        st[base + vec(e)] = pack4(cmul(f0, lo2(x[k])), cmul(f1, hi2(x[k])));
+        st[base + vec(first + e)] = pack4(cmul(f0, lo2(x[k])), cmul(f1, hi2(x[k])));
       }
     }
     __syncthreads();
@@ -156,10 +160,12 @@ extern "C" int qmk_apply_diagonal(float *state, uint32_t n, uint32_t nt,
   const int vec_bit = q >= 0 && q < static_cast<int>(W) ? q - 1 : -1;
   const uint64_t ntiles = 1ull << (n - W - (tile_bit >= 0 ? 1 : 0));
   const uint64_t cap = static_cast<uint64_t>(qmk_host::num_sms()) * 8;
-  const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(ntiles, cap));
+  const uint32_t part_bits = tile_part_bits(ntiles, vec_bit < 0 ? W - 1 : W - 2);
+  const uint64_t nparts = ntiles << part_bits;
+  const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(nparts, cap));
   k_diag<<<grid, kThreads, 0, s>>>(reinterpret_cast<float4 *>(state), dd,
-                                   reinterpret_cast<const float4 *>(table), ntiles, tile_bit,
-                                   vec_bit);
+                                   reinterpret_cast<const float4 *>(table), nparts, part_bits,
+                                   tile_bit, vec_bit);
   rc = launch_status();
   if (rc) return rc;
   for (size_t b = 0; b < gm.size(); b += kGenericTerms) {
