@@ -287,9 +287,8 @@ k_group5_pair(float4 *__restrict__ st, uint64_t nsites, GroupArgs g) {
 // number, carried by the store addresses, so the pass takes no longer.
 struct BlkGroupArgs {
   uint32_t pos[7];   // the wires' vector bits (wire - 1), ascending, all >= 5
-  uint32_t act;      // bit j: wire j of the site has a 2x2
-  uint32_t moved;    // rows move after the 2x2s:
-  uint8_t img[7];    //   the image of each row bit
+  uint32_t act;      // MOVES: bit j: wire j of the site has a 2x2
+  uint8_t img[7];    // MOVES: the image of each row bit
   M2 m[7];
   M2 m0;             // wire 0 when W0
 };
@@ -308,7 +307,10 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // thread that issued them) once every warp of the site has read the current
 // second layout, so the copies overlap the second half of the arithmetic and
 // the stores.
-template <int WB, bool W0, int CLS>
+// MOVES: gates follow, and not every wire need have a 2x2 (a test per wire
+// that the compiler schedules around: without it an HEA layer's pass is 1.17
+// times as fast).
+template <int WB, bool W0, int CLS, bool MOVES>
 __global__ void __launch_bounds__(kThreads, 2)
 k_group_blk(float4 *__restrict__ st, uint64_t nsites, BlkGroupArgs g) {
   constexpr int NV = 16;
@@ -335,7 +337,7 @@ k_group_blk(float4 *__restrict__ st, uint64_t nsites, BlkGroupArgs g) {
   {
     const int l = lane & (NV - 1);
     uint32_t row = lane < NV ? row_a(l) : row_b(l);
-    if (lane >= NV && g.moved) {
+    if (MOVES && lane >= NV) {
       uint32_t to = 0;
 #pragma unroll
       for (int j = 0; j < KB; j++)
@@ -376,7 +378,7 @@ k_group_blk(float4 *__restrict__ st, uint64_t nsites, BlkGroupArgs g) {
     cp_async_commit();
   };
   auto reg_wire = [&](float4 (&r)[NV], int j, int wire) {
-    if (!((g.act >> wire) & 1u)) return;
+    if (MOVES && !((g.act >> wire) & 1u)) return;
     const M2 &m = g.m[wire];
 #pragma unroll
     for (int l = 0; l < NV; l++) {
@@ -920,7 +922,7 @@ static int launch_group5_pair_cls(float4 *st, uint64_t nsites, const GroupArgs &
   return launch_status();
 }
 
-template <int WB, bool W0, int CLS>
+template <int WB, bool W0, int CLS, bool MOVES>
 static int launch_group_blk_cls(float4 *st, uint64_t nsites, const BlkGroupArgs &g,
                                 cudaStream_t s) {
   constexpr int SPB = (kThreads / 32) >> WB;
@@ -931,25 +933,25 @@ static int launch_group_blk_cls(float4 *st, uint64_t nsites, const BlkGroupArgs 
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
   if (!opted[dev]) {
     const cudaError_t e = cudaFuncSetAttribute(
-        k_group_blk<WB, W0, CLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        k_group_blk<WB, W0, CLS, MOVES>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
     opted[dev] = true;
   }
   // Resident blocks only: each loops over its sites.
   const unsigned grid = std::min<unsigned>(grid_for(nsites, SPB),
                                            static_cast<unsigned>(qmk_host::num_sms()) * 2);
-  k_group_blk<WB, W0, CLS><<<grid, kThreads, smem, s>>>(st, nsites, g);
+  k_group_blk<WB, W0, CLS, MOVES><<<grid, kThreads, smem, s>>>(st, nsites, g);
   return launch_status();
 }
 
-template <int WB, bool W0>
+template <int WB, bool W0, bool MOVES = false>
 static int launch_group_blk(float4 *st, uint64_t nsites, const BlkGroupArgs &g, int cls,
                             cudaStream_t s) {
   switch (cls) {
-    case kMatDiag: return launch_group_blk_cls<WB, W0, kMatDiag>(st, nsites, g, s);
-    case kMatRx: return launch_group_blk_cls<WB, W0, kMatRx>(st, nsites, g, s);
-    case kMatReal: return launch_group_blk_cls<WB, W0, kMatReal>(st, nsites, g, s);
-    default: return launch_group_blk_cls<WB, W0, kMatGeneral>(st, nsites, g, s);
+    case kMatDiag: return launch_group_blk_cls<WB, W0, kMatDiag, MOVES>(st, nsites, g, s);
+    case kMatRx: return launch_group_blk_cls<WB, W0, kMatRx, MOVES>(st, nsites, g, s);
+    case kMatReal: return launch_group_blk_cls<WB, W0, kMatReal, MOVES>(st, nsites, g, s);
+    default: return launch_group_blk_cls<WB, W0, kMatGeneral, MOVES>(st, nsites, g, s);
   }
 }
 
@@ -1045,7 +1047,6 @@ extern "C" int qmk_apply_group(float *state, uint32_t n, uint32_t k,
           bg.m0 = m;
         } else {
           bg.pos[kb] = qubits[j] - 1;
-          bg.act |= 1u << kb;
           bg.m[kb] = m;
           kb++;
         }
@@ -1192,14 +1193,13 @@ extern "C" int qmk_apply_group_moves(float *state, uint32_t n, uint32_t k, const
     g.pos[j] = pos[j] - 1;
     g.img[j] = static_cast<uint8_t>(img[j]);
   }
-  g.moved = 1;
   for (uint32_t j = 0; j < k; j++) {
     g.act |= 1u << bit_of[qubits[j]];
     g.m[bit_of[qubits[j]]] = all[j];
   }
   const uint64_t nsites = 1ull << (n - 6 - fill);
-  return fill == 6 ? launch_group_blk<2, false>(st, nsites, g, cls, s)
-                   : launch_group_blk<3, false>(st, nsites, g, cls, s);
+  return fill == 6 ? launch_group_blk<2, false, true>(st, nsites, g, cls, s)
+                   : launch_group_blk<3, false, true>(st, nsites, g, cls, s);
 }
 
 extern "C" int qmk_apply_blocked(float *state, uint32_t n, uint32_t b,
