@@ -164,7 +164,8 @@ size_t qm_circuit_plan_export(qm_circuit c, int collapse_1q_windows,
 
 /* The executor's launch schedules, computed on the host only (no device
  * needed), in a flat double layout:
- *   which = 0: the merged forward pass of the default plan (qm_run_merged);
+ *   which = 0: the merged forward pass of the default plan (gradients, and
+ *              qm_run_merged unless which = 3 moves fewer bytes);
  *   which = 1: the block-wise backward sweep (qm_energy_and_gradient) with
  *              `tile_high` wires >= 6 per window pass (1..6);
  *   which = 2: the co-state lambda = H psi of `h` for the circuit's width;
@@ -174,7 +175,8 @@ size_t qm_circuit_plan_export(qm_circuit c, int collapse_1q_windows,
  * Forward steps: 0 group (nw, then wire and a row-major 2x2 as re/im pairs per
  * wire), 1 gather (n, cols[n], off, nops, plan op indices), 2 plan op (index),
  * 3 group with CX / SWAP gates after it (nw and its matrices as 0, then ngates
- * and swap 0/1, a, b per gate). Backward steps: 0 window tile (nops, then wire, inverse 2x2, generator 0-3,
+ * and swap 0/1, a, b per gate), 4 stages (ns, then wire, has matrix, its 2x2, phase
+ * 0 none / 1 after / 2 before the 2x2, and n angles per stage). Backward steps: 0 window tile (nops, then wire, inverse 2x2, generator 0-3,
  * gradient slot per op), 1 diagonal block (undo, nt, (mask, angle) x nt,
  * global phase, ng, (Z mask, slot) x ng), 2 gather undo (n, cols[n], off,
  * ngates, gate indices), 3 gate undo (index). Co-state steps: 0 Z strings

@@ -176,6 +176,23 @@ int qmk_run_small(float *state, uint32_t n, size_t num_ops,
                   const qmk_small_op *ops, const qmk_small_adjoint *adjoint,
                   void *workspace, size_t workspace_bytes, void *stream);
 
+/* Stages in one in-place pass, in order, n >= 13. A stage is a 2x2 on its wire
+ * (has_matrix) and a fan of controlled phases from it (phase 1: after the 2x2,
+ * 2: before it): amplitudes with the wire set are multiplied by e^{i f}, f the
+ * sum of angles[w] over the wires w that are set, its own among them (n
+ * entries). The wires are distinct: up to seven >= 6, or up to four >= 6 and
+ * then any of 0..5. Serves apply_1q and apply_diagonal_layer dispatches
+ * (simulator.mm:453-463, 559-592). */
+typedef struct {
+  uint32_t wire;
+  uint32_t has_matrix, phase;
+  float m[8];
+  float m_lo;             /* what m[0] lacks; used where m is m[0] times a Hadamard's signs */
+  const double *angles;
+} qmk_stage;
+int qmk_apply_stages(float *state, uint32_t n, uint32_t count,
+                     const qmk_stage *stages, void *stream);
+
 /* Returned when a size exceeds a fixed capacity (nothing is launched). */
 #define QMK_ERR_TOO_LARGE (-2)
 

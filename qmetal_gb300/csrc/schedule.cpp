@@ -356,6 +356,75 @@ std::vector<ForwardStep> move_passes(const WireRun &held, const std::vector<Perm
 
 }  // namespace
 
+namespace {
+
+// The wires every mask of a diagonal layer holds, if it is a fan: one or two
+// wires a mask, no constant phase. 0 otherwise.
+uint64_t fan_centres(const PlanOp &op, uint32_t n) {
+  if (op.kind != PlanOp::Kind::DiagonalLayer || op.global_phase != 0.0 || op.masks.empty() ||
+      op.angles.size() != op.masks.size())
+    return 0;
+  uint64_t common = ~0ull;
+  for (uint64_t m : op.masks) {
+    if (popc(m) < 1 || popc(m) > 2 || (m >> n)) return 0;
+    common &= m;
+  }
+  return common;
+}
+
+// The longest pass of stages from plan op `first` on. Returns the plan ops it
+// takes, 0 where they are better off by themselves.
+size_t match_stages(const Plan &p, size_t first, ForwardStep &step) {
+  const uint32_t n = p.num_qubits;
+  step = ForwardStep{};
+  step.kind = ForwardStep::Stages;
+  std::vector<Stage> &st = step.stages;
+  uint64_t held = 0;
+  uint32_t high = 0;
+  bool low = false;
+  double alone = 0.0;   // in S
+  auto open = [&](uint32_t w) {
+    if ((held >> w) & 1ull) return false;
+    if (w >= 6 ? low || high == 7 : high > 4) return false;
+    held |= 1ull << w;
+    if (w >= 6) high++;
+    else low = true;
+    st.emplace_back();
+    st.back().wire = w;
+    return true;
+  };
+  size_t k = first;
+  for (; k < p.ops.size(); k++) {
+    const PlanOp &op = p.ops[k];
+    if (op.kind == PlanOp::Kind::Dense1q) {
+      const uint32_t w = op.qubits[0];
+      if (w >= n) break;
+      const bool joins = !st.empty() && st.back().wire == w && !st.back().has_matrix;
+      if (!joins && !open(w)) break;
+      st.back().has_matrix = true;
+      std::copy(op.matrix, op.matrix + 4, st.back().m);
+      alone += 2.0;
+      continue;
+    }
+    const uint64_t centres = fan_centres(op, n);
+    if (!centres) break;
+    const bool after = !st.empty() && st.back().phase == 0 && ((centres >> st.back().wire) & 1ull);
+    if (!after && !open(static_cast<uint32_t>(63 - __builtin_clzll(centres)))) break;
+    Stage &s = st.back();
+    s.phase = after ? 1 : 2;
+    s.angles.assign(n, 0.0);
+    for (size_t t = 0; t < op.masks.size(); t++) {
+      const uint64_t other = op.masks[t] & ~(1ull << s.wire);
+      s.angles[other ? static_cast<uint32_t>(__builtin_ctzll(other)) : s.wire] += op.angles[t];
+    }
+    alone += op.masks.size() == 1 ? 0.5 : 1.0;
+  }
+  for (size_t i = first; i < k; i++) step.ops.push_back(i);
+  return alone >= 4.0 && st.size() >= 2 ? k - first : 0;
+}
+
+}  // namespace
+
 std::vector<ForwardStep> inplace_schedule(const Plan &p) {
   const uint32_t n = p.num_qubits;
   std::vector<ForwardStep> out;
@@ -388,6 +457,16 @@ std::vector<ForwardStep> inplace_schedule(const Plan &p) {
   };
   for (size_t i = 0; i < p.ops.size(); i++) {
     const PlanOp &op = p.ops[i];
+    ForwardStep stages;
+    if (n >= kStagesMinQubits && i + 1 < p.ops.size() &&
+        (op.kind == PlanOp::Kind::Dense1q || op.kind == PlanOp::Kind::DiagonalLayer)) {
+      if (const size_t taken = match_stages(p, i, stages)) {
+        flush();
+        out.push_back(std::move(stages));
+        i += taken - 1;
+        continue;
+      }
+    }
     if (is_wire_move(op, n)) {
       run.push_back({op.kind == PlanOp::Kind::Swap, op.qubits[0], op.qubits[1]});
       run_ops.push_back(i);
@@ -410,6 +489,23 @@ std::vector<ForwardStep> inplace_schedule(const Plan &p) {
   }
   flush();
   return out;
+}
+
+double schedule_cost(const Plan &p, const std::vector<ForwardStep> &steps) {
+  double cost = 0.0;
+  for (const ForwardStep &st : steps) {
+    if (st.kind == ForwardStep::Stages) {
+      cost += 2.7;
+    } else if (st.kind != ForwardStep::Op) {
+      cost += 2.0;
+    } else {
+      const PlanOp &op = p.ops[st.ops[0]];
+      const bool half = op.kind == PlanOp::Kind::Controlled1q || op.kind == PlanOp::Kind::Swap ||
+                        fan_centres(op, p.num_qubits) != 0;
+      cost += op.kind == PlanOp::Kind::CCX ? 0.5 : half ? 1.0 : 2.0;
+    }
+  }
+  return cost;
 }
 
 // ---------------------------------------------------------------------------
@@ -982,6 +1078,15 @@ void serialise_schedule(const std::vector<ForwardStep> &s, uint32_t n, std::vect
           v.push_back(m.a);
           v.push_back(m.b);
         }
+      }
+    } else if (st.kind == ForwardStep::Stages) {
+      v.push_back(static_cast<double>(st.stages.size()));
+      for (const Stage &s : st.stages) {
+        v.push_back(s.wire);
+        v.push_back(s.has_matrix ? 1.0 : 0.0);
+        put_mat(v, s.m);
+        v.push_back(s.phase);
+        for (uint32_t w = 0; w < n; w++) v.push_back(s.phase ? s.angles[w] : 0.0);
       }
     } else if (st.kind == ForwardStep::Permute) {
       put_map(v, n, st.cols, st.off);

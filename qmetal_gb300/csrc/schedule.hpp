@@ -43,12 +43,23 @@ bool permutation_pays(const Affine &m, size_t gates);
 
 // --- merged forward --------------------------------------------------------
 
+// A 2x2 on a wire and a fan of controlled phases from it: amplitudes with the
+// wire set are multiplied by e^{i f}, f the sum of angles over the set wires.
+struct Stage {
+  uint32_t wire = 0;
+  bool has_matrix = false;
+  uint32_t phase = 0;            // 0: none, 1: after the 2x2, 2: before it
+  cdouble m[4];
+  std::vector<double> angles;    // one per wire where there is a phase
+};
+
 struct ForwardStep {
-  enum Kind : uint8_t { Group, Permute, Op, Moves };
+  enum Kind : uint8_t { Group, Permute, Op, Moves, Stages };
   Kind kind = Op;
   std::vector<uint32_t> wires;   // Group / Moves: ascending, distinct
   std::vector<cdouble> mats;     // Group / Moves: one row-major 2x2 per wire
   std::vector<PermGate> moves;   // Moves: CX / SWAP gates after the 2x2s, in order
+  std::vector<Stage> stages;     // Stages: in order
   std::vector<uint64_t> cols;    // Permute: gather map
   uint64_t off = 0;
   // Op: the one plan op to apply. Permute: the run's plan ops, applied one
@@ -71,8 +82,19 @@ std::vector<ForwardStep> merged_schedule(const Plan &p);
 // >= 6, or up to seven wires >= 6; it needs kMovesMinQubits. An HEA layer of
 // 30 wires and its ladder go as five passes (10 S) instead of eight groups
 // and 29 CX (45 S): three layers and the 60 terms of their Hamiltonian 187 -> 57 ms.
+//
+// Single gates alternating with diagonal layers whose masks share a wire (the
+// stages of a Fourier transform) go as one pass for up to seven stages on
+// wires >= 6, or up to four and then up to six on wires 0..5, from two stages
+// on: alone a stage costs 2 S for its gate and S for its fan, the pass 2 S to
+// 3 S in time.
 constexpr uint32_t kMovesMinQubits = 13;
+constexpr uint32_t kStagesMinQubits = 13;
 std::vector<ForwardStep> inplace_schedule(const Plan &p);
+
+// What a schedule of p moves, in states read or written (S bytes each; a pass
+// of stages counts 2.7 S for its multiply-adds).
+double schedule_cost(const Plan &p, const std::vector<ForwardStep> &steps);
 
 // The plan for a state that one block holds: one-qubit ops three wires a
 // step, every run of CX / SWAP ops as one gather, other ops as they are.
@@ -166,6 +188,7 @@ int generator_of(const Gate &g);
 //     1 (Permute) n, cols[n], off, nops, ops[nops]
 //     2 (Op)      op
 //     3 (Moves)   nw, (wire, m00.re, ..) x nw, ngates, (swap, a, b) x ngates
+//     4 (Stages)  ns, (wire, has matrix, m00.re, .., phase, angle x n) x ns
 //   co-state: [steps] then per step
 //     0 (ZDiag)   nt, (zmask, coeff) x nt
 //     1 (Local)   overwrite, nt, (wire, sign, ny, coeff) x nt

@@ -493,8 +493,28 @@ void Simulator::run_inplace(const Plan &p) {
   }
   for (const ForwardStep &st : inplace_schedule(p)) {
     if (st.kind == ForwardStep::Op) apply_op_to(state_, p.ops[st.ops[0]]);
+    else if (st.kind == ForwardStep::Stages) apply_stages_step(st);
     else apply_group_step(st);
   }
+}
+
+void Simulator::apply_stages_step(const ForwardStep &st) {
+  std::vector<qmk_stage> stages;
+  for (const Stage &s : st.stages) {
+    qmk_stage o{};
+    o.wire = s.wire;
+    o.has_matrix = s.has_matrix;
+    o.phase = s.phase;
+    if (s.has_matrix) {
+      narrow(s.m, o.m);
+      o.m_lo = static_cast<float>(s.m[0].real() - o.m[0]);
+    }
+    o.angles = s.phase ? s.angles.data() : nullptr;
+    stages.push_back(o);
+  }
+  check(qmk_apply_stages(state_, n_, static_cast<uint32_t>(stages.size()), stages.data(), stream_),
+        "stages");
+  dispatches_++;
 }
 
 // One 2x2 per wire, then the step's moves, in one launch.
@@ -965,17 +985,25 @@ void Simulator::run_cached(const Circuit &c) {
 
 // The plan through merged_schedule(): one group pass per merged set of
 // one-qubit ops, one gather pass per CX / SWAP run that pays, the plan's op
-// kernel for everything else.
+// kernel for everything else; or through inplace_schedule() where that moves
+// less (the stages of a Fourier transform).
 void Simulator::run_merged(const Plan &p) {
   if (p.num_qubits != n_) throw std::runtime_error("plan/simulator size mismatch");
   activate();
-  if (small() && !keep_ckpts_) {
+  if (small()) {
     const uint64_t own = dispatches_;
     run_small(p);
     dispatches_ = own + 1;
     return;
   }
-  for (const ForwardStep &st : merged_schedule(p)) {
+  std::vector<ForwardStep> steps = merged_schedule(p);
+  std::vector<ForwardStep> inplace = inplace_schedule(p);
+  if (schedule_cost(p, inplace) < schedule_cost(p, steps)) steps = std::move(inplace);
+  run_steps(p, steps);
+}
+
+void Simulator::run_steps(const Plan &p, const std::vector<ForwardStep> &steps) {
+  for (const ForwardStep &st : steps) {
     switch (st.kind) {
       case ForwardStep::Group:
       case ForwardStep::Moves:
@@ -1000,6 +1028,9 @@ void Simulator::run_merged(const Plan &p) {
       }
       case ForwardStep::Op:
         apply_op_to(state_, p.ops[st.ops[0]]);
+        break;
+      case ForwardStep::Stages:
+        apply_stages_step(st);
         break;
     }
   }
@@ -1628,7 +1659,7 @@ void Simulator::fused_gradient(const Circuit &c, const Hamiltonian &h, size_t sh
   const Plan plan = build_plan(c, FusionOptions{});
   if (small() && small_gradient(c, h, plan, shots, seed)) return;
   keep_ckpts_ = checkpoints_pair(c, plan);
-  run_merged(plan);
+  run_steps(plan, merged_schedule(plan));
   keep_ckpts_ = false;
   if (shots) launch_sample(shots, seed);
   energy_and_costate(h);
@@ -1744,7 +1775,7 @@ void Simulator::serve_enqueue(const Circuit &c, const Hamiltonian &h, size_t sho
   reset();
   const Plan plan = build_plan(c, FusionOptions{});
   if (!small() || !small_gradient(c, h, plan, shots, seed)) {
-    run_merged(plan);
+    run_steps(plan, merged_schedule(plan));
     if (shots) launch_sample(shots, seed);
     energy_and_costate(h);
     sweep_fused(c);

@@ -15,11 +15,16 @@ CX, CZ, SWAP, CP = W.CX, W.CZ, W.SWAP, W.CP
 
 
 def _steps(c):
+    n = c.num_qubits
     v = c.schedule_export("inplace")
     r, out = Reader(v), []
     for _ in range(r.i()):
         kind = r.i()
-        assert kind in (0, 2, 3)
+        assert kind in (0, 2, 3, 4)
+        if kind == 4:
+            out.append(("stages", [(r.i(), r.i(), r.mat(), r.i(), [r.f() for _ in range(n)])
+                                   for _ in range(r.i())]))
+            continue
         if kind == 2:
             out.append(("op", r.i()))
             continue
@@ -38,6 +43,32 @@ def _move(st, swap, a, b):
     return out
 
 
+def _fan(n, wire, angles):
+    i = np.arange(1 << n)
+    f = sum(a * ((i >> w) & 1) for w, a in enumerate(angles))
+    return np.where((i >> wire) & 1, np.exp(1j * f), 1.0)
+
+
+def _inverse_qft(n):
+    return [(k, q, tuple(-x for x in ps)) for k, q, ps in reversed(W.qft(n))]
+
+
+def _fans(n, rng, count=30):
+    """Single gates and controlled phases from random wires, as many stages' passes meet them."""
+    gates = []
+    for _ in range(count):
+        w = int(rng.integers(n))
+        gates.append((int(rng.choice([W.H, W.RY, W.RX])), (w,), ()) if rng.integers(2) else (W.H, (w,), ()))
+        if gates[-1][0] != W.H:
+            gates[-1] = (gates[-1][0], (w,), (float(rng.uniform(-3, 3)),))
+        c = w if rng.integers(4) else int(rng.integers(n))
+        others = [int(q) for q in rng.choice(n, int(rng.integers(1, 6)), replace=False) if q != c]
+        gates += [(CP, (q, c), (float(rng.uniform(-3, 3)),)) for q in others]
+        if rng.integers(3) == 0:
+            gates.append((W.P, (c,), (0.4,)))
+    return gates
+
+
 def _replay(n, gates):
     c = W.to_circuit(n, gates)
     plan = np.array(c.plan_export())
@@ -47,6 +78,18 @@ def _replay(n, gates):
     for s in steps:
         if s[0] == "op":
             st = oracle.run_plan(n, plan_op(plan, s[1]), init=st)
+            continue
+        if s[0] == "stages":
+            wires = [x[0] for x in s[1]]
+            high = [w for w in wires if w >= 6]
+            assert n >= 13 and len(set(wires)) == len(wires) >= 2
+            assert wires[:len(high)] == high
+            assert len(high) <= (7 if len(high) == len(wires) else 4)
+            for w, has, m, phase, angles in s[1]:
+                turn = _fan(n, w, angles)
+                st = st * turn if phase == 2 else st
+                st = apply_1q(st, n, w, m) if has else st
+                st = st * turn if phase == 1 else st
             continue
         wires = [w for w, _ in s[1]]
         assert wires == sorted(set(wires))
@@ -84,7 +127,8 @@ def test_inplace_schedule(n):
     layer = [(W.RY, (q,), (0.1 + q,)) for q in range(n)]
     for gates in (W.ghz(n), W.hea(n, 2), W.qft_swap(n), W.tfim_chain(n, 2), W.random_u3(n, 2),
                   W.qaoa_ring_seeded(n, 2), layer + reverse + layer + swaps, layer + swaps + reverse,
-                  _random(n, 60, rng), _random(n, 60, rng)):
+                  _random(n, 60, rng), _random(n, 60, rng), W.qft(n) + _inverse_qft(n),
+                  _fans(n, rng), _fans(n, rng)):
         got, _ = _replay(n, gates)
         assert np.abs(got - oracle.run(n, gates)).max() <= 1e-12
 
@@ -123,3 +167,13 @@ def test_small_schedule(n):
             else:
                 st = oracle.run_plan(n, plan_op(plan, s[1]), init=st)
         assert np.abs(st - oracle.run(n, gates)).max() <= 1e-12
+
+
+@pytest.mark.parametrize("n, passes", [(13, 2), (20, 3), (28, 4), (31, 4), (33, 5)])
+def test_qft_passes(n, passes):
+    steps = _steps(W.to_circuit(n, W.qft(n)))
+    assert [s[0] for s in steps] == ["stages"] * passes
+    # the inverse meets wires 0..5 first, and may end on a stage of its own
+    steps = _steps(W.to_circuit(n, _inverse_qft(n)))
+    assert sum(s[0] == "stages" for s in steps) >= 1 + (n - 6) // 7
+    assert len(steps) <= 1 + (n - 6) // 7 + 2
