@@ -8,7 +8,7 @@
 // with an FP64 warp scan, and only the drawn indices travel to the host.
 #include <algorithm>
 
-#include "kcommon.cuh"
+#include "kreduce.cuh"
 #include "../../include/qmetal/qmetal_kernels.h"
 
 using namespace qmk;
@@ -122,7 +122,14 @@ __device__ __forceinline__ uint64_t splitmix_at(uint64_t seed, uint64_t k) {
   return z ^ (z >> 31);
 }
 
-// One warp per shot.
+// One warp per shot. The block is searched 32 ways a step (four reads deep for
+// 2^18 blocks where a binary search is eighteen), and the walk reads eight
+// 32-amplitude chunks at a time: their totals in FP32 pairs (2^-46, where a
+// block's sum carries FP32) by one transposed butterfly, then an FP64 scan of
+// the chunk that the draw falls in. Bound by the reads' latency: 4096 shots at
+// 28 qubits 130 -> 19 us.
+constexpr int kChunks = 8;
+
 __global__ void __launch_bounds__(kThreads)
 k_draw(const float2 *__restrict__ st, uint64_t dim, const double *__restrict__ cdf, uint64_t nb,
        uint64_t shots, uint64_t seed, uint64_t *__restrict__ out) {
@@ -134,43 +141,70 @@ k_draw(const float2 *__restrict__ st, uint64_t dim, const double *__restrict__ c
     if (lane == 0) out[k] = 0;
     return;
   }
-  uint64_t b = 0;
-  double rem = 0.0;
-  if (lane == 0) {
-    const double u = static_cast<double>(splitmix_at(seed, k) >> 11) *
-                     (1.0 / 9007199254740992.0) * total;
-    uint64_t lo = 0, hi = nb - 1;
-    while (lo < hi) {
-      const uint64_t mid = (lo + hi) >> 1;
-      if (cdf[mid] > u) hi = mid; else lo = mid + 1;
+  const double u =
+      static_cast<double>(splitmix_at(seed, k) >> 11) * (1.0 / 9007199254740992.0) * total;
+  // The first block whose running sum passes u, or the last.
+  uint64_t lo = 0, hi = nb - 1;
+  while (hi - lo >= 32) {
+    const uint64_t step = (hi - lo) >> 5;
+    const unsigned past = __ballot_sync(0xffffffffu, cdf[lo + (lane + 1) * step - 1] > u);
+    if (past) {
+      const uint32_t f = __ffs(past) - 1;
+      hi = lo + (f + 1) * step - 1;
+      lo += f * step;
+    } else {
+      lo += 32 * step;
     }
-    b = lo;
-    rem = u - (lo > 0 ? cdf[lo - 1] : 0.0);
   }
-  b = __shfl_sync(0xffffffffu, b, 0);
-  rem = __shfl_sync(0xffffffffu, rem, 0);
-  const uint64_t s = b * kBlock, e = min(s + kBlock, dim);
+  {
+    const unsigned past =
+        __ballot_sync(0xffffffffu, lo + lane < hi && cdf[min(lo + lane, hi)] > u);
+    lo = past ? lo + __ffs(past) - 1 : hi;
+  }
+  const double rem = u - (lo > 0 ? cdf[lo - 1] : 0.0);
+  const uint64_t s = lo * kBlock, e = min(s + kBlock, dim);
   double acc = 0.0;
-  int64_t last_nz = -1;
+  for (uint64_t c0 = s; c0 < e; c0 += 32 * kChunks) {
+    Two tot[kChunks];
+    float2 a[kChunks];
+#pragma unroll
+    for (int c = 0; c < kChunks; c++) {
+      const uint64_t i = c0 + 32 * c + lane;
+      a[c] = i < e ? st[i] : make_float2(0.0f, 0.0f);
+    }
+#pragma unroll
+    for (int c = 0; c < kChunks; c++) {
+      const float xx = a[c].x * a[c].x, yy = a[c].y * a[c].y;
+      tot[c] = add(Two{xx, fmaf(a[c].x, a[c].x, -xx)}, Two{yy, fmaf(a[c].y, a[c].y, -yy)});
+    }
+    const double mine = widen(warp_slot_sums(tot, lane));   // lane c: chunk c's total
+#pragma unroll
+    for (int c = 0; c < kChunks; c++) {
+      const double next = acc + __shfl_sync(0xffffffffu, mine, c);
+      if (next > rem) {
+        const double re = a[c].x, im = a[c].y, pr = re * re + im * im;
+        const double pre = warp_scan(pr, lane);
+        unsigned hit = __ballot_sync(0xffffffffu, acc + pre > rem);
+        if (!hit) {   // the two sums of the chunk round apart: its last amplitude that is not zero
+          const unsigned nz = __ballot_sync(0xffffffffu, pr > 0.0);
+          hit = 1u << (31 - __clz(nz | 1u));
+        }
+        if (lane == 0) out[k] = c0 + 32 * c + (__ffs(hit) - 1);
+        return;
+      }
+      acc = next;
+    }
+  }
+  // Rounding left the draw past the block's sum: its last amplitude that is not zero.
+  int64_t last = -1;
   for (uint64_t c0 = s; c0 < e; c0 += 32) {
     const uint64_t i = c0 + lane;
-    double pr = 0.0;
-    if (i < e) {
-      const float2 a = st[i];
-      const double re = a.x, im = a.y;
-      pr = re * re + im * im;
-    }
-    const double pre = warp_scan(pr, lane);
-    const unsigned hit = __ballot_sync(0xffffffffu, i < e && acc + pre > rem);
-    if (hit) {
-      if (lane == 0) out[k] = c0 + (__ffs(hit) - 1);
-      return;
-    }
-    const unsigned nz = __ballot_sync(0xffffffffu, pr > 0.0);
-    if (nz) last_nz = static_cast<int64_t>(c0 + (31 - __clz(nz)));
-    acc += __shfl_sync(0xffffffffu, pre, 31);
+    const float2 a = i < e ? st[i] : make_float2(0.0f, 0.0f);
+    const double re = a.x, im = a.y;
+    const unsigned nz = __ballot_sync(0xffffffffu, re * re + im * im > 0.0);
+    if (nz) last = static_cast<int64_t>(c0 + (31 - __clz(nz)));
   }
-  if (lane == 0) out[k] = last_nz >= 0 ? static_cast<uint64_t>(last_nz) : e - 1;
+  if (lane == 0) out[k] = last >= 0 ? static_cast<uint64_t>(last) : e - 1;
 }
 
 }  // namespace
