@@ -193,6 +193,16 @@ typedef struct {
 int qmk_apply_stages(float *state, uint32_t n, uint32_t count,
                      const qmk_stage *stages, void *stream);
 
+/* qmk_apply_diagonal (masks of at most two bits) and then one 2x2 on each of
+ * k = 1..4 ascending wires >= 13, in one pass; the same arithmetic as the two
+ * calls. */
+int qmk_apply_diagonal_group(float *state, uint32_t n, uint32_t num_terms,
+                             const uint64_t *masks, const double *angles,
+                             double global_phase, uint32_t k,
+                             const uint32_t *wires, const float *mats,
+                             void *workspace, size_t workspace_bytes,
+                             void *stream);
+
 /* Returned when a size exceeds a fixed capacity (nothing is launched). */
 #define QMK_ERR_TOO_LARGE (-2)
 

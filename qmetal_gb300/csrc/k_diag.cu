@@ -110,6 +110,109 @@ __global__ void k_diag_generic(float2 *__restrict__ st, uint64_t dim, GenericTer
   st[i] = cmul(expi_reduced(phi), st[i]);
 }
 
+// A diagonal layer and then 2x2s on K wires >= 13 in one pass. A thread holds
+// the 2^K vectors that the wires pick, one of each of 2^K tiles, so the layer's
+// table is read once for all of them and the 2x2s pair registers. The same
+// arithmetic in the same order as the layer's pass and then a group's.
+//
+// A Trotter step of 25 wires is then four passes instead of five (the layer,
+// 10 + 7 + 7 + 1 wires), a QAOA layer of 28 wires too (10 + 7 + 7 + 4). Bound by
+// the state's read and write.
+constexpr int kDiagWires = 4;
+struct DiagGroupArgs {
+  uint32_t pos[kDiagWires];   // tile-number bits (wire - 13), ascending
+  M2 m[kDiagWires];
+};
+
+template <int K, int CLS>
+__global__ void __launch_bounds__(kThreads, K == 4 ? 2 : 3)
+k_diag_group(float4 *__restrict__ st, const DiagDesc *__restrict__ d,
+             const float4 *__restrict__ table4, uint64_t nsuper, DiagGroupArgs g) {
+  constexpr int NT = 1 << K;
+  constexpr int UN = K == 1 ? 4 : K == 2 ? 2 : 1;   // vectors of each tile in flight
+  constexpr uint32_t kVecs = 1u << (kWMax - 1);
+  __shared__ float2 f[NT][kWMax];
+  __shared__ float2 eH[NT];
+  __shared__ __align__(16) float2 Y1[NT][64];
+  __shared__ float2 Y2[NT][1 << (kWMax - 6)];
+  __shared__ uint64_t off[NT];   // vector t of a thread against vector 0
+  const uint32_t tid = threadIdx.x, warp = tid >> 5;
+  if (tid < NT) {
+    uint64_t v = 0;
+#pragma unroll
+    for (int j = 0; j < K; j++)
+      if ((tid >> j) & 1u) v |= static_cast<uint64_t>(kVecs) << g.pos[j];
+    off[tid] = v;
+  }
+  for (uint64_t sup = blockIdx.x; sup < nsuper; sup += gridDim.x) {
+    uint64_t tile0 = sup;
+#pragma unroll
+    for (int j = 0; j < K; j++) tile0 = ins0(tile0, g.pos[j]);
+    auto tile_of = [&](int t) {
+      uint64_t tile = tile0;
+#pragma unroll
+      for (int j = 0; j < K; j++)
+        if ((t >> j) & 1) tile |= 1ull << g.pos[j];
+      return tile;
+    };
+    for (int t = static_cast<int>(warp); t < NT; t += kThreads / 32)
+      warp_tile_coeffs(d, tile_of(t), f[t], &eH[t]);
+    __syncthreads();
+    for (int t = 0; t < NT; t++) tile_phase_tables(kWMax, f[t], eH[t], Y1[t], Y2[t]);
+    __syncthreads();
+    float4 *row0 = st + tile0 * kVecs;
+    for (uint32_t e0 = tid; e0 < kVecs; e0 += kThreads * UN) {
+      float4 r[UN][NT], x[UN];
+#pragma unroll
+      for (int u = 0; u < UN; u++) {
+        x[u] = table4[e0 + u * kThreads];
+#pragma unroll
+        for (int t = 0; t < NT; t++) r[u][t] = row0[off[t] + e0 + u * kThreads];
+      }
+#pragma unroll
+      for (int u = 0; u < UN; u++) {
+        const uint32_t lo = 2 * (e0 + u * kThreads);
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+          const float4 y1 = *reinterpret_cast<const float4 *>(&Y1[t][lo & 63]);
+          const float2 y2 = Y2[t][lo >> 6];
+          const float2 f0 = cmul(cmul(lo2(x[u]), lo2(y1)), y2);
+          const float2 f1 = cmul(cmul(hi2(x[u]), hi2(y1)), y2);
+          r[u][t] = pack4(cmul(f0, lo2(r[u][t])), cmul(f1, hi2(r[u][t])));
+        }
+#pragma unroll
+        for (int j = 0; j < K; j++) {
+#pragma unroll
+          for (int t = 0; t < NT; t++) {
+            if ((t >> j) & 1) continue;
+            float4 &a = r[u][t], &b = r[u][t | (1 << j)];
+            float2 a0 = lo2(a), b0 = lo2(b), a1 = hi2(a), b1 = hi2(b);
+            apply2c(CLS, g.m[j], a0, b0);
+            apply2c(CLS, g.m[j], a1, b1);
+            a = pack4(a0, a1);
+            b = pack4(b0, b1);
+          }
+        }
+#pragma unroll
+        for (int t = 0; t < NT; t++) row0[off[t] + e0 + u * kThreads] = r[u][t];
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <int K>
+void launch_diag_group(int cls, float4 *st, const DiagDesc *d, const float4 *table4,
+                       uint64_t nsuper, const DiagGroupArgs &g, cudaStream_t s) {
+  const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(
+      nsuper, static_cast<uint64_t>(qmk_host::num_sms()) * (K == 4 ? 2 : 3)));
+  switch (cls) {
+    case kMatReal: k_diag_group<K, kMatReal><<<grid, kThreads, 0, s>>>(st, d, table4, nsuper, g); break;
+    case kMatRx: k_diag_group<K, kMatRx><<<grid, kThreads, 0, s>>>(st, d, table4, nsuper, g); break;
+    default: k_diag_group<K, kMatGeneral><<<grid, kThreads, 0, s>>>(st, d, table4, nsuper, g); break;
+  }
+}
+
 // One term of one to three wires and no global phase.
 bool diagonal_is_phase(uint32_t n, uint32_t nt, const uint64_t *masks, double global_phase) {
   return nt == 1 && global_phase == 0.0 && masks[0] && !(masks[0] >> n) &&
@@ -182,4 +285,45 @@ extern "C" int qmk_apply_diagonal(float *state, uint32_t n, uint32_t nt,
     if (rc) return rc;
   }
   return 0;
+}
+
+extern "C" int qmk_apply_diagonal_group(float *state, uint32_t n, uint32_t nt,
+                                        const uint64_t *masks, const double *angles,
+                                        double global_phase, uint32_t k, const uint32_t *wires,
+                                        const float *mats, void *ws, size_t ws_bytes,
+                                        void *stream) {
+  if (!state || (reinterpret_cast<uintptr_t>(state) & 15u) || n < kWMax + 1 || n > 40 ||
+      (nt && (!masks || !angles)) || k < 1 || k > static_cast<uint32_t>(kDiagWires) || !wires || !mats)
+    return -1;
+  if (!ws || ws_bytes < qmk_workspace_bytes(n)) return -1;
+  DiagGroupArgs g{};
+  bool rx = true, real = true;
+  for (uint32_t j = 0; j < k; j++) {
+    if (wires[j] < kWMax || wires[j] >= n || (j && wires[j] <= wires[j - 1])) return -1;
+    g.pos[j] = wires[j] - kWMax;
+    g.m[j] = m2_from(mats + 8 * j);
+    const M2 &m = g.m[j];
+    real = real && m.a.y == 0.0f && m.b.y == 0.0f && m.c.y == 0.0f && m.d.y == 0.0f;
+    rx = rx && m.a.y == 0.0f && m.d.y == 0.0f && m.b.x == 0.0f && m.c.x == 0.0f;
+  }
+  DiagDesc d;
+  if (build_quad_desc(n, nt, masks, angles, global_phase, d, nullptr, nullptr) != 0) return -1;
+  cudaStream_t s = (cudaStream_t)stream;
+  uint8_t *base = static_cast<uint8_t *>(ws);
+  DiagDesc *dd = reinterpret_cast<DiagDesc *>(base);
+  k_quad_prep<true><<<grid_for(1u << d.W, kPrepThreads), kPrepThreads, 0, s>>>(d, dd,
+                                                                               base + kDescBytes);
+  const int rc = launch_status();
+  if (rc) return rc;
+  const int cls = real ? kMatReal : rx ? kMatRx : kMatGeneral;
+  const uint64_t nsuper = 1ull << (n - kWMax - k);
+  float4 *st = reinterpret_cast<float4 *>(state);
+  const float4 *table = reinterpret_cast<const float4 *>(base + kDescBytes);
+  switch (k) {
+    case 1: launch_diag_group<1>(cls, st, dd, table, nsuper, g, s); break;
+    case 2: launch_diag_group<2>(cls, st, dd, table, nsuper, g, s); break;
+    case 3: launch_diag_group<3>(cls, st, dd, table, nsuper, g, s); break;
+    default: launch_diag_group<4>(cls, st, dd, table, nsuper, g, s); break;
+  }
+  return launch_status();
 }

@@ -166,6 +166,29 @@ __device__ __forceinline__ void tile_coeffs(const DiagDesc *__restrict__ d, uint
   }
 }
 
+// The same by one warp, as phases: f[r] = e^{i c_r} and *eh = e^{i h}.
+__device__ __forceinline__ void warp_tile_coeffs(const DiagDesc *__restrict__ d, uint64_t tile,
+                                                 float2 *f, float2 *eh) {
+  const uint32_t W = d->W, n = d->n, lane = threadIdx.x & 31;
+  if (lane < W) {
+    double s = 0.0;
+    const uint32_t b0 = d->nlow + d->coff[lane], b1 = d->nlow + d->coff[lane + 1];
+    for (uint32_t p = b0; p < b1; p++)
+      if (tile >> ((d->pq[p] >> 8) - W) & 1) s += d->pb[p];
+    f[lane] = expi_reduced(s);
+  }
+  double s = 0.0;
+  for (uint32_t q = W + lane; q < n; q += 32)
+    if (tile >> (q - W) & 1) s += d->a[q];
+  const uint32_t p0 = d->nlow + d->ncross, p1 = p0 + d->nhigh;
+  for (uint32_t p = p0 + lane; p < p1; p += 32) {
+    const uint32_t q = d->pq[p] & 255, r = d->pq[p] >> 8;
+    if ((tile >> (q - W) & 1) && (tile >> (r - W) & 1)) s += d->pb[p];
+  }
+  s = warp_sum(s);
+  if (lane == 0) *eh = expi_reduced(d->g + s);
+}
+
 // Factor tables of one tile: Y1[u] over low bits 0..5 (threads 0..63) and
 // Y2[e] over bits 6..W-1 (threads 64..), Y2 carrying the tile constant.
 // Complex products of the unit factors, or real sums.

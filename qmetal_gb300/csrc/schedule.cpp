@@ -488,6 +488,68 @@ std::vector<ForwardStep> inplace_schedule(const Plan &p) {
     for (size_t j = 0; j < count; j++) held.add(w[j], m + 4 * j);
   }
   flush();
+  return fold_diagonals(p, std::move(out));
+}
+
+std::vector<ForwardStep> fold_diagonals(const Plan &p, std::vector<ForwardStep> steps) {
+  const uint32_t n = p.num_qubits;
+  if (n <= kDiagGroupMinWire) return steps;
+  auto layer = [&](const ForwardStep &st) {
+    if (st.kind != ForwardStep::Op) return false;
+    const PlanOp &op = p.ops[st.ops[0]];
+    if (op.kind != PlanOp::Kind::DiagonalLayer || op.masks.empty() ||
+        op.angles.size() != op.masks.size() || fan_centres(op, n))
+      return false;
+    for (uint64_t m : op.masks)
+      if ((m >> n) || popc(m) > 2) return false;
+    return op.masks.size() > 1 || op.global_phase != 0.0;   // (one term is a masked phase)
+  };
+  std::vector<ForwardStep> out;
+  for (size_t i = 0; i < steps.size(); i++) {
+    if (!layer(steps[i])) {
+      out.push_back(std::move(steps[i]));
+      continue;
+    }
+    // The group passes that follow, as far as their wires differ.
+    WireRun run;
+    size_t j = i + 1;
+    for (; j < steps.size() && steps[j].kind == ForwardStep::Group; j++) {
+      bool again = false;
+      for (uint32_t w : steps[j].wires) again = again || run.holds(w);
+      if (again) break;
+      for (size_t k = 0; k < steps[j].wires.size(); k++)
+        run.add(steps[j].wires[k], &steps[j].mats[4 * k]);
+    }
+    std::vector<size_t> order(run.wires.size());
+    for (size_t k = 0; k < order.size(); k++) order[k] = k;
+    std::sort(order.begin(), order.end(),
+              [&](size_t a, size_t b) { return run.wires[a] < run.wires[b]; });
+    size_t best = j - i - 1, take = 0;
+    std::vector<std::vector<size_t>> passes;
+    WireRun left;
+    for (size_t k = 1; k <= kDiagGroupWires && k <= order.size(); k++) {
+      if (run.wires[order[order.size() - k]] < kDiagGroupMinWire) break;
+      WireRun rest;
+      for (size_t m = 0; m + k < order.size(); m++)
+        rest.add(run.wires[order[m]], &run.mats[4 * order[m]]);
+      auto split = split_run(n, rest);
+      if (split.size() >= best) continue;
+      best = split.size();
+      take = k;
+      passes = std::move(split);
+      left = std::move(rest);
+    }
+    if (!take) {
+      out.push_back(std::move(steps[i]));
+      continue;
+    }
+    ForwardStep s = group_step(run, {order.end() - take, order.end()});
+    s.kind = ForwardStep::DiagGroup;
+    s.ops = steps[i].ops;
+    out.push_back(std::move(s));
+    for (const auto &pass : passes) out.push_back(group_step(left, pass));
+    i = j - 1;
+  }
   return out;
 }
 
@@ -1065,7 +1127,9 @@ void serialise_schedule(const std::vector<ForwardStep> &s, uint32_t n, std::vect
   v.push_back(static_cast<double>(s.size()));
   for (const ForwardStep &st : s) {
     v.push_back(st.kind);
-    if (st.kind == ForwardStep::Group || st.kind == ForwardStep::Moves) {
+    if (st.kind == ForwardStep::Group || st.kind == ForwardStep::Moves ||
+        st.kind == ForwardStep::DiagGroup) {
+      if (st.kind == ForwardStep::DiagGroup) v.push_back(static_cast<double>(st.ops.at(0)));
       v.push_back(static_cast<double>(st.wires.size()));
       for (size_t i = 0; i < st.wires.size(); i++) {
         v.push_back(st.wires[i]);

@@ -54,10 +54,10 @@ struct Stage {
 };
 
 struct ForwardStep {
-  enum Kind : uint8_t { Group, Permute, Op, Moves, Stages };
+  enum Kind : uint8_t { Group, Permute, Op, Moves, Stages, DiagGroup };
   Kind kind = Op;
-  std::vector<uint32_t> wires;   // Group / Moves: ascending, distinct
-  std::vector<cdouble> mats;     // Group / Moves: one row-major 2x2 per wire
+  std::vector<uint32_t> wires;   // Group / Moves / DiagGroup: ascending, distinct
+  std::vector<cdouble> mats;     // ... one row-major 2x2 per wire
   std::vector<PermGate> moves;   // Moves: CX / SWAP gates after the 2x2s, in order
   std::vector<Stage> stages;     // Stages: in order
   std::vector<uint64_t> cols;    // Permute: gather map
@@ -91,6 +91,13 @@ std::vector<ForwardStep> merged_schedule(const Plan &p);
 constexpr uint32_t kMovesMinQubits = 13;
 constexpr uint32_t kStagesMinQubits = 13;
 std::vector<ForwardStep> inplace_schedule(const Plan &p);
+
+// The steps with up to kDiagGroupWires wires >= 13 of the groups after a
+// diagonal layer taken into the layer's pass where that saves one (25 wires:
+// the layer, then 10 + 7 + 7 + 1, becomes the layer with one wire, 10 + 7 + 7).
+constexpr uint32_t kDiagGroupWires = 4;
+constexpr uint32_t kDiagGroupMinWire = 13;
+std::vector<ForwardStep> fold_diagonals(const Plan &p, std::vector<ForwardStep> steps);
 
 // What a schedule of p moves, in states read or written (S bytes each; a pass
 // of stages counts 2.7 S for its multiply-adds).
@@ -188,6 +195,7 @@ int generator_of(const Gate &g);
 //     1 (Permute) n, cols[n], off, nops, ops[nops]
 //     2 (Op)      op
 //     3 (Moves)   nw, (wire, m00.re, ..) x nw, ngates, (swap, a, b) x ngates
+//     5 (DiagGroup) op, nw, (wire, m00.re, ..) x nw
 //     4 (Stages)  ns, (wire, has matrix, m00.re, .., phase, angle x n) x ns
 //   co-state: [steps] then per step
 //     0 (ZDiag)   nt, (zmask, coeff) x nt

@@ -494,8 +494,21 @@ void Simulator::run_inplace(const Plan &p) {
   for (const ForwardStep &st : inplace_schedule(p)) {
     if (st.kind == ForwardStep::Op) apply_op_to(state_, p.ops[st.ops[0]]);
     else if (st.kind == ForwardStep::Stages) apply_stages_step(st);
+    else if (st.kind == ForwardStep::DiagGroup) apply_diag_group_step(p, st);
     else apply_group_step(st);
   }
+}
+
+void Simulator::apply_diag_group_step(const Plan &p, const ForwardStep &st) {
+  const PlanOp &op = p.ops[st.ops[0]];
+  const uint32_t k = static_cast<uint32_t>(st.wires.size());
+  std::vector<float> fm(8 * k);
+  for (uint32_t i = 0; i < k; i++) narrow(&st.mats[4 * i], &fm[8 * i]);
+  check(qmk_apply_diagonal_group(state_, n_, static_cast<uint32_t>(op.masks.size()),
+                                 op.masks.data(), op.angles.data(), op.global_phase, k,
+                                 st.wires.data(), fm.data(), ws_, ws_bytes_, stream_),
+        "diagonal layer");
+  dispatches_ += 2;
 }
 
 void Simulator::apply_stages_step(const ForwardStep &st) {
@@ -996,7 +1009,7 @@ void Simulator::run_merged(const Plan &p) {
     dispatches_ = own + 1;
     return;
   }
-  std::vector<ForwardStep> steps = merged_schedule(p);
+  std::vector<ForwardStep> steps = fold_diagonals(p, merged_schedule(p));
   std::vector<ForwardStep> inplace = inplace_schedule(p);
   if (schedule_cost(p, inplace) < schedule_cost(p, steps)) steps = std::move(inplace);
   run_steps(p, steps);
@@ -1031,6 +1044,9 @@ void Simulator::run_steps(const Plan &p, const std::vector<ForwardStep> &steps) 
         break;
       case ForwardStep::Stages:
         apply_stages_step(st);
+        break;
+      case ForwardStep::DiagGroup:
+        apply_diag_group_step(p, st);
         break;
     }
   }
@@ -1659,7 +1675,7 @@ void Simulator::fused_gradient(const Circuit &c, const Hamiltonian &h, size_t sh
   const Plan plan = build_plan(c, FusionOptions{});
   if (small() && small_gradient(c, h, plan, shots, seed)) return;
   keep_ckpts_ = checkpoints_pair(c, plan);
-  run_steps(plan, merged_schedule(plan));
+  run_steps(plan, fold_diagonals(plan, merged_schedule(plan)));
   keep_ckpts_ = false;
   if (shots) launch_sample(shots, seed);
   energy_and_costate(h);
@@ -1775,7 +1791,7 @@ void Simulator::serve_enqueue(const Circuit &c, const Hamiltonian &h, size_t sho
   reset();
   const Plan plan = build_plan(c, FusionOptions{});
   if (!small() || !small_gradient(c, h, plan, shots, seed)) {
-    run_steps(plan, merged_schedule(plan));
+    run_steps(plan, fold_diagonals(plan, merged_schedule(plan)));
     if (shots) launch_sample(shots, seed);
     energy_and_costate(h);
     sweep_fused(c);

@@ -141,6 +141,7 @@ class Simulator {
   void apply_dense_1q(float *state, uint32_t q, const cdouble *m);
   void apply_group_step(const ForwardStep &st);
   void apply_stages_step(const ForwardStep &st);
+  void apply_diag_group_step(const Plan &p, const ForwardStep &st);
   void run_inplace(const Plan &p);
   void run_steps(const Plan &p, const std::vector<ForwardStep> &steps);   // merged_schedule's
   void run_small(const Plan &p);

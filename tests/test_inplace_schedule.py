@@ -20,7 +20,8 @@ def _steps(c):
     r, out = Reader(v), []
     for _ in range(r.i()):
         kind = r.i()
-        assert kind in (0, 2, 3, 4)
+        assert kind in (0, 2, 3, 4, 5)
+        op = r.i() if kind == 5 else None
         if kind == 4:
             out.append(("stages", [(r.i(), r.i(), r.mat(), r.i(), [r.f() for _ in range(n)])
                                    for _ in range(r.i())]))
@@ -30,7 +31,7 @@ def _steps(c):
             continue
         mats = [(r.i(), r.mat()) for _ in range(r.i())]
         moves = [(r.i(), r.i(), r.i()) for _ in range(r.i())] if kind == 3 else []
-        out.append(("moves" if kind == 3 else "group", mats, moves))
+        out.append(({0: "group", 3: "moves", 5: "diag"}[kind], mats, moves, op))
     assert r.p == len(v)
     return out
 
@@ -93,6 +94,9 @@ def _replay(n, gates):
             continue
         wires = [w for w, _ in s[1]]
         assert wires == sorted(set(wires))
+        if s[0] == "diag":
+            assert 1 <= len(wires) <= 4 and wires[0] >= 13
+            st = oracle.run_plan(n, plan_op(plan, s[3]), init=st)
         for w, m in s[1]:
             st = apply_1q(st, n, w, m)
         if s[0] == "moves":
@@ -119,7 +123,7 @@ def _random(n, count, rng):
     return gates
 
 
-@pytest.mark.parametrize("n", [5, 11, 12, 13, 14])
+@pytest.mark.parametrize("n", [5, 11, 12, 13, 14, 18])
 def test_inplace_schedule(n):
     rng = np.random.default_rng(40 + n)
     reverse = [(CX, (q + 1, q), ()) for q in reversed(range(n - 1))]
@@ -177,3 +181,10 @@ def test_qft_passes(n, passes):
     steps = _steps(W.to_circuit(n, _inverse_qft(n)))
     assert sum(s[0] == "stages" for s in steps) >= 1 + (n - 6) // 7
     assert len(steps) <= 1 + (n - 6) // 7 + 2
+
+
+@pytest.mark.parametrize("n, passes", [(14, 3), (18, 3), (21, 3), (25, 4), (28, 4), (30, 5)])
+def test_layer_passes(n, passes):
+    steps = _steps(W.to_circuit(n, W.tfim_chain(n, 1)))
+    assert len(steps) == passes
+    assert sorted(w for s in steps if s[0] != "op" for w, _ in s[1]) == list(range(n))
