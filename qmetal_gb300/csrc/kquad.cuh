@@ -227,12 +227,12 @@ __device__ __forceinline__ void tile_real_tables(uint32_t W, const float *c, flo
 }
 
 // Up to 19 qubits there are fewer tiles than multiprocessors: each is then
-// shared out among 2^bits blocks, of at least 256 vectors each, which form its
-// factors for themselves.
-inline uint32_t tile_part_bits(uint64_t ntiles, uint32_t vec_bits) {
+// shared out among 2^bits blocks, of at least 2^least (256) vectors each, which
+// form its factors for themselves.
+inline uint32_t tile_part_bits(uint64_t ntiles, uint32_t vec_bits, uint32_t least = 8) {
   uint32_t bits = 0;
   while ((ntiles << (bits + 1)) <= 2 * static_cast<uint64_t>(qmk_host::num_sms()) &&
-         vec_bits - bits > 8)
+         vec_bits > least + bits)
     bits++;
   return bits;
 }
