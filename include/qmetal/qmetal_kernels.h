@@ -180,7 +180,7 @@ int qmk_run_small(float *state, uint32_t n, size_t num_ops,
  * (has_matrix) and a fan of controlled phases from it (phase 1: after the 2x2,
  * 2: before it): amplitudes with the wire set are multiplied by e^{i f}, f the
  * sum of angles[w] over the wires w that are set, its own among them (n
- * entries). The wires are distinct: up to seven >= 6, or up to four >= 6 and
+ * finite entries). The wires are distinct: up to seven >= 6, or up to four >= 6 and
  * then any of 0..5. Serves apply_1q and apply_diagonal_layer dispatches
  * (simulator.mm:453-463, 559-592). */
 typedef struct {

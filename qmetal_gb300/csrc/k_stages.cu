@@ -450,6 +450,8 @@ extern "C" int qmk_apply_stages(float *state, uint32_t n, uint32_t count, const 
   for (uint32_t k = 0; k < count; k++) {
     const qmk_stage &o = stages[k];
     if (o.wire >= n || ((seen >> o.wire) & 1ull) || o.phase > 2 || (o.phase && !o.angles)) return -1;
+    for (uint32_t w = 0; o.phase && w < n; w++)
+      if (!std::isfinite(o.angles[w])) return -1;
     seen |= 1ull << o.wire;
     if (o.wire >= 6) {
       if (nhigh != k) return -1;   // wires >= 6 come first

@@ -2,6 +2,7 @@
 #include "schedule.hpp"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <map>
 #include <stdexcept>
@@ -359,14 +360,15 @@ std::vector<ForwardStep> move_passes(const WireRun &held, const std::vector<Perm
 namespace {
 
 // The wires every mask of a diagonal layer holds, if it is a fan: one or two
-// wires a mask, no constant phase. 0 otherwise.
+// wires a mask, finite angles, no constant phase. 0 otherwise.
 uint64_t fan_centres(const PlanOp &op, uint32_t n) {
   if (op.kind != PlanOp::Kind::DiagonalLayer || op.global_phase != 0.0 || op.masks.empty() ||
       op.angles.size() != op.masks.size())
     return 0;
   uint64_t common = ~0ull;
-  for (uint64_t m : op.masks) {
-    if (popc(m) < 1 || popc(m) > 2 || (m >> n)) return 0;
+  for (size_t t = 0; t < op.masks.size(); t++) {
+    const uint64_t m = op.masks[t];
+    if (popc(m) < 1 || popc(m) > 2 || (m >> n) || !std::isfinite(op.angles[t])) return 0;
     common &= m;
   }
   return common;

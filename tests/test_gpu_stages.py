@@ -105,7 +105,8 @@ def test_refused():
                       (14, [(3, m, 0, None)] * 2), (14, [(0, m, 0, None), (6, m, 0, None)]),
                       (14, [(w, m, 0, None) for w in range(6, 14)]),
                       (14, [(w, m, 0, None) for w in (6, 7, 8, 9, 10, 0)]),
-                      (14, [(2, m, 3, ok)]), (14, [(2, m, 1, None)])):
+                      (14, [(2, m, 3, ok)]), (14, [(2, m, 1, None)]),
+                      (14, [(2, m, 1, ok[:13] + [float("inf")])])):
         rc, got = _run(n, psi, stages)
         assert rc == -1
         assert np.array_equal(got, psi)

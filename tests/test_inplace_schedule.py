@@ -188,3 +188,13 @@ def test_layer_passes(n, passes):
     steps = _steps(W.to_circuit(n, W.tfim_chain(n, 1)))
     assert len(steps) == passes
     assert sorted(w for s in steps if s[0] != "op" for w, _ in s[1]) == list(range(n))
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_angles_without_a_value_stay_diagonal_layers(bad):
+    gates = [(k, q, (bad,) if q == (3, 9) else ps) for k, q, ps in W.qft(14)]
+    steps = _steps(W.to_circuit(14, gates))
+    assert any(s[0] == "op" for s in steps)
+    for s in steps:
+        if s[0] == "stages":
+            assert np.isfinite([a for x in s[1] for a in x[4]]).all()
