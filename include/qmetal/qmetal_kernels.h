@@ -120,7 +120,7 @@ int qmk_apply_diagonal(float *state, uint32_t n, uint32_t num_terms,
  * and with `adjoint` also
  *   both        the op on the state and the co-state
  *   save k      MAP: keep the state from before it as number k (from 1, up to
- *               QMK_SMALL_MAX_SAVES); with `both`: the state comes from number
+ *               qmk_small_saves(n)); with `both`: the state comes from number
  *               k, and only the co-state through the map
  *   COSTATE     lambda = H psi and the energy: layer's Z strings with their
  *               coefficients as angles, then num_items strings of (x|y, y|z, Y
@@ -135,7 +135,6 @@ int qmk_apply_diagonal(float *state, uint32_t n, uint32_t num_terms,
  * (kernels.metal:48-218, 313-408). */
 #define QMK_SMALL_MAX_QUBITS 13
 #define QMK_SMALL_MAX_TERMS 3000   /* per op */
-#define QMK_SMALL_MAX_SAVES 32
 #define QMK_SMALL_MAX_WINDOW 24
 enum {
   QMK_SMALL_GROUP = 0,
@@ -172,6 +171,7 @@ typedef struct {
   double *energy;       /* device */
 } qmk_small_adjoint;
 size_t qmk_small_workspace_bytes(uint32_t n);
+uint32_t qmk_small_saves(uint32_t n);
 int qmk_run_small(float *state, uint32_t n, size_t num_ops,
                   const qmk_small_op *ops, const qmk_small_adjoint *adjoint,
                   void *workspace, size_t workspace_bytes, void *stream);

@@ -35,8 +35,12 @@ using qmk_host::launch_status;
 namespace {
 
 constexpr uint32_t kMaxN = QMK_SMALL_MAX_QUBITS;
-constexpr uint32_t kMaxLayers = 32;        // phase tables per launch
-constexpr uint32_t kMaxSaves = QMK_SMALL_MAX_SAVES;
+// Phase tables per launch and states kept: what fits with the rest of a
+// simulator's workspace in 2 MiB, the device's allocation unit (a second one
+// takes 35 us of a simulator's creation).
+constexpr uint32_t kMaxLayers = 32;
+constexpr uint32_t layers_of(uint32_t n) { return n >= 13 ? 16 : kMaxLayers; }
+constexpr uint32_t saves_of(uint32_t n) { return n >= 13 ? 8 : n >= 12 ? 16 : 32; }
 // Widest blocks: eight amplitudes a thread at 13 qubits, sixteen of each state
 // with the co-state.
 constexpr unsigned kSmallThreads = 1024, kSmallThreads2 = 512;
@@ -669,8 +673,10 @@ void put(std::vector<uint32_t> &code, const float *f, int count) {
 }  // namespace
 
 extern "C" size_t qmk_small_workspace_bytes(uint32_t n) {
-  return n >= 1 && n <= kMaxN ? (sizeof(float2) << n) * (kMaxLayers + kMaxSaves) : 0;
+  return n >= 1 && n <= kMaxN ? (sizeof(float2) << n) * (layers_of(n) + saves_of(n)) : 0;
 }
+
+extern "C" uint32_t qmk_small_saves(uint32_t n) { return n >= 1 && n <= kMaxN ? saves_of(n) : 0; }
 
 // Checks of one op; two: the ops that need the co-state are allowed.
 static bool small_op_ok(const qmk_small_op &o, uint32_t n, bool two) {
@@ -694,7 +700,7 @@ static bool small_op_ok(const qmk_small_op &o, uint32_t n, bool two) {
     case QMK_SMALL_CONTROLLED:
       return o.q[0] < n && !(o.mask >> n) && !((o.mask >> o.q[0]) & 1ull) && o.mats;
     case QMK_SMALL_MAP:
-      if (!o.cols || o.save > kMaxSaves) return false;
+      if (!o.cols || o.save > saves_of(n)) return false;
       for (uint32_t j = 0; j < n; j++)
         if (o.cols[j] >> n) return false;
       return true;
@@ -751,7 +757,7 @@ extern "C" int qmk_run_small(float *state, uint32_t n, size_t num_ops, const qmk
   SmallOut out{};
   if (adjoint)
     out = {reinterpret_cast<float2 *>(adjoint->costate), adjoint->grad, adjoint->energy,
-           tables + (static_cast<size_t>(kMaxLayers) << n)};
+           tables + (static_cast<size_t>(layers_of(n)) << n)};
   std::vector<uint32_t> code;
   std::vector<qmk_phase_layer> layers;
   uint32_t terms = 0, real = 0;
@@ -777,7 +783,7 @@ extern "C" int qmk_run_small(float *state, uint32_t n, size_t num_ops, const qmk
            !(((real >> l) & 1u) == (is_real ? 1u : 0u) && same_layer(layers[l], layer)))
       l++;
     if (l == layers.size()) {
-      if (l == kMaxLayers || terms + layer.num_terms > static_cast<uint32_t>(kLongTerms)) {
+      if (l == layers_of(n) || terms + layer.num_terms > static_cast<uint32_t>(kLongTerms)) {
         if (const int rc = flush()) return rc;
         l = 0;
       }

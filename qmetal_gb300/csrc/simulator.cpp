@@ -809,8 +809,8 @@ void Simulator::run_small(const Plan &p) {
 // Forward pass, samples, co-state and backward sweep of a gradient on a narrow
 // state: one launch (two with samples), through small_schedule and
 // backward_schedule. Every map of the forward pass keeps the state from before
-// it, which the sweep takes back instead of undoing the map on it, where the
-// two schedules' maps pair up one to one. False, with nothing launched, for a
+// it (the last ones, as there is room), which the sweep takes back instead of
+// undoing the map on it, where the two schedules' maps pair up one to one. False, with nothing launched, for a
 // circuit that the launch cannot take.
 bool Simulator::small_gradient(const Circuit &c, const Hamiltonian &h, const Plan &plan,
                                size_t shots, uint64_t seed) {
@@ -851,17 +851,19 @@ bool Simulator::small_gradient(const Circuit &c, const Hamiltonian &h, const Pla
     if (st.kind == ForwardStep::Permute) kept.push_back(&st.cols);
   for (const Undo &u : undos)
     if (!u.step) undone.push_back(&u.cols);
-  bool pair = kept.size() == undone.size() && kept.size() <= QMK_SMALL_MAX_SAVES;
+  bool pair = kept.size() == undone.size();
   for (size_t i = 0; pair && i < kept.size(); i++)
     pair = inverts(n_, *kept[kept.size() - 1 - i], 0, *undone[i], 0);
 
+  // The last maps' states are kept, as many as there is room for.
+  const size_t room = pair ? std::min<size_t>(kept.size(), qmk_small_saves(n_)) : 0;
+  size_t ahead = kept.size();   // maps of the forward pass still to come
   SmallProgram prog(n_);
-  uint32_t saves = 0;
   for (const ForwardStep &st : fwd) {
     if (st.kind == ForwardStep::Group)
       prog.group(st.wires.data(), static_cast<uint32_t>(st.wires.size()), st.mats.data());
     else if (st.kind == ForwardStep::Permute)
-      prog.map(st.cols, pair ? ++saves : 0);
+      prog.map(st.cols, ahead-- <= room ? static_cast<uint32_t>(ahead + 1) : 0);
     else if (!prog.plan_op(plan.ops[st.ops[0]]))
       return false;
   }
@@ -869,7 +871,7 @@ bool Simulator::small_gradient(const Circuit &c, const Hamiltonian &h, const Pla
   if (!prog.costate(h)) return false;
   for (const Undo &u : undos) {
     if (!u.step) {
-      prog.map(u.cols, pair ? saves-- : 0, true);
+      prog.map(u.cols, ++ahead <= room ? static_cast<uint32_t>(ahead) : 0, true);
       continue;
     }
     const BackwardStep &st = *u.step;
