@@ -523,19 +523,30 @@ k_group_warp(float4 *__restrict__ st, uint64_t nwsites, WarpGroupArgs g) {
 }
 
 // The warp tile of wires 0..5 and four wires >= 6, with CX and SWAP gates
-// among them after the 2x2s: a linear map of the tile's ten index bits. Each
-// warp scatters its 1024 amplitudes by that map into 8 KiB of shared memory of
-// its own and reads them back in order, so the stores stay whole rows and no
-// block barrier is needed.
+// among them after the 2x2s: a linear map of the tile's ten index bits.
+//
+// DIRECT: the map leaves wire 0 as it is, and the two amplitudes that share a
+// vector after it come from one register of two lanes (a CX ladder's: wire 0
+// and 1): a shuffle of the odd ones makes the new vectors, which are stored
+// where the map puts them, a row's in halves of two rows. Otherwise each warp
+// scatters its 1024 amplitudes into 8 KiB of shared memory of its own and reads
+// them back in order. Neither needs a block barrier. ALL: every wire has a 2x2
+// (tests of each cost registers: 1305 us against 941 in the case that follows).
+// Bound by the 2x2s' multiply-adds and shuffles: at 28 qubits ten general wires
+// and their ladder take 877 us direct and 941 scattered, the 2x2s alone 904.
 struct WarpMovesArgs {
   uint32_t lact, hact;   // bit j: wire j / the j-th wire >= 6 has a 2x2
   uint32_t hpos[4];      // site-number bits (wire - 6), ascending
   M2 lm[6];
   MX hm[4];
   uint16_t img[10];      // the image of each index bit: wires 0..5, then the four
+  // DIRECT: the images of wires 1..5 and the four as vector-index bits, and the
+  // lanes that trade their odd amplitudes.
+  uint64_t to[9];
+  uint32_t trade;
 };
 
-template <int CLS>
+template <int CLS, bool DIRECT, bool ALL>
 __global__ void __launch_bounds__(kThreads, 2)
 k_group_moves(float4 *__restrict__ st, uint64_t nwsites, WarpMovesArgs g) {
   constexpr int NV = 16;
@@ -557,13 +568,13 @@ k_group_moves(float4 *__restrict__ st, uint64_t nwsites, WarpMovesArgs g) {
   Cx2 r[NV];
 #pragma unroll
   for (int l = 0; l < NV; l++) r[l] = split2(st[vec_of(l)]);
-  if (g.lact & 1u) {
+  if (ALL || (g.lact & 1u)) {
 #pragma unroll
     for (int l = 0; l < NV; l++) apply_w0x<CLS>(g.lm[0], r[l]);
   }
 #pragma unroll
   for (int q = 1; q < 6; q++) {
-    if (!((g.lact >> q) & 1u)) continue;
+    if (!ALL && !((g.lact >> q) & 1u)) continue;
     const bool one = (lane >> (q - 1)) & 1;
     const M2 m = g.lm[q];
     // own' = s own + t other: (a, b) on the wire's 0 side, (d, c) on its 1 side
@@ -581,10 +592,28 @@ k_group_moves(float4 *__restrict__ st, uint64_t nwsites, WarpMovesArgs g) {
   }
 #pragma unroll
   for (int j = 0; j < 4; j++) {
-    if (!((g.hact >> j) & 1u)) continue;
+    if (!ALL && !((g.hact >> j) & 1u)) continue;
 #pragma unroll
     for (int l = 0; l < NV; l++)
       if (!((l >> j) & 1)) applyx<CLS>(g.hm[j], r[l], r[l | (1 << j)]);
+  }
+  if (DIRECT) {
+    uint64_t at = b << 5;
+#pragma unroll
+    for (int k = 0; k < 5; k++)
+      if ((lane >> k) & 1u) at ^= g.to[k];
+    __syncwarp();   // every lane has read its vectors: their places take the new ones
+#pragma unroll
+    for (int l = 0; l < NV; l++) {
+      const float re = __shfl_xor_sync(0xffffffffu, r[l].re.y, g.trade);
+      const float im = __shfl_xor_sync(0xffffffffu, r[l].im.y, g.trade);
+      uint64_t v = at;
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if ((l >> j) & 1) v ^= g.to[5 + j];
+      st[v] = make_float4(r[l].re.x, r[l].im.x, re, im);
+    }
+    return;
   }
   float4 *mine = xw + (threadIdx.x >> 5) * NV * 32;
   float2 *amp = reinterpret_cast<float2 *>(mine);
@@ -1100,20 +1129,32 @@ extern "C" int qmk_apply_group(float *state, uint32_t n, uint32_t k,
   return launch_status();
 }
 
-template <int CLS>
-static int launch_group_moves(float4 *st, uint64_t nw, const WarpMovesArgs &g, cudaStream_t s) {
-  constexpr size_t smem = static_cast<size_t>(kThreads / 32) * 16 * 32 * sizeof(float4);
+template <int CLS, bool DIRECT, bool ALL>
+static int launch_group_moves_as(float4 *st, uint64_t nw, const WarpMovesArgs &g, cudaStream_t s) {
+  constexpr size_t smem =
+      DIRECT ? 0 : static_cast<size_t>(kThreads / 32) * 16 * 32 * sizeof(float4);
   static std::atomic<bool> opted[64];   // zero-initialised: false
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
-  if (!opted[dev]) {   // the opt-in above 48 KiB is per device
-    const cudaError_t e = cudaFuncSetAttribute(
-        k_group_moves<CLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (!DIRECT && !opted[dev]) {   // the opt-in above 48 KiB is per device
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_group_moves<CLS, DIRECT, ALL>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
     opted[dev] = true;
   }
-  k_group_moves<CLS><<<grid_for(nw, kThreads / 32), kThreads, smem, s>>>(st, nw, g);
+  k_group_moves<CLS, DIRECT, ALL><<<grid_for(nw, kThreads / 32), kThreads, smem, s>>>(st, nw, g);
   return launch_status();
+}
+
+template <int CLS>
+static int launch_group_moves(float4 *st, uint64_t nw, const WarpMovesArgs &g, bool direct,
+                              cudaStream_t s) {
+  const bool all = g.lact == 63u && g.hact == 15u;
+  if (direct) return all ? launch_group_moves_as<CLS, true, true>(st, nw, g, s)
+                         : launch_group_moves_as<CLS, true, false>(st, nw, g, s);
+  return all ? launch_group_moves_as<CLS, false, true>(st, nw, g, s)
+             : launch_group_moves_as<CLS, false, false>(st, nw, g, s);
 }
 
 extern "C" int qmk_apply_group_moves(float *state, uint32_t n, uint32_t k, const uint32_t *qubits,
@@ -1181,11 +1222,33 @@ extern "C" int qmk_apply_group_moves(float *state, uint32_t n, uint32_t k, const
       }
     }
     std::copy(img, img + 10, g.img);
+    // Wire 0 stays wire 0, and the index that the map takes to 1 has no bit of
+    // the four wires (the moves undone on 1, last first).
+    bool direct = true;
+    for (uint32_t j = 0; j < 10; j++) direct = direct && (img[j] & 1u) == (j == 0 ? 1u : 0u);
+    uint32_t from = 1;
+    for (uint32_t m = num_moves; m-- > 0;) {
+      const uint32_t a = bit_of[moves[3 * m + 1]], b = bit_of[moves[3 * m + 2]];
+      if (moves[3 * m]) {
+        const uint32_t d = ((from >> a) ^ (from >> b)) & 1u;
+        from ^= (d << a) | (d << b);
+      } else {
+        from ^= ((from >> a) & 1u) << b;
+      }
+    }
+    direct = direct && from < 64;
+    g.trade = (from >> 1) & 31u;
+    for (uint32_t j = 0; j < 9; j++) {
+      const uint32_t v = img[1 + j] >> 1;   // wires 1..5, then the four
+      g.to[j] = v & 31u;
+      for (uint32_t k = 0; k < 4; k++)
+        if ((v >> (5 + k)) & 1u) g.to[j] |= 1ull << (g.hpos[k] + 5);
+    }
     const uint64_t nw = 1ull << (n - 10);
     switch (cls) {
-      case kMatRx: return launch_group_moves<kMatRx>(st, nw, g, s);
-      case kMatReal: return launch_group_moves<kMatReal>(st, nw, g, s);
-      default: return launch_group_moves<kMatGeneral>(st, nw, g, s);
+      case kMatRx: return launch_group_moves<kMatRx>(st, nw, g, direct, s);
+      case kMatReal: return launch_group_moves<kMatReal>(st, nw, g, direct, s);
+      default: return launch_group_moves<kMatGeneral>(st, nw, g, direct, s);
     }
   }
   BlkGroupArgs g{};

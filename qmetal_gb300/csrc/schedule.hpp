@@ -81,7 +81,7 @@ std::vector<ForwardStep> merged_schedule(const Plan &p);
 // one by one. A pass with moves holds any of wires 0..5 and up to four wires
 // >= 6, or up to seven wires >= 6; it needs kMovesMinQubits. An HEA layer of
 // 30 wires and its ladder go as five passes (10 S) instead of eight groups
-// and 29 CX (45 S): three layers and the 60 terms of their Hamiltonian 187 -> 57 ms.
+// and 29 CX (45 S): three layers and the 60 terms of their Hamiltonian 187 -> 52 ms.
 //
 // Single gates alternating with diagonal layers whose masks share a wire (the
 // stages of a Fourier transform) go as one pass for up to seven stages on

@@ -72,7 +72,10 @@ def test_moves(n, cls):
     for tile in sets:
         tile = [int(q) for q in tile]
         ladder = [(0, a, b) for a, b in zip(tile, tile[1:])]
-        for moves in (ladder, ladder[::-1], _random_moves(tile, 12, rng)):
+        rows = [q for q in tile if q] or tile
+        kept = _random_moves(rows, 9, rng) if len(rows) > 1 else ladder   # wire 0 as it is
+        for moves in (ladder, ladder[::-1], _random_moves(tile, 12, rng), kept,
+                      [(0, 0, tile[-1])] + kept if 0 in tile else kept[::-1]):
             for wires in ([], tile[:1], tile[1:], tile):
                 psi = _state(n, rng)
                 mats = [_matrix(rng, cls) for _ in wires]
