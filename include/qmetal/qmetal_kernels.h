@@ -157,6 +157,7 @@ typedef struct {
   uint32_t q[3];
   uint32_t both, conj, save;
   const float *mats;
+  const float *mats_lo;      /* GROUP, WINDOW: what mats lack; may be NULL */
   uint64_t mask;
   double phase[2];
   const uint64_t *cols;

@@ -17,9 +17,9 @@
 //
 // Bound by latency: a barrier, shared-memory round trip and up to three
 // dependent 2x2s an op. The 9-qubit U3 circuit of depth 10 with its read-out:
-// 310 -> 75 us. Gradients of four HEA layers, host work and read-out in: at 6,
-// 10 and 12 qubits 213 -> 96, 233 -> 147 and 304 -> 210 us, at 13, the widest
-// a block holds with its co-state, 334 -> 278 us.
+// 310 -> 80 us; gradients of four HEA layers, host work and read-out in, at 6, 10
+// and 12 qubits 213 -> 112, 233 -> 163 and 304 -> 254 us. At 13 qubits, where one
+// block took 369 us and the launches 334, a gradient goes by launches.
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -46,13 +46,13 @@ constexpr uint32_t saves_of(uint32_t n) { return n >= 13 ? 8 : n >= 12 ? 16 : 32
 constexpr unsigned kSmallThreads = 1024, kSmallThreads2 = 512;
 // Warps beside a gradient's threads (while those are at most 256) that add up
 // the rows of partial sums, so that no working warp waits for them (6 qubits,
-// four HEA layers: 132 -> 100 us).
+// four HEA layers: 32 us less).
 constexpr unsigned kHelpers = 4;
 constexpr int kRows = 12;                  // gradients per step
 
 // The ops as words, in four sizes of kernel arguments up to their limit of
 // 32 KiB (10 qubits, four
-// HEA layers, a gradient: 177 us with two sizes, 166 with four). An op's first word and each of its
+// HEA layers, a gradient: 11 us less with four sizes than with two). An op's first word and each of its
 // matrices start on 16 bytes. The block copies them into shared memory first.
 template <int WORDS>
 struct Code {
@@ -61,6 +61,12 @@ struct Code {
 };
 constexpr int kCode1 = 960, kCode2 = 1920, kCode3 = 3840, kLongCode = 7936;
 constexpr uint32_t kOpHead = 4;   // words before an op's matrices
+// A matrix: eight words narrowed to FP32, eight of what they lack. The narrowing
+// errors of one angle add up over wires and layers, and forward and back (ten
+// qubits, eight Trotter layers: most of a gradient's 2e-6); the low parts cost a
+// few multiply-adds in a kernel that waits for latency.
+constexpr uint32_t kMatWords = 16;
+constexpr uint32_t kItemWords = kOpHead + kMatWords;
 
 // A phase layer of the first launch: merged terms and the constant.
 template <int TERMS>
@@ -120,6 +126,36 @@ __device__ __forceinline__ M2 m2(const uint32_t *w) {   // on 16 bytes
   return {lo2(a), hi2(a), lo2(b), hi2(b)};
 }
 
+// A 2x2 in two parts, of the class of its high part.
+struct M2x {
+  M2 hi, lo;
+};
+__device__ __forceinline__ M2x m2x(const uint32_t *w) { return {m2(w), m2(w + 8)}; }
+
+__device__ __forceinline__ float2 cmul_add(float2 a, float2 x, float2 c) {   // a x + c
+  return make_float2(fmaf(a.x, x.x, fmaf(-a.y, x.y, c.x)), fmaf(a.x, x.y, fmaf(a.y, x.x, c.y)));
+}
+// s u + t v, s and t of a class-CLS matrix (cmac2c's forms).
+template <int CLS>
+__device__ __forceinline__ float2 row_of(float2 s, float2 sl, float2 u, float2 t, float2 tl,
+                                         float2 v) {
+  if (CLS == kMatReal)
+    return make_float2(fmaf(s.x, u.x, fmaf(t.x, v.x, fmaf(sl.x, u.x, tl.x * v.x))),
+                       fmaf(s.x, u.y, fmaf(t.x, v.y, fmaf(sl.x, u.y, tl.x * v.y))));
+  if (CLS == kMatRx)
+    return make_float2(fmaf(s.x, u.x, fmaf(-t.y, v.y, fmaf(sl.x, u.x, -tl.y * v.y))),
+                       fmaf(s.x, u.y, fmaf(t.y, v.x, fmaf(sl.x, u.y, tl.y * v.x))));
+  if (CLS == kMatDiag) return cmul_add(s, u, cmul(sl, u));
+  return cmul_add(s, u, cmul_add(t, v, cmul_add(sl, u, cmul(tl, v))));
+}
+template <int CLS>
+__device__ __forceinline__ void apply2x(const M2x &m, float2 &u, float2 &v) {
+  const float2 nu = row_of<CLS>(m.hi.a, m.lo.a, u, m.hi.b, m.lo.b, v);
+  const float2 nv = row_of<CLS>(m.hi.d, m.lo.d, v, m.hi.c, m.lo.c, u);
+  u = nu;
+  v = nv;
+}
+
 // K 2x2s on distinct wires q[0] < q[1] < q[2]: 2^K amplitudes in registers.
 template <int K, int CLS>
 __device__ __forceinline__ void group(float2 *amp, uint32_t n, const uint32_t *w, uint32_t me,
@@ -144,10 +180,10 @@ __device__ __forceinline__ void group(float2 *amp, uint32_t n, const uint32_t *w
     }
 #pragma unroll
     for (int j = 0; j < K; j++) {
-      const M2 m = m2(w + kOpHead + 8 * j);
+      const M2x m = m2x(w + kOpHead + kMatWords * j);
 #pragma unroll
       for (int l = 0; l < (1 << K); l++)
-        if (!((l >> j) & 1)) apply2c(CLS, m, r[l], r[l | (1 << j)]);
+        if (!((l >> j) & 1)) apply2x<CLS>(m, r[l], r[l | (1 << j)]);
     }
 #pragma unroll
     for (int l = 0; l < (1 << K); l++) amp[at[l]] = r[l];
@@ -186,17 +222,17 @@ __device__ __forceinline__ float window_overlap(const float2 (&p)[1 << K], const
   return s[0] + s[1];
 }
 template <int K, int J, int CLS>
-__device__ __forceinline__ void window_apply(float2 (&p)[1 << K], float2 (&l)[1 << K], const M2 &m) {
+__device__ __forceinline__ void window_apply(float2 (&p)[1 << K], float2 (&l)[1 << K], const M2x &m) {
 #pragma unroll
   for (int k = 0; k < (1 << K); k++) {
     if ((k >> J) & 1) continue;
-    apply2c(CLS, m, p[k], p[k | (1 << J)]);
-    apply2c(CLS, m, l[k], l[k | (1 << J)]);
+    apply2x<CLS>(m, p[k], p[k | (1 << J)]);
+    apply2x<CLS>(m, l[k], l[k | (1 << J)]);
   }
 }
 template <int K, int J>
 __device__ __forceinline__ float window_op(float2 (&p)[1 << K], float2 (&l)[1 << K], uint32_t gen,
-                                           uint32_t cls, const M2 &m) {
+                                           uint32_t cls, const M2x &m) {
   float s = 0.0f;
   if (gen == 1) s = window_overlap<K, J, 1>(p, l);
   else if (gen == 2) s = window_overlap<K, J, 2>(p, l);
@@ -239,9 +275,9 @@ __device__ __forceinline__ void window(float2 *psi, float2 *lam, uint32_t n, con
     }
     uint32_t row = 0;
     for (uint32_t o = 0; o < nops; o++) {
-      const uint32_t *op = w + kOpHead + 12 * o;
+      const uint32_t *op = w + kOpHead + kItemWords * o;
       const uint32_t j = op[0] & 3u, gen = (op[0] >> 2) & 3u, cls = op[0] >> 4;
-      const M2 m = m2(op + kOpHead);
+      const M2x m = m2x(op + kOpHead);
       float v;
       if (K > 2 && j == 2) v = window_op<K, (K > 2 ? 2 : 0)>(p, l, gen, cls, m);
       else if (K > 1 && j == 1) v = window_op<K, (K > 1 ? 1 : 0)>(p, l, gen, cls, m);
@@ -263,6 +299,22 @@ __device__ __forceinline__ void window(float2 *psi, float2 *lam, uint32_t n, con
   }
 }
 
+// (h, l) (a, b) in two parts.
+__device__ __forceinline__ void times(float2 h, float2 l, float2 a, float2 b, float2 &rh,
+                                      float2 &rl) {
+  const float xx = __fmul_rn(h.x, a.x), yy = __fmul_rn(h.y, a.y);
+  const float xy = __fmul_rn(h.x, a.y), yx = __fmul_rn(h.y, a.x);
+  const float re = __fadd_rn(xx, -yy), im = __fadd_rn(xy, yx);
+  // what the products and their sum lost, then the cross terms
+  const float er = (fmaf(h.x, a.x, -xx) - fmaf(h.y, a.y, -yy)) +
+                   add(Two{xx, 0.0f}, Two{-yy, 0.0f}).lo;
+  const float ei = (fmaf(h.x, a.y, -xy) + fmaf(h.y, a.x, -yx)) +
+                   add(Two{xy, 0.0f}, Two{yx, 0.0f}).lo;
+  const float2 c = cmul_add(h, b, cmul(l, a));
+  rh = make_float2(re, im);
+  rl = make_float2(er + c.x, ei + c.y);
+}
+
 // The same where every wire has one RX (SIG 1) or RZ then RY (SIG 2), with
 // their gradients: no dispatch per op, and the wires' RZ in one go -- their
 // gradients from one Im(conj(lambda) psi) an amplitude, their undo one phase an
@@ -275,7 +327,7 @@ __device__ __forceinline__ void window_uniform(float2 *psi, float2 *lam, uint32_
   uint32_t q[K];
 #pragma unroll
   for (int j = 0; j < K; j++) q[j] = (w[0] >> (8 + 5 * j)) & 31u;
-  auto matrix = [&](int item) { return m2(w + 2 * kOpHead + 12 * item); };
+  auto matrix = [&](int item) { return m2x(w + 2 * kOpHead + kItemWords * item); };
   auto add_to = [&](int row, float v, bool first) {
     float *mine = part + row * step + me;
     *mine = first ? v : *mine + v;
@@ -312,30 +364,32 @@ __device__ __forceinline__ void window_uniform(float2 *psi, float2 *lam, uint32_
         }
         add_to(2 * j, lo - hi, first);
       }
-      float2 ph[A];
+      float2 ph[A], pl[A];   // high and low parts
 #pragma unroll
       for (int j = 0; j < K; j++) {
-        const M2 m = matrix(2 * j);
+        const M2x m = matrix(2 * j);
         if (j == 0) {
-          ph[0] = m.a;
-          ph[1] = m.d;
+          ph[0] = m.hi.a;
+          ph[1] = m.hi.d;
+          pl[0] = m.lo.a;
+          pl[1] = m.lo.d;
         } else {
 #pragma unroll
           for (int k = 0; k < (1 << j); k++) {
-            ph[k | (1 << j)] = cmul(ph[k], m.d);
-            ph[k] = cmul(ph[k], m.a);
+            times(ph[k], pl[k], m.hi.d, m.lo.d, ph[k | (1 << j)], pl[k | (1 << j)]);
+            times(ph[k], pl[k], m.hi.a, m.lo.a, ph[k], pl[k]);
           }
         }
       }
 #pragma unroll
       for (int k = 0; k < A; k++) {
-        p[k] = cmul(ph[k], p[k]);
-        l[k] = cmul(ph[k], l[k]);
+        p[k] = cmul_add(ph[k], p[k], cmul(pl[k], p[k]));
+        l[k] = cmul_add(ph[k], l[k], cmul(pl[k], l[k]));
       }
     }
 #pragma unroll
     for (int j = 0; j < K; j++) {
-      const M2 m = matrix(SIG == 2 ? 2 * j + 1 : j);
+      const M2x m = matrix(SIG == 2 ? 2 * j + 1 : j);
       float v[2] = {0.0f, 0.0f};
       int pair = 0;
 #pragma unroll
@@ -343,8 +397,8 @@ __device__ __forceinline__ void window_uniform(float2 *psi, float2 *lam, uint32_
         if ((k >> j) & 1) continue;
         const int h = k | (1 << j);
         v[pair++ & 1] += qmk_adj::overlap(SIG == 2 ? 2 : 1, p[k], p[h], l[k], l[h]);
-        apply2c(SIG == 2 ? kMatReal : kMatRx, m, p[k], p[h]);
-        apply2c(SIG == 2 ? kMatReal : kMatRx, m, l[k], l[h]);
+        apply2x<SIG == 2 ? kMatReal : kMatRx>(m, p[k], p[h]);
+        apply2x<SIG == 2 ? kMatReal : kMatRx>(m, l[k], l[h]);
       }
       add_to(SIG == 2 ? 2 * j + 1 : j, v[0] + v[1], first);
     }
@@ -422,7 +476,7 @@ k_small(float2 *__restrict__ st, uint32_t n, uint32_t step,
           else if (k == 2) group_cls<2>(x, n, w, me, step);
           else group_cls<1>(x, n, w, me, step);
         }
-        at += kOpHead + 8 * k;
+        at += kOpHead + kMatWords * k;
         break;
       }
       case kPhase: {   // amplitudes with every mask bit set, by FP32 high and low parts
@@ -528,8 +582,8 @@ k_small(float2 *__restrict__ st, uint32_t n, uint32_t step,
             else if (k == 2 && sig == 1) window_uniform<2, 1>(amp, lam, n, w, rows, me, step);
             else if (k == 2) window<2>(amp, lam, n, w, rows, me, step);
             else window<1>(amp, lam, n, w, rows, me, step);
-            add_rows(w[3], w + kOpHead + 12 * nops, 1, out.grad);
-            at += kOpHead + 12 * nops + ((w[3] + 3) & ~3u);
+            add_rows(w[3], w + kOpHead + kItemWords * nops, 1, out.grad);
+            at += kOpHead + kItemWords * nops + ((w[3] + 3) & ~3u);
             continue;
           } else if ((head & 7u) == kCostate) {
             // lambda = H psi: the Z strings' tabulated sum, then string by string.
@@ -801,6 +855,11 @@ extern "C" int qmk_run_small(float *state, uint32_t n, size_t num_ops, const qmk
                       uint32_t fourth = 0) {
     code.insert(code.end(), {head, second, third, fourth});
   };
+  auto put_matrix = [&](const qmk_small_op &o, uint32_t k) {
+    put(code, o.mats + 8 * k, 8);
+    const float none[8] = {};
+    put(code, o.mats_lo ? o.mats_lo + 8 * k : none, 8);
+  };
   // 1: one RX on every wire, 2: RZ then RY, each with its gradient; 0: any other.
   auto window_signature = [&](const qmk_small_op &o) -> uint32_t {
     const uint32_t per = o.num_items / o.count;
@@ -816,7 +875,7 @@ extern "C" int qmk_run_small(float *state, uint32_t n, size_t num_ops, const qmk
   for (size_t k = 0; k < num_ops; k++) {
     const qmk_small_op &o = ops[k];
     const uint32_t both = o.both ? kBoth : 0u;
-    const size_t need = 40 + (o.kind == QMK_SMALL_WINDOW ? 13 : 2) * static_cast<size_t>(o.num_items);
+    const size_t need = kOpHead + 3 * kMatWords + 16 + (o.kind == QMK_SMALL_WINDOW ? kItemWords + 1 : 2) * static_cast<size_t>(o.num_items);
     if (code.size() + need > static_cast<size_t>(kLongCode))
       if (const int rc = flush()) return rc;
     switch (o.kind) {
@@ -831,7 +890,7 @@ extern "C" int qmk_run_small(float *state, uint32_t n, size_t num_ops, const qmk
                         (static_cast<uint32_t>(real_m ? kMatReal : rx ? kMatRx : kMatGeneral) << 6);
         for (uint32_t j = 0; j < o.count; j++) head |= o.q[j] << (8 + 5 * j);
         start_op(head);
-        put(code, o.mats, static_cast<int>(8 * o.count));
+        for (uint32_t j = 0; j < o.count; j++) put_matrix(o, j);
         break;
       }
       case QMK_SMALL_PHASE: {
@@ -866,7 +925,7 @@ extern "C" int qmk_run_small(float *state, uint32_t n, size_t num_ops, const qmk
         for (uint32_t i = 0; i < o.num_items; i++) {
           const float *m = o.mats + 8 * i;
           start_op(o.items[3 * i] | (o.items[3 * i + 1] << 2) | (matrix_class(m) << 4));
-          put(code, m, 8);
+          put_matrix(o, i);
         }
         for (uint32_t i = 0; i < o.num_items; i++)   // each row's gradient slot
           if (o.items[3 * i + 1]) code.push_back(o.items[3 * i + 2]);

@@ -30,6 +30,8 @@ constexpr uint32_t kTermsPerPass = 16;
 constexpr uint32_t kSmallExpect = 14;    // widest state whose strings go a block each
 constexpr size_t kSmallTerms = 64;       // strings per such launch
 constexpr size_t kZTermsPerPass = 32;
+constexpr uint32_t kSmallGradient = 12;  // widest gradient in one block (four HEA layers at 13
+                                         // qubits: 369 us there, 334 by launches)
 
 cudaStream_t S(void *p) { return static_cast<cudaStream_t>(p); }
 
@@ -581,6 +583,7 @@ class SmallProgram {
     o.count = count;
     std::copy(wires, wires + count, o.q);
     o.mats = matrices(m, count);
+    o.mats_lo = low_parts(m, count, o.mats);
   }
 
   void controlled(uint64_t ctrl, uint32_t q, const cdouble *m, bool both = false) {
@@ -702,20 +705,22 @@ class SmallProgram {
     std::map<uint32_t, std::vector<const WireOp *>> by_wire;
     for (const WireOp &o : tile) by_wire[o.wire].push_back(&o);
     std::vector<uint32_t> wires, items;
-    std::vector<float> mats;
+    std::vector<cdouble> mats;
     uint32_t grads = 0;
     auto flush = [&]() {
       if (items.empty()) return;
-      words_.push_back(std::move(items));
-      floats_.push_back(std::move(mats));
-      items.clear();
+      const float *hi = matrices(mats.data(), mats.size() / 4);
+      const float *lo = low_parts(mats.data(), mats.size() / 4, hi);
       mats.clear();
+      words_.push_back(std::move(items));
+      items.clear();
       qmk_small_op &o = add(QMK_SMALL_WINDOW, false);
       o.count = static_cast<uint32_t>(wires.size());
       std::copy(wires.begin(), wires.end(), o.q);
       o.num_items = static_cast<uint32_t>(words_.back().size() / 3);
       o.items = words_.back().data();
-      o.mats = floats_.back().data();
+      o.mats = hi;
+      o.mats_lo = lo;
       wires.clear();
       grads = 0;
     };
@@ -734,8 +739,7 @@ class SmallProgram {
         in_step++;
         items.insert(items.end(), {static_cast<uint32_t>(wires.size() - 1),
                                    static_cast<uint32_t>(o->gen), o->gen ? o->slot : 0u});
-        mats.resize(mats.size() + 8);
-        narrow(o->minv, mats.data() + mats.size() - 8);
+        mats.insert(mats.end(), o->minv, o->minv + 4);
         grads += o->gen != 0;
       }
     }
@@ -762,6 +766,16 @@ class SmallProgram {
   const float *matrices(const cdouble *m, size_t count) {
     floats_.emplace_back(8 * count);
     for (size_t j = 0; j < count; j++) narrow(m + 4 * j, floats_.back().data() + 8 * j);
+    return floats_.back().data();
+  }
+
+  // What the narrowed matrices `hi` lack.
+  const float *low_parts(const cdouble *m, size_t count, const float *hi) {
+    floats_.emplace_back(8 * count);
+    for (size_t k = 0; k < 4 * count; k++) {
+      floats_.back()[2 * k] = static_cast<float>(m[k].real() - hi[2 * k]);
+      floats_.back()[2 * k + 1] = static_cast<float>(m[k].imag() - hi[2 * k + 1]);
+    }
     return floats_.back().data();
   }
 
@@ -1675,7 +1689,7 @@ void Simulator::sweep_fused(const Circuit &c) {
 void Simulator::fused_gradient(const Circuit &c, const Hamiltonian &h, size_t shots,
                                uint64_t seed) {
   const Plan plan = build_plan(c, FusionOptions{});
-  if (small() && small_gradient(c, h, plan, shots, seed)) return;
+  if (n_ <= kSmallGradient && small_gradient(c, h, plan, shots, seed)) return;
   keep_ckpts_ = checkpoints_pair(c, plan);
   run_steps(plan, fold_diagonals(plan, merged_schedule(plan)));
   keep_ckpts_ = false;
@@ -1792,7 +1806,7 @@ void Simulator::serve_enqueue(const Circuit &c, const Hamiltonian &h, size_t sho
   prepare_adjoint(c, h);
   reset();
   const Plan plan = build_plan(c, FusionOptions{});
-  if (!small() || !small_gradient(c, h, plan, shots, seed)) {
+  if (n_ > kSmallGradient || !small_gradient(c, h, plan, shots, seed)) {
     run_steps(plan, fold_diagonals(plan, merged_schedule(plan)));
     if (shots) launch_sample(shots, seed);
     energy_and_costate(h);
