@@ -94,6 +94,7 @@ struct PlanOp {
   std::vector<uint32_t> group_qubits;
   std::vector<cdouble> group_matrices;
   uint32_t block_bits = 0;
+  size_t gate = SIZE_MAX;   // the circuit's gate, of an op that is one gate
   size_t term_count() const { return masks.size(); }
 };
 

@@ -300,6 +300,7 @@ Plan build_plan(const Circuit &c, const FusionOptions &opts) {
       }
     }
     plan.ops.push_back(lower_one(c.ops[i]));
+    plan.ops.back().gate = i;
     i++;
   }
 

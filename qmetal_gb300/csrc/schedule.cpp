@@ -579,6 +579,7 @@ std::vector<ForwardStep> small_schedule(const Plan &p) {
   std::vector<ForwardStep> out;
   WireRun held;
   std::vector<PermGate> run;
+  std::vector<size_t> run_ops;
   auto flush = [&]() {
     std::vector<size_t> idx(held.wires.size());
     for (size_t i = 0; i < idx.size(); i++) idx[i] = i;
@@ -593,13 +594,16 @@ std::vector<ForwardStep> small_schedule(const Plan &p) {
     s.kind = ForwardStep::Permute;
     s.cols = map.cols;
     s.off = map.off;
+    s.ops = std::move(run_ops);
     out.push_back(std::move(s));
     run.clear();
+    run_ops.clear();
   };
   for (size_t i = 0; i < p.ops.size(); i++) {
     const PlanOp &op = p.ops[i];
     if (is_wire_move(op, n)) {
       run.push_back({op.kind == PlanOp::Kind::Swap, op.qubits[0], op.qubits[1]});
+      run_ops.push_back(i);
       continue;
     }
     const uint32_t *w = nullptr;
@@ -619,6 +623,13 @@ std::vector<ForwardStep> small_schedule(const Plan &p) {
   }
   flush();
   return out;
+}
+
+bool undone_by(const Plan &p, const ForwardStep &gather, const std::vector<size_t> &gates) {
+  if (gather.ops.size() != gates.size()) return false;
+  for (size_t k = 0; k < gates.size(); k++)
+    if (p.ops[gather.ops[k]].gate != gates[gates.size() - 1 - k]) return false;
+  return true;
 }
 
 // ---------------------------------------------------------------------------

@@ -107,6 +107,13 @@ double schedule_cost(const Plan &p, const std::vector<ForwardStep> &steps);
 // step, every run of CX / SWAP ops as one gather, other ops as they are.
 std::vector<ForwardStep> small_schedule(const Plan &p);
 
+// Does undoing the circuit's gates `gates` (last first) undo this gather and
+// nothing else? Only then is the state from before the gather the one that the
+// undo leads to. Two runs with one map need not be the same run: a window
+// whose 2x2s are the identity is not in the plan, which then has one run where
+// the circuit, and its sweep, have two.
+bool undone_by(const Plan &p, const ForwardStep &gather, const std::vector<size_t> &gates);
+
 // --- co-state lambda = H psi and the energy ---------------------------------
 
 struct CostateStep {

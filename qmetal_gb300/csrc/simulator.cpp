@@ -361,8 +361,8 @@ bool inverts(uint32_t n, const std::vector<uint64_t> &a, uint64_t aoff,
 
 // The forward schedule's gathers, last first, against the backward
 // schedule's undo gathers in the order the sweep meets them: the same
-// number, each undoing its partner, and no CX or SWAP undone one gate at a
-// time (which would leave a forward gather without its partner).
+// number, each undoing its partner's gates, and no CX or SWAP undone one gate
+// at a time (which would leave a forward gather without its partner).
 bool Simulator::checkpoints_pair(const Circuit &c, const Plan &p) const {
   std::vector<const ForwardStep *> fwd;
   const auto fs = merged_schedule(p);
@@ -377,7 +377,7 @@ bool Simulator::checkpoints_pair(const Circuit &c, const Plan &p) const {
     } else if (st.kind == BackwardStep::PermuteUndo) {
       if (i == 0) return false;
       --i;
-      if (!inverts(n_, fwd[i]->cols, fwd[i]->off, st.cols, st.off)) return false;
+      if (!undone_by(p, *fwd[i], st.gates)) return false;
     }
   }
   return i == 0;
@@ -824,8 +824,8 @@ void Simulator::run_small(const Plan &p) {
 // state: one launch (two with samples), through small_schedule and
 // backward_schedule. Every map of the forward pass keeps the state from before
 // it (the last ones, as there is room), which the sweep takes back instead of
-// undoing the map on it, where the two schedules' maps pair up one to one. False, with nothing launched, for a
-// circuit that the launch cannot take.
+// undoing the map on it, where the two schedules' maps are of the same gates one
+// to one. False, with nothing launched, for a circuit that the launch cannot take.
 bool Simulator::small_gradient(const Circuit &c, const Hamiltonian &h, const Plan &plan,
                                size_t shots, uint64_t seed) {
   const auto fwd = small_schedule(plan);
@@ -834,14 +834,17 @@ bool Simulator::small_gradient(const Circuit &c, const Hamiltonian &h, const Pla
   struct Undo {
     const BackwardStep *step = nullptr;   // null: a map
     std::vector<uint64_t> cols;
+    std::vector<size_t> gates;            // a map's, in undo order
   };
   std::vector<Undo> undos;
   std::vector<PermGate> run;   // in undo order
+  std::vector<size_t> run_gates;
   auto end_run = [&]() {
     if (run.empty()) return;
     std::reverse(run.begin(), run.end());
-    undos.push_back({nullptr, run_map(n_, run, true).cols});
+    undos.push_back({nullptr, run_map(n_, run, true).cols, std::move(run_gates)});
     run.clear();
+    run_gates.clear();
   };
   for (const BackwardStep &st : bwd) {
     if (st.kind == BackwardStep::GateUndo || st.kind == BackwardStep::PermuteUndo) {
@@ -853,21 +856,23 @@ bool Simulator::small_gradient(const Circuit &c, const Hamiltonian &h, const Pla
       if (moves) {
         for (size_t k : st.gates)
           run.push_back({c.ops[k].kind == G_SWAP, c.ops[k].qubits[0], c.ops[k].qubits[1]});
+        run_gates.insert(run_gates.end(), st.gates.begin(), st.gates.end());
         continue;
       }
     }
     end_run();
-    undos.push_back({&st, {}});
+    undos.push_back({&st, {}, {}});
   }
   end_run();
-  std::vector<const std::vector<uint64_t> *> kept, undone;
+  std::vector<const ForwardStep *> kept;
+  std::vector<const Undo *> undone;
   for (const ForwardStep &st : fwd)
-    if (st.kind == ForwardStep::Permute) kept.push_back(&st.cols);
+    if (st.kind == ForwardStep::Permute) kept.push_back(&st);
   for (const Undo &u : undos)
-    if (!u.step) undone.push_back(&u.cols);
+    if (!u.step) undone.push_back(&u);
   bool pair = kept.size() == undone.size();
   for (size_t i = 0; pair && i < kept.size(); i++)
-    pair = inverts(n_, *kept[kept.size() - 1 - i], 0, *undone[i], 0);
+    pair = undone_by(plan, *kept[kept.size() - 1 - i], undone[i]->gates);
 
   // The last maps' states are kept, as many as there is room for.
   const size_t room = pair ? std::min<size_t>(kept.size(), qmk_small_saves(n_)) : 0;
