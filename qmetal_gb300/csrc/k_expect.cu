@@ -3,8 +3,12 @@
 // seven wires >= 6 and wires 0..5), and narrow states (one block per string,
 // one launch for all).
 //
-// Precision: FP32 runs of at most ten dependent additions, FP64 from there
-// (per thread, then the block and grid sums of finish()).
+// Precision: an amplitude's or a pair's product is rounded to FP32, and sums of
+// them are FP32 high and low parts from there (gather(), then the block and grid
+// sums of finish()). Sums of 128 and 32 products in FP32 first had two to four
+// times the error (15 qubits, rms: Z strings 7.0e-9, now 1.9e-9; X terms 4.3e-9,
+// now 1.1e-9). X terms from 22 qubits on add four pairs in FP32 first: errors of
+// 6e-10 and less, where sums of eight pairs and FP64 from there had the same.
 #include <algorithm>
 #include <atomic>
 #include <vector>
@@ -24,15 +28,18 @@ namespace {
 // transforms their probabilities by a 32-point Walsh-Hadamard transform in
 // registers: entry c is then the sum over the 32 with the sign of the bits of
 // c, so each string costs one entry and one sign instead of 32 signed adds.
+// Each probability goes in two parts: its multiple of 2^-18 of a power of two
+// above the thread's largest, whose sums of 32 are exact in FP32, and the rest,
+// whose transform rounds 2^-19 lower.
 // Strings by the sign word: bit t is the parity of string t over the thread's
 // lane bits (once per kernel) and over the warp's site number (one string per
-// lane, a ballot per site). Four sites are added in FP32 (transform depth 5
-// and 3 additions), then to FP64 sums in shared memory.
+// lane, a ballot per site).
 //
-// Bound by the read of the state.
+// One block a multiprocessor: the sums take 64 registers a thread, the next
+// site's vectors 64 while they arrive. Bound by the read of the state and the
+// transforms' adds about equally.
 
 constexpr int kZTerms = 32;
-constexpr int kZSites = 4;      // sites per FP32 run
 
 struct ZTermArgs {
   uint32_t nt;
@@ -41,66 +48,77 @@ struct ZTermArgs {
   uint8_t coef[kZTerms];        // transform entry: wire 0, wires 6..9
 };
 
+__device__ __forceinline__ void transform32(float (&p)[32]) {
+#pragma unroll
+  for (int h = 1; h < 32; h <<= 1) {
+#pragma unroll
+    for (int i = 0; i < 32; i++) {
+      if (i & h) continue;
+      const float u = p[i], v = p[i | h];
+      p[i] = u + v;
+      p[i | h] = u - v;
+    }
+  }
+}
+
 template <int T>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, 1)
 k_zterms(const float4 *__restrict__ st, uint64_t nwsites, ZTermArgs z, Area a, OutContig out) {
-  extern __shared__ __align__(16) float zsm[];
-  float *w = zsm + threadIdx.x;                                    // [32][kThreads]
-  double *sums = reinterpret_cast<double *>(zsm + 32 * kThreads) + threadIdx.x;   // [T][kThreads]
+  extern __shared__ __align__(16) float2 zsm[];
+  float2 *w = zsm + threadIdx.x;   // [32][kThreads]
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t gw = (static_cast<uint64_t>(blockIdx.x) * kThreads + threadIdx.x) >> 5;
   const uint64_t nwarps = static_cast<uint64_t>(gridDim.x) * (kThreads / 32);
   uint32_t lsign = 0;
 #pragma unroll
-  for (int t = 0; t < T; t++) {
+  for (int t = 0; t < T; t++)
     lsign |= (static_cast<uint32_t>(__popc(lane & z.lane[t])) & 1u) << t;
-    sums[t * kThreads] = 0.0;
-  }
   const uint64_t mine =   // the site mask of the string this lane answers for
       lane < T ? (static_cast<uint64_t>(z.hi[lane][1]) << 32) | z.hi[lane][0] : 0ull;
-  float part[T];
-#pragma unroll
-  for (int t = 0; t < T; t++) part[t] = 0.0f;
-  int held = 0;
-  for (uint64_t ws = gw; ws < nwsites; ws += nwarps) {
+  Two acc[T] = {};
+  float4 x[16];
+  auto load = [&](uint64_t ws) {
     const float4 *row = st + (ws << 9) + lane;
-    float p[32];
+#pragma unroll
+    for (int l = 0; l < 16; l++) x[l] = row[l * 32];
+  };
+  if (gw < nwsites) load(gw);
+  for (uint64_t ws = gw; ws < nwsites; ws += nwarps) {
+    float h[32], r[32], most = 0.0f;
 #pragma unroll
     for (int l = 0; l < 16; l++) {
-      const float4 x = row[l * 32];
-      p[2 * l] = fmaf(x.x, x.x, x.y * x.y);
-      p[2 * l + 1] = fmaf(x.z, x.z, x.w * x.w);
+      r[2 * l] = fmaf(x[l].x, x[l].x, x[l].y * x[l].y);
+      r[2 * l + 1] = fmaf(x[l].z, x[l].z, x[l].w * x[l].w);
+      most = fmaxf(most, fmaxf(r[2 * l], r[2 * l + 1]));
     }
+    if (ws + nwarps < nwsites) load(ws + nwarps);
+    // c = 1.5 * 2^(e + 6) for most in [2^e, 2^(e + 1)): adding it rounds to a
+    // multiple of 2^(e - 17). Without a part where that or a sum would overflow.
+    const uint32_t e = __float_as_uint(most) & 0x7f800000u;
+    const bool parts = e < (240u << 23);
+    const float c = parts ? __uint_as_float((e + (6u << 23)) | 0x400000u) : 0.0f;
 #pragma unroll
-    for (int h = 1; h < 32; h <<= 1) {
-#pragma unroll
-      for (int i = 0; i < 32; i++) {
-        if (i & h) continue;
-        const float u = p[i], v = p[i | h];
-        p[i] = u + v;
-        p[i | h] = u - v;
-      }
+    for (int i = 0; i < 32; i++) {
+      h[i] = __fadd_rn(__fadd_rn(r[i], c), -c);
+      r[i] = __fadd_rn(r[i], -h[i]);
     }
+    if (!parts) {
 #pragma unroll
-    for (int c = 0; c < 32; c++) w[c * kThreads] = p[c];
+      for (int i = 0; i < 32; i++) r[i] = 0.0f;
+    }
+    transform32(h);
+    transform32(r);
+#pragma unroll
+    for (int i = 0; i < 32; i++) w[i * kThreads] = make_float2(h[i], r[i]);
     const uint32_t sign = lsign ^ __ballot_sync(0xffffffffu, parity64(ws & mine));
 #pragma unroll
     for (int t = 0; t < T; t++) {
-      const uint32_t bits = __float_as_uint(w[z.coef[t] * kThreads]);
-      part[t] += __uint_as_float(bits ^ ((sign << (31 - t)) & 0x80000000u));
-    }
-    if (++held == kZSites) {
-      held = 0;
-#pragma unroll
-      for (int t = 0; t < T; t++) {
-        sums[t * kThreads] += part[t];
-        part[t] = 0.0f;
-      }
+      const float2 v = w[z.coef[t] * kThreads];
+      const uint32_t minus = (sign << (31 - t)) & 0x80000000u;
+      acc[t] = gather(acc[t], __uint_as_float(__float_as_uint(v.x) ^ minus));
+      acc[t].lo = __fadd_rn(acc[t].lo, __uint_as_float(__float_as_uint(v.y) ^ minus));
     }
   }
-  double acc[T];
-#pragma unroll
-  for (int t = 0; t < T; t++) acc[t] = sums[t * kThreads] + part[t];
   finish<T>(acc, static_cast<int>(z.nt), a, out);
 }
 
@@ -122,10 +140,10 @@ template <int T>
 int launch_z(const float4 *st, uint64_t nwsites, const ZTermArgs &z, Area a, OutContig out,
              cudaStream_t s) {
   static std::atomic<bool> opted[64];   // zero-initialised: false
-  const size_t smem = kThreads * (32 * sizeof(float) + T * sizeof(double));
+  const size_t smem = kThreads * 32 * sizeof(float2);
   if (const int rc = opt_in(k_zterms<T>, smem, opted)) return rc;
   const unsigned grid = std::min<unsigned>(grid_for(nwsites, kThreads / 32),
-                                           static_cast<unsigned>(qmk_host::num_sms()) * 2);
+                                           static_cast<unsigned>(qmk_host::num_sms()));
   k_zterms<T><<<grid, kThreads, smem, s>>>(st, nwsites, z, a, out);
   return launch_status();
 }
@@ -141,8 +159,8 @@ int launch_z(const float4 *st, uint64_t nwsites, const ZTermArgs &z, Area a, Out
 // bit so that both do half; wires 1..5 read the partner lane, wire 0 is the
 // other half of the vector.
 //
-// Bound by the read of the state: a pass reads it once for up to 13 wires
-// where one wire at a time read it 13 times.
+// Bound by the read of the state and its adds about equally: a pass reads the
+// state once for up to 13 wires where one wire at a time read it 13 times.
 
 struct XTermArgs {
   uint32_t pos[7];     // vector bits (wire - 1) of the site's wires >= 6, ascending
@@ -175,7 +193,34 @@ __device__ __forceinline__ float re_dot(const float4 &x, const float4 &y) {
   return fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, x.w * y.w)));
 }
 
-template <int WB, bool LOW>
+// Where a thread's products go. RUNS: four pairs (two vectors) are added in
+// FP32, then the run to the sum; otherwise every pair by itself.
+template <bool RUNS>
+struct XSum {
+  Two &acc;
+  float run = 0.0f;
+  __device__ __forceinline__ explicit XSum(Two &a) : acc(a) {}
+  __device__ __forceinline__ void vectors(const float4 &x, const float4 &y) {
+    if (RUNS) {
+      run += re_dot(x, y);
+    } else {
+      acc = gather(acc, fmaf(x.x, y.x, x.y * y.y));
+      acc = gather(acc, fmaf(x.z, y.z, x.w * y.w));
+    }
+  }
+  __device__ __forceinline__ void halves(const float4 &x) {   // wire 0
+    const float v = fmaf(x.x, x.z, x.y * x.w);
+    if (RUNS) run += v;
+    else acc = gather(acc, v);
+  }
+  __device__ __forceinline__ void end_run() {
+    if (!RUNS) return;
+    acc = gather(acc, run);
+    run = 0.0f;
+  }
+};
+
+template <int WB, bool LOW, bool RUNS>
 __global__ void __launch_bounds__(kThreads, 2)
 k_xterms(const float4 *__restrict__ st, uint64_t nsites, XTermArgs c, Area a,
          OutWanted<4 + WB + (LOW ? 6 : 0)> out) {
@@ -223,9 +268,7 @@ k_xterms(const float4 *__restrict__ st, uint64_t nsites, XTermArgs c, Area a,
     }
     cp_async_commit();
   };
-  double acc[T];
-#pragma unroll
-  for (int t = 0; t < T; t++) acc[t] = 0.0;
+  Two acc[T] = {};
   prefetch(0);
   for (uint64_t r = 0; r < rounds; r++) {
     const bool active = site_of(r) < nsites;   // uniform over the site's warps
@@ -237,41 +280,43 @@ k_xterms(const float4 *__restrict__ st, uint64_t nsites, XTermArgs c, Area a,
       for (int l = 0; l < NV; l++) own[l] = site[(l | (wsl << 4)) * 32 + lane];
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        float s[2] = {0.0f, 0.0f};   // two runs of four pairs
+        XSum<RUNS> s(acc[j]);
         int k = 0;
 #pragma unroll
         for (int l = 0; l < NV; l++) {
           if ((l >> j) & 1) continue;
-          s[k++ >> 2] += re_dot(own[l], own[l | (1 << j)]);
+          s.vectors(own[l], own[l | (1 << j)]);
+          if (++k % 2 == 0) s.end_run();
         }
-        acc[j] += s[0] + s[1];
       }
 #pragma unroll
       for (int j = 0; j < WB; j++) {
         const uint32_t b = (wsl >> j) & 1u;   // this warp takes the rows with bit 0 == b
-        float s[2] = {0.0f, 0.0f};
+        XSum<RUNS> s(acc[4 + j]);
 #pragma unroll
         for (int l = 0; l < NV; l += 2) {
           const float4 x = b ? own[l + 1] : own[l];
-          s[l >> 3] += re_dot(x, site[((l | b) | ((wsl ^ (1u << j)) << 4)) * 32 + lane]);
+          s.vectors(x, site[((l | b) | ((wsl ^ (1u << j)) << 4)) * 32 + lane]);
+          if (l % 4 == 2) s.end_run();
         }
-        acc[4 + j] += s[0] + s[1];
       }
       if constexpr (LOW) {
-        float s0[2] = {0.0f, 0.0f};
+        XSum<RUNS> s0(acc[KB]);
 #pragma unroll
-        for (int l = 0; l < NV; l++) s0[l >> 3] += fmaf(own[l].x, own[l].z, own[l].y * own[l].w);
-        acc[KB] += s0[0] + s0[1];
+        for (int l = 0; l < NV; l++) {
+          s0.halves(own[l]);
+          if (l % 4 == 3) s0.end_run();
+        }
 #pragma unroll
         for (int k = 0; k < 5; k++) {
           const uint32_t b = (lane >> k) & 1u;   // this lane takes the rows with bit 0 == b
-          float s[2] = {0.0f, 0.0f};
+          XSum<RUNS> s(acc[KB + 1 + k]);
 #pragma unroll
           for (int l = 0; l < NV; l += 2) {
             const float4 x = b ? own[l + 1] : own[l];
-            s[l >> 3] += re_dot(x, site[((l | b) | (wsl << 4)) * 32 + (lane ^ (1u << k))]);
+            s.vectors(x, site[((l | b) | (wsl << 4)) * 32 + (lane ^ (1u << k))]);
+            if (l % 4 == 2) s.end_run();
           }
-          acc[KB + 1 + k] += s[0] + s[1];
         }
       }
     }
@@ -282,25 +327,38 @@ k_xterms(const float4 *__restrict__ st, uint64_t nsites, XTermArgs c, Area a,
   finish<T>(acc, T, a, out);
 }
 
-template <int WB, bool LOW>
-int launch_x(const float4 *st, uint64_t nsites, const XTermArgs &c, Area a, double *d_out,
+template <int WB, bool LOW, bool RUNS>
+int launch_x_as(const float4 *st, uint64_t nsites, const XTermArgs &c, Area a, double *d_out,
              const int8_t (&slot)[13], cudaStream_t s) {
   constexpr int SPB = (kThreads / 32) >> WB;
   static std::atomic<bool> opted[64];   // zero-initialised: false
   const size_t smem = static_cast<size_t>(kThreads / 32) * 16 * 32 * sizeof(float4);
-  if (const int rc = opt_in(k_xterms<WB, LOW>, smem, opted)) return rc;
+  if (const int rc = opt_in(k_xterms<WB, LOW, RUNS>, smem, opted)) return rc;
   OutWanted<4 + WB + (LOW ? 6 : 0)> out;
   out.p = d_out;
   for (int t = 0; t < 4 + WB + (LOW ? 6 : 0); t++) out.slot[t] = slot[t];
   const unsigned grid = std::min<unsigned>(grid_for(nsites, SPB),
                                            static_cast<unsigned>(qmk_host::num_sms()) * 2);
-  k_xterms<WB, LOW><<<grid, kThreads, smem, s>>>(st, nsites, c, a, out);
+  k_xterms<WB, LOW, RUNS><<<grid, kThreads, smem, s>>>(st, nsites, c, a, out);
   return launch_status();
+}
+
+// From 22 qubits on four pairs at a time in FP32: by then their errors average
+// out over 2^18 such sums. At 27 qubits all X terms, 27 ZZ and four longer
+// strings take 1.86 ms so, 2.04 with every pair by itself.
+constexpr uint32_t kXRunQubits = 22;
+
+template <int WB, bool LOW>
+int launch_x(const float4 *st, uint64_t nsites, const XTermArgs &c, Area a, double *d_out,
+             const int8_t (&slot)[13], cudaStream_t s) {
+  return nsites >> (kXRunQubits - 10 - WB)
+             ? launch_x_as<WB, LOW, true>(st, nsites, c, a, d_out, slot, s)
+             : launch_x_as<WB, LOW, false>(st, nsites, c, a, d_out, slot, s);
 }
 
 // ---------------------------------------------------------------------------
 // Narrow states: a block per string, any masks, one launch. The state is in
-// L2 (128 KiB at 14 qubits); a thread's runs are eight products in FP32.
+// L2 (128 KiB at 14 qubits).
 
 constexpr int kSmallTerms = 64;
 struct SmallArgs {
@@ -316,9 +374,8 @@ k_expect_small(const float2 *__restrict__ st, uint32_t n, SmallArgs p, double *o
   const bool im = (p.useim >> t) & 1ull;
   const uint32_t hbit = flip ? 63 - __clzll(flip) : 0;
   const uint32_t items = flip ? 1u << (n - 1) : 1u << n;
-  double acc = 0.0;
+  Two acc = {};
   for (uint32_t u0 = threadIdx.x; u0 < items; u0 += kThreads * 8) {
-    float part = 0.0f;
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       const uint32_t u = u0 + k * kThreads;
@@ -326,13 +383,12 @@ k_expect_small(const float2 *__restrict__ st, uint32_t n, SmallArgs p, double *o
         const uint64_t i = flip ? ins0(u, hbit) : u;
         const float2 x = st[i], y = st[i ^ flip];
         const float v = im ? x.x * y.y - x.y * y.x : x.x * y.x + x.y * y.y;
-        part += parity64(i & sign) ? -v : v;
+        acc = gather(acc, parity64(i & sign) ? -v : v);
       }
     }
-    acc += part;
   }
-  acc = block_sum(acc, sm);
-  if (threadIdx.x == 0) out[t] = acc;
+  const double sum = block_sum(widen(settle(acc)), sm);
+  if (threadIdx.x == 0) out[t] = sum;
 }
 
 bool ok_state(const float *p) { return p && (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

@@ -1,10 +1,12 @@
 // k_reduce.cu -- reductions over the state (norm, Pauli expectations, dot),
 // the co-state build and the fused adjoint step.
 //
-// Precision: each thread sums a short run (a chunk of vectors) in FP32, adds
-// the chunk into an FP64 accumulator, and everything from the warp up is
-// FP64. Blocks write FP64 partials; the last block to finish adds them in
-// block order, so a result depends only on the grid size, never on timing.
+// Precision: products of a vector or a pair in FP32, their sums as FP32 high and
+// low parts (in FP64 from the warp up for the norm and the dot product). With
+// runs of eight pairs in FP32 the strings of a narrow state were off by up to
+// four times as much (a thread holds few of them there, and nothing averages out).
+// The last block to finish adds the blocks' partials in a fixed order, so a
+// result depends only on the grid size, never on timing.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -20,11 +22,11 @@ namespace {
 
 constexpr int kMaxT = 16;
 
-constexpr int kChunk = 4;  // vectors per FP32 run and per thread iteration
+constexpr int kChunk = 4;  // vectors per thread iteration
 
 __global__ void __launch_bounds__(kThreads)
 k_abs2(const float4 *__restrict__ st, uint64_t nvec, Area a, double *out) {
-  double acc[1] = {0.0};
+  Two sum = {};
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kThreads;
   for (uint64_t v0 = static_cast<uint64_t>(blockIdx.x) * kThreads + threadIdx.x; v0 < nvec;
        v0 += stride * kChunk) {
@@ -34,19 +36,19 @@ k_abs2(const float4 *__restrict__ st, uint64_t nvec, Area a, double *out) {
       const uint64_t v = v0 + k * stride;
       x[k] = (v < nvec) ? st[v] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    float s = 0.0f;
 #pragma unroll
     for (int k = 0; k < kChunk; k++)
-      s = fmaf(x[k].x, x[k].x, fmaf(x[k].y, x[k].y, fmaf(x[k].z, x[k].z, fmaf(x[k].w, x[k].w, s))));
-    acc[0] += s;
+      sum = gather(sum, fmaf(x[k].x, x[k].x, fmaf(x[k].y, x[k].y,
+                                                  fmaf(x[k].z, x[k].z, x[k].w * x[k].w))));
   }
+  double acc[1] = {widen(settle(sum))};
   finish<1>(acc, 1, a, OutContig{out, false});
 }
 
 __global__ void __launch_bounds__(kThreads)
 k_dot_re(const float4 *__restrict__ x4, const float4 *__restrict__ y4, uint64_t nvec,
          Area a, double *out) {
-  double acc[1] = {0.0};
+  Two sum = {};
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kThreads;
   for (uint64_t v0 = static_cast<uint64_t>(blockIdx.x) * kThreads + threadIdx.x; v0 < nvec;
        v0 += stride * kChunk) {
@@ -57,12 +59,12 @@ k_dot_re(const float4 *__restrict__ x4, const float4 *__restrict__ y4, uint64_t 
       x[k] = (v < nvec) ? x4[v] : make_float4(0.f, 0.f, 0.f, 0.f);
       y[k] = (v < nvec) ? y4[v] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    float s = 0.0f;
 #pragma unroll
     for (int k = 0; k < kChunk; k++)
-      s = fmaf(x[k].x, y[k].x, fmaf(x[k].y, y[k].y, fmaf(x[k].z, y[k].z, fmaf(x[k].w, y[k].w, s))));
-    acc[0] += s;
+      sum = gather(sum, fmaf(x[k].x, y[k].x, fmaf(x[k].y, y[k].y,
+                                                  fmaf(x[k].z, y[k].z, x[k].w * y[k].w))));
   }
+  double acc[1] = {widen(settle(sum))};
   finish<1>(acc, 1, a, OutContig{out, false});
 }
 
@@ -77,13 +79,13 @@ struct PauliArgs {
 // flip != 0: over pairs (i, j = i ^ flip) with bit hbit of i clear,
 // sum s_t(i) * (Re or Im of conj(psi_i) psi_j); the host applies +-2. Two
 // pairs a vector: j's vector is v ^ (flip >> 1), its halves traded when bit 0
-// is flipped too. INV: flip is bit 0 alone, the pair is one vector's halves.
-template <int T, bool INV>
+// is flipped too. INV: flip is bit 0 alone, the pair is one vector's halves. RUNS:
+// four pairs (two vectors) are added in FP32 first.
+template <int T, bool INV, bool RUNS>
 __global__ void __launch_bounds__(kThreads)
 k_pauli_x(const float4 *__restrict__ st, uint64_t nsites, PauliArgs p, Area a, double *out) {
-  double acc[T];
-#pragma unroll
-  for (int t = 0; t < T; t++) acc[t] = 0.0;
+  Two acc[T] = {};
+  float run[T] = {};
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kThreads;
   const uint64_t vflip = p.flip >> 1;
   for (uint64_t s0 = static_cast<uint64_t>(blockIdx.x) * kThreads + threadIdx.x; s0 < nsites;
@@ -97,9 +99,6 @@ k_pauli_x(const float4 *__restrict__ st, uint64_t nsites, PauliArgs p, Area a, d
       x[k] = (s < nsites) ? st[v[k]] : make_float4(0.f, 0.f, 0.f, 0.f);
       if (!INV) y[k] = (s < nsites) ? st[v[k] ^ vflip] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    float part[T];
-#pragma unroll
-    for (int t = 0; t < T; t++) part[t] = 0.0f;
 #pragma unroll
     for (int k = 0; k < kChunk; k++) {
       const float2 i0 = lo2(x[k]), i1 = hi2(x[k]);
@@ -108,7 +107,7 @@ k_pauli_x(const float4 *__restrict__ st, uint64_t nsites, PauliArgs p, Area a, d
 #pragma unroll
         for (int t = 0; t < T; t++) {
           const float w = (p.useim >> t & 1) ? im : re;
-          part[t] += parity64((v[k] << 1) & p.sign[t]) ? -w : w;
+          acc[t] = gather(acc[t], parity64((v[k] << 1) & p.sign[t]) ? -w : w);
         }
       } else {
         const bool odd = p.flip & 1ull;
@@ -119,13 +118,20 @@ k_pauli_x(const float4 *__restrict__ st, uint64_t nsites, PauliArgs p, Area a, d
         for (int t = 0; t < T; t++) {
           const bool im = p.useim >> t & 1;
           const float w0 = im ? im0 : re0, w1 = im ? im1 : re1;
-          const float w = (p.sign[t] & 1ull) ? w0 - w1 : w0 + w1;
-          part[t] += parity64((v[k] << 1) & p.sign[t]) ? -w : w;
+          const bool minus = parity64((v[k] << 1) & p.sign[t]);
+          if (RUNS) {
+            const float w = (p.sign[t] & 1ull) ? w0 - w1 : w0 + w1;
+            run[t] = minus ? run[t] - w : run[t] + w;
+            if (k % 2 == 0) continue;
+            acc[t] = gather(acc[t], run[t]);
+            run[t] = 0.0f;
+          } else {
+            acc[t] = gather(acc[t], minus ? -w0 : w0);
+            acc[t] = gather(acc[t], minus != static_cast<bool>(p.sign[t] & 1ull) ? -w1 : w1);
+          }
         }
       }
     }
-#pragma unroll
-    for (int t = 0; t < T; t++) acc[t] += part[t];
   }
   finish<T>(acc, p.nt, a, OutContig{out, false});
 }
@@ -226,8 +232,12 @@ void launch_pauli(const float *state, uint32_t n, const PauliArgs &p, Area a,
   const float4 *st = reinterpret_cast<const float4 *>(state);
   const uint64_t nsites = p.flip == 1 ? 1ull << (n - 1) : 1ull << (n - 2);
   const unsigned g = std::min<unsigned>(reduce_grid(), grid_for(nsites, kThreads * kChunk));
-  if (p.flip == 1) k_pauli_x<T, true><<<g, kThreads, 0, s>>>(st, nsites, p, a, out);
-  else k_pauli_x<T, false><<<g, kThreads, 0, s>>>(st, nsites, p, a, out);
+  // From 22 qubits on (k_xterms' limit): sixteen strings of one flip at 26 qubits
+  // take 633 us pair by pair.
+  const bool runs = n >= 22;
+  if (p.flip == 1) k_pauli_x<T, true, true><<<g, kThreads, 0, s>>>(st, nsites, p, a, out);
+  else if (runs) k_pauli_x<T, false, true><<<g, kThreads, 0, s>>>(st, nsites, p, a, out);
+  else k_pauli_x<T, false, false><<<g, kThreads, 0, s>>>(st, nsites, p, a, out);
 }
 
 template <int T>

@@ -74,6 +74,17 @@ __device__ __forceinline__ double add(double a, double b) { return a + b; }
 __device__ __forceinline__ double widen(Two v) {
   return static_cast<double>(v.hi) + static_cast<double>(v.lo);
 }
+// a + v for a long run of FP32 values, seven operations: the low part collects
+// what each sum loses and is settled once, at the run's end.
+__device__ __forceinline__ Two gather(Two a, float v) {
+  const float s = __fadd_rn(a.hi, v), t = __fadd_rn(s, -a.hi);
+  const float e = __fadd_rn(__fadd_rn(a.hi, -__fadd_rn(s, -t)), __fadd_rn(v, -t));
+  return {s, __fadd_rn(a.lo, e)};
+}
+__device__ __forceinline__ Two settle(Two a) {
+  if (!isfinite(a.hi)) a.lo = 0.0f;
+  return add(a, Two{0.0f, 0.0f});
+}
 __device__ __forceinline__ double widen(double v) { return v; }
 __device__ __forceinline__ Two shfl_xor(Two v, int mask) {
   return {__shfl_xor_sync(0xffffffffu, v.hi, mask), __shfl_xor_sync(0xffffffffu, v.lo, mask)};
@@ -194,6 +205,15 @@ __device__ __forceinline__ void finish_as(const V (&acc)[T], int nt, Area a, con
 template <int T, typename Out>
 __device__ __forceinline__ void finish(double (&acc)[T], int nt, Area a, const Out &out) {
   finish_as<T, double>(acc, nt, a, out);
+}
+
+// For threads that hold what gather() adds up.
+template <int T, typename Out>
+__device__ __forceinline__ void finish(Two (&acc)[T], int nt, Area a, const Out &out) {
+  Two v[T];
+#pragma unroll
+  for (int t = 0; t < T; t++) v[t] = settle(acc[t]);
+  finish_as<T, Two>(v, nt, a, out);
 }
 
 // For threads that hold FP32 sums.
