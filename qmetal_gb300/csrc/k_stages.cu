@@ -371,8 +371,11 @@ k_stages_low(float4 *__restrict__ st, uint64_t nsites, LowSite h, StageArgs<kLow
   }
 }
 
-// An angle as turns in units of 2^-64.
+// An angle as turns in units of 2^-64. The quotient's rounding is 2^-52 of it: of
+// many turns, the angle within one turn comes from its cosine and sine, which
+// the C library reduces without loss.
 uint64_t turns(double angle) {
+  if (std::abs(angle) > 1024.0) angle = std::atan2(std::sin(angle), std::cos(angle));
   double t = angle / (2.0 * 3.14159265358979323846);
   t -= std::floor(t);
   const double x = std::ldexp(t, 64);

@@ -368,7 +368,8 @@ uint64_t fan_centres(const PlanOp &op, uint32_t n) {
   uint64_t common = ~0ull;
   for (size_t t = 0; t < op.masks.size(); t++) {
     const uint64_t m = op.masks[t];
-    if (popc(m) < 1 || popc(m) > 2 || (m >> n) || !std::isfinite(op.angles[t])) return 0;
+    // (angles that a sum with others of their wire keeps finite)
+    if (popc(m) < 1 || popc(m) > 2 || (m >> n) || !(std::abs(op.angles[t]) <= 1e300)) return 0;
     common &= m;
   }
   return common;
