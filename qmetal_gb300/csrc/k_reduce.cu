@@ -80,10 +80,15 @@ struct PauliArgs {
 // sum s_t(i) * (Re or Im of conj(psi_i) psi_j); the host applies +-2. Two
 // pairs a vector: j's vector is v ^ (flip >> 1), its halves traded when bit 0
 // is flipped too. INV: flip is bit 0 alone, the pair is one vector's halves. RUNS:
-// four pairs (two vectors) are added in FP32 first.
+// four pairs (two vectors) are added in FP32 first. The state may lie on 8 bytes
+// only: `wide` where it lies on 16.
 template <int T, bool INV, bool RUNS>
 __global__ void __launch_bounds__(kThreads)
-k_pauli_x(const float4 *__restrict__ st, uint64_t nsites, PauliArgs p, Area a, double *out) {
+k_pauli_x(const float2 *__restrict__ st, bool wide, uint64_t nsites, PauliArgs p, Area a,
+          double *out) {
+  auto vector = [&](uint64_t v) {
+    return wide ? reinterpret_cast<const float4 *>(st)[v] : pack4(st[2 * v], st[2 * v + 1]);
+  };
   Two acc[T] = {};
   float run[T] = {};
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kThreads;
@@ -96,8 +101,8 @@ k_pauli_x(const float4 *__restrict__ st, uint64_t nsites, PauliArgs p, Area a, d
     for (int k = 0; k < kChunk; k++) {
       const uint64_t s = s0 + k * stride;
       v[k] = INV ? s : ins0(s, p.hbit - 1);
-      x[k] = (s < nsites) ? st[v[k]] : make_float4(0.f, 0.f, 0.f, 0.f);
-      if (!INV) y[k] = (s < nsites) ? st[v[k] ^ vflip] : make_float4(0.f, 0.f, 0.f, 0.f);
+      x[k] = (s < nsites) ? vector(v[k]) : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (!INV) y[k] = (s < nsites) ? vector(v[k] ^ vflip) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
     for (int k = 0; k < kChunk; k++) {
@@ -229,15 +234,16 @@ k_adj1q(float4 *__restrict__ psi, float4 *__restrict__ lam, uint64_t nsites, uin
 template <int T>
 void launch_pauli(const float *state, uint32_t n, const PauliArgs &p, Area a,
                   double *out, cudaStream_t s) {
-  const float4 *st = reinterpret_cast<const float4 *>(state);
+  const float2 *st = reinterpret_cast<const float2 *>(state);
+  const bool wide = (reinterpret_cast<uintptr_t>(state) & 15u) == 0;
   const uint64_t nsites = p.flip == 1 ? 1ull << (n - 1) : 1ull << (n - 2);
   const unsigned g = std::min<unsigned>(reduce_grid(), grid_for(nsites, kThreads * kChunk));
   // From 22 qubits on (k_xterms' limit): sixteen strings of one flip at 26 qubits
   // take 633 us pair by pair.
   const bool runs = n >= 22;
-  if (p.flip == 1) k_pauli_x<T, true, true><<<g, kThreads, 0, s>>>(st, nsites, p, a, out);
-  else if (runs) k_pauli_x<T, false, true><<<g, kThreads, 0, s>>>(st, nsites, p, a, out);
-  else k_pauli_x<T, false, false><<<g, kThreads, 0, s>>>(st, nsites, p, a, out);
+  if (p.flip == 1) k_pauli_x<T, true, true><<<g, kThreads, 0, s>>>(st, wide, nsites, p, a, out);
+  else if (runs) k_pauli_x<T, false, true><<<g, kThreads, 0, s>>>(st, wide, nsites, p, a, out);
+  else k_pauli_x<T, false, false><<<g, kThreads, 0, s>>>(st, wide, nsites, p, a, out);
 }
 
 template <int T>
@@ -380,7 +386,7 @@ extern "C" int qmk_pauli_expect(const float *state, uint32_t n, uint64_t flip,
       !ok_ws(ws, ws_bytes, n))
     return -1;
   if (n < 64 && (flip >> n)) return -1;
-  if (reinterpret_cast<uintptr_t>(state) & 15u) return -1;
+  if (reinterpret_cast<uintptr_t>(state) & (flip ? 7u : 15u)) return -1;
   if (flip == 0) {
     const uint64_t none[kMaxT] = {};
     const uint32_t even[kMaxT] = {};
