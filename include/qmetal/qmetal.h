@@ -85,8 +85,10 @@ int qm_synchronize(qm_simulator s);
 
 uint32_t qm_num_qubits(qm_simulator s);
 uint64_t qm_dim(qm_simulator s);
-/* Kernels launched; up to 13 qubits, where qm_run and its variants run a
- * circuit's plan in one launch, the plan's ops count as one each. */
+/* Kernels launched. Up to 13 qubits, where a circuit's plan runs in one launch
+ * (a few if it is long), qm_run, qm_run_unfused, qm_run_options and qm_run_cached
+ * count its ops as one each, as without that launch; qm_run_merged and the
+ * gradients count their launches. */
 uint64_t qm_dispatch_count(qm_simulator s);
 
 /* View of the interleaved state, 2 * qm_dim() floats, valid until the next

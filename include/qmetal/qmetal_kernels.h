@@ -176,6 +176,11 @@ uint32_t qmk_small_saves(uint32_t n);
 int qmk_run_small(float *state, uint32_t n, size_t num_ops,
                   const qmk_small_op *ops, const qmk_small_adjoint *adjoint,
                   void *workspace, size_t workspace_bytes, void *stream);
+/* The same; *launches receives the number of kernels launched. */
+int qmk_run_small_counted(float *state, uint32_t n, size_t num_ops,
+                          const qmk_small_op *ops, const qmk_small_adjoint *adjoint,
+                          void *workspace, size_t workspace_bytes, void *stream,
+                          uint32_t *launches);
 
 /* Stages in one in-place pass, in order, n >= 13. A stage is a 2x2 on its wire
  * (has_matrix) and a fan of controlled phases from it (phase 1: after the 2x2,

@@ -792,6 +792,16 @@ static bool small_op_ok(const qmk_small_op &o, uint32_t n, bool two) {
 extern "C" int qmk_run_small(float *state, uint32_t n, size_t num_ops, const qmk_small_op *ops,
                              const qmk_small_adjoint *adjoint, void *ws, size_t ws_bytes,
                              void *stream) {
+  uint32_t launches = 0;
+  return qmk_run_small_counted(state, n, num_ops, ops, adjoint, ws, ws_bytes, stream, &launches);
+}
+
+extern "C" int qmk_run_small_counted(float *state, uint32_t n, size_t num_ops,
+                                     const qmk_small_op *ops, const qmk_small_adjoint *adjoint,
+                                     void *ws, size_t ws_bytes, void *stream,
+                                     uint32_t *launches) {
+  if (!launches) return -1;
+  *launches = 0;
   if (!state || n < 1 || n > kMaxN || (num_ops && !ops) || !ws ||
       ws_bytes < qmk_small_workspace_bytes(n))
     return -1;
@@ -818,6 +828,7 @@ extern "C" int qmk_run_small(float *state, uint32_t n, size_t num_ops, const qmk
   auto flush = [&]() -> int {
     if (code.empty()) return 0;
     int rc = 0;
+    *launches += layers.empty() ? 1 : 2;
     if (!layers.empty())
       rc = terms <= static_cast<uint32_t>(kShortTerms)
                ? launch_tables<kShortTerms>(n, layers, real, tables, s)

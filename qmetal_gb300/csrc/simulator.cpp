@@ -788,20 +788,26 @@ class SmallProgram {
 
 }  // namespace
 
-void Simulator::launch_program(const std::vector<qmk_small_op> &ops, const qmk_small_adjoint *adj) {
-  if (ops.empty()) return;
-  check(qmk_run_small(state_, n_, ops.size(), ops.data(), adj,
-                      static_cast<uint8_t *>(ws_) + ws_bytes_, small_ws_bytes_, stream_),
+// Returns the number of kernels launched.
+uint64_t Simulator::launch_program(const std::vector<qmk_small_op> &ops,
+                                   const qmk_small_adjoint *adj) {
+  if (ops.empty()) return 0;
+  uint32_t launches = 0;
+  check(qmk_run_small_counted(state_, n_, ops.size(), ops.data(), adj,
+                              static_cast<uint8_t *>(ws_) + ws_bytes_, small_ws_bytes_, stream_,
+                              &launches),
         "circuit");
+  return launches;
 }
 
 // The plan on a narrow state, its ops in one launch. A dispatch is counted for
 // each plan op. An op the launch cannot take (malformed, or a layer of too
-// many terms) runs, or is refused, by itself in its place.
-void Simulator::run_small(const Plan &p) {
+// many terms) runs, or is refused, by itself in its place. Returns the number of
+// kernels launched.
+uint64_t Simulator::run_small(const Plan &p) {
   SmallProgram prog(n_);
   const uint64_t start = dispatches_;
-  uint64_t extra = 0;   // launches of an op beyond one
+  uint64_t launched = 0, extra = 0;   // extra: launches of an op beyond one
   const auto steps = small_schedule(p);
   for (const ForwardStep &st : steps) {
     if (st.kind == ForwardStep::Group) {
@@ -809,15 +815,17 @@ void Simulator::run_small(const Plan &p) {
     } else if (st.kind == ForwardStep::Permute) {
       prog.map(st.cols, 0);
     } else if (!prog.plan_op(p.ops[st.ops[0]])) {
-      launch_program(prog.ops, nullptr);
+      launched += launch_program(prog.ops, nullptr);
       prog.clear();
       const uint64_t own = dispatches_;
       apply_op_to(state_, p.ops[st.ops[0]]);
+      launched += dispatches_ - own;
       if (dispatches_ > own) extra += dispatches_ - own - 1;
     }
   }
-  launch_program(prog.ops, nullptr);
+  launched += launch_program(prog.ops, nullptr);
   dispatches_ = start + p.ops.size() + extra;
+  return launched;
 }
 
 // Forward pass, samples, co-state and backward sweep of a gradient on a narrow
@@ -908,13 +916,11 @@ bool Simulator::small_gradient(const Circuit &c, const Hamiltonian &h, const Pla
   const qmk_small_adjoint adj{costate_, d_grad_, d_grad_cap_, d_results_};
   if (shots) {
     std::vector<qmk_small_op> head(prog.ops.begin(), prog.ops.begin() + forward_ops);
-    launch_program(head, &adj);
+    dispatches_ += launch_program(head, &adj);
     launch_sample(shots, seed);
     prog.ops.erase(prog.ops.begin(), prog.ops.begin() + forward_ops);
-    dispatches_++;
   }
-  launch_program(prog.ops, &adj);
-  dispatches_++;
+  dispatches_ += launch_program(prog.ops, &adj);
   return true;
 }
 
@@ -1026,8 +1032,8 @@ void Simulator::run_merged(const Plan &p) {
   activate();
   if (small()) {
     const uint64_t own = dispatches_;
-    run_small(p);
-    dispatches_ = own + 1;
+    const uint64_t launched = run_small(p);
+    dispatches_ = own + launched;
     return;
   }
   std::vector<ForwardStep> steps = fold_diagonals(p, merged_schedule(p));

@@ -144,11 +144,11 @@ class Simulator {
   void apply_diag_group_step(const Plan &p, const ForwardStep &st);
   void run_inplace(const Plan &p);
   void run_steps(const Plan &p, const std::vector<ForwardStep> &steps);   // merged_schedule's
-  void run_small(const Plan &p);
+  uint64_t run_small(const Plan &p);
   bool small_gradient(const Circuit &c, const Hamiltonian &h, const Plan &plan, size_t shots,
                       uint64_t seed);
   void fused_gradient(const Circuit &c, const Hamiltonian &h, size_t shots, uint64_t seed);
-  void launch_program(const std::vector<qmk_small_op> &ops, const qmk_small_adjoint *adj);
+  uint64_t launch_program(const std::vector<qmk_small_op> &ops, const qmk_small_adjoint *adj);
   // The state fits one block: circuits run in one launch.
   bool small() const { return small_ws_bytes_ != 0; }
   void pauli_values(const float *state, const Hamiltonian &h, std::vector<double> &vals);
