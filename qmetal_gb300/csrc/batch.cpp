@@ -83,11 +83,14 @@ struct LanesMemory {
   LanesMemory() = default;
   LanesMemory(const LanesMemory &) = delete;
   LanesMemory &operator=(const LanesMemory &) = delete;
-  ~LanesMemory() {
+  ~LanesMemory() { release(); }
+  void release() {
     cudaFree(device);
     if (pinned) cudaFreeHost(pinned);
+    device = pinned = nullptr;
   }
-  // widths[k]: the widest circuit lane k serves. False if it does not fit.
+  // widths[k]: the widest circuit lane k serves. False, holding nothing, if it
+  // does not fit.
   bool allocate(const std::vector<uint32_t> &widths, size_t max_gates, size_t max_shots) {
     size_t bytes = 0;
     std::vector<size_t> at;
@@ -101,6 +104,7 @@ struct LanesMemory {
         cudaMalloc(&device, bytes) != cudaSuccess ||
         cudaMallocHost(&pinned, widths.size() * Simulator::lane_pinned_bytes()) != cudaSuccess) {
       cudaGetLastError();
+      release();
       return false;
     }
     for (size_t k = 0; k < widths.size(); k++) {

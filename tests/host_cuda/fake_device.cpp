@@ -1,0 +1,130 @@
+// A CUDA runtime and kernel layer without a device, for tests of what the host
+// does about memory: allocations are addresses with nothing behind them, every
+// call succeeds unless memory_left or fail_pinned says otherwise, kernels do
+// nothing, and copies to the host are zeros.
+#include "fake_device.hpp"
+
+#include <cuda_runtime_api.h>
+
+#include <cstdlib>
+#include <cstring>
+#include <map>
+#include <mutex>
+
+namespace fake {
+
+std::mutex lock;
+size_t total = size_t(1) << 40, used = 0;
+int fail_pinned = 0;
+size_t used_after_failed_pinned = 0;
+bool pinned_failed = false;
+std::map<uint32_t, int> permutations;
+
+namespace {
+std::map<char *, size_t> blocks;
+char *next = reinterpret_cast<char *>(size_t(1) << 44);
+}  // namespace
+
+}  // namespace fake
+
+using namespace fake;
+
+extern "C" {
+
+cudaError_t cudaMalloc(void **p, size_t bytes) {
+  std::lock_guard<std::mutex> g(lock);
+  if (pinned_failed) {
+    used_after_failed_pinned = used;
+    pinned_failed = false;
+  }
+  if (used + bytes > total) return cudaErrorMemoryAllocation;
+  *p = next;
+  blocks[next] = bytes;
+  next += (bytes + 511) & ~size_t(255);
+  used += bytes;
+  return cudaSuccess;
+}
+cudaError_t cudaFree(void *p) {
+  std::lock_guard<std::mutex> g(lock);
+  const auto it = blocks.find(static_cast<char *>(p));
+  if (it != blocks.end()) {
+    used -= it->second;
+    blocks.erase(it);
+  }
+  return cudaSuccess;
+}
+cudaError_t cudaMemGetInfo(size_t *free_bytes, size_t *all) {
+  std::lock_guard<std::mutex> g(lock);
+  *free_bytes = total - used;
+  *all = total;
+  return cudaSuccess;
+}
+cudaError_t cudaMallocHost(void **p, size_t bytes) {
+  std::lock_guard<std::mutex> g(lock);
+  if (fail_pinned > 0) {
+    fail_pinned--;
+    pinned_failed = true;
+    return cudaErrorMemoryAllocation;
+  }
+  *p = std::calloc(bytes, 1);
+  return cudaSuccess;
+}
+cudaError_t cudaHostAlloc(void **p, size_t bytes, unsigned) { return cudaMallocHost(p, bytes); }
+cudaError_t cudaFreeHost(void *p) {
+  std::free(p);
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void *to, const void *, size_t bytes, cudaMemcpyKind kind, cudaStream_t) {
+  if (kind == cudaMemcpyDeviceToHost) std::memset(to, 0, bytes);
+  return cudaSuccess;
+}
+cudaError_t cudaMemsetAsync(void *, int, size_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaGetDevice(int *d) { return *d = 0, cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetDeviceCount(int *n) { return *n = 1, cudaSuccess; }
+cudaError_t cudaGetDeviceProperties(cudaDeviceProp *p, int) { return *p = {}, cudaSuccess; }
+const char *cudaGetErrorString(cudaError_t) { return "fake"; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { return *s = nullptr, cudaSuccess; }
+cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaSuccess; }
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *g) { return *g = nullptr, cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t *e) { return *e = nullptr, cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { return *e = nullptr, cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { return *ms = 0.0f, cudaSuccess; }
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
+cudaError_t cudaGraphGetNodes(cudaGraph_t, cudaGraphNode_t *, size_t *n) { return *n = 0, cudaSuccess; }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t *e, cudaGraph_t, unsigned long long) {
+  return *e = nullptr, cudaSuccess;
+}
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
+
+// The kernel layer; calls pass more arguments than are named here.
+size_t qmk_workspace_bytes() { return 1u << 20; }
+size_t qmk_sample_workspace_bytes() { return 1u << 20; }
+size_t qmk_small_workspace_bytes(uint32_t n) { return n <= 13 ? 1u << 20 : 0; }
+uint32_t qmk_small_saves() { return 0; }
+int qmk_apply_permutation(float *, const float *, uint32_t n) {
+  std::lock_guard<std::mutex> g(lock);
+  permutations[n]++;
+  return 0;
+}
+void *qmk_wait_counter(void *ws) { return ws; }
+#define LAUNCH(name) int name() { return 0; }
+LAUNCH(qmk_abs2sum) LAUNCH(qmk_adjoint_1q) LAUNCH(qmk_adjoint_diagonal) LAUNCH(qmk_adjoint_group)
+LAUNCH(qmk_apply_1q) LAUNCH(qmk_apply_blocked) LAUNCH(qmk_apply_controlled)
+LAUNCH(qmk_apply_diagonal) LAUNCH(qmk_apply_diagonal_group) LAUNCH(qmk_apply_group)
+LAUNCH(qmk_apply_group_moves) LAUNCH(qmk_apply_phase64) LAUNCH(qmk_apply_stages)
+LAUNCH(qmk_apply_swap) LAUNCH(qmk_dot_re) LAUNCH(qmk_expect_small) LAUNCH(qmk_init_basis)
+LAUNCH(qmk_pauli_accum) LAUNCH(qmk_pauli_accum_local) LAUNCH(qmk_pauli_expect)
+LAUNCH(qmk_run_small_counted) LAUNCH(qmk_sample) LAUNCH(qmk_set_wait_poll_limit)
+LAUNCH(qmk_take_wait_timeouts) LAUNCH(qmk_workspace_init) LAUNCH(qmk_x_expect)
+LAUNCH(qmk_xfield_costate) LAUNCH(qmk_z_expect) LAUNCH(qmk_zdiag_costate)
+
+}  // extern "C"

@@ -1,0 +1,41 @@
+"""A batch lane where device or page-locked memory runs out, on a device that is
+not there (tests/host_cuda)."""
+import os
+import re
+import shutil
+import subprocess
+
+import pytest
+
+import qmetal_gb300 as qm
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+OBJ = os.path.join(os.path.dirname(qm.library_path()), "_build")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+@pytest.fixture(scope="module")
+def client(tmp_path_factory):
+    if shutil.which("g++") is None:
+        pytest.skip("no g++")
+    exe = str(tmp_path_factory.mktemp("lanes") / "lanes")
+    cmd = ["g++", "-std=c++17", "-O1", "-w", "-pthread", "-I" + os.path.join(CUDA, "include")]
+    cmd += [os.path.join(HERE, "host_cuda", f) for f in ("lanes.cpp", "fake_device.cpp")]
+    cmd += [os.path.join(OBJ, f + ".cpp.o") for f in ("simulator", "batch", "schedule", "plan", "circuit")]
+    r = subprocess.run(cmd + ["-o", exe], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-3000:]
+
+    def run(what):
+        out = subprocess.run([exe, what], capture_output=True, text=True, timeout=120)
+        assert out.returncode == 0, out.stderr
+        return {k: int(v) for k, v in re.findall(r"(\w+) (\d+)", out.stdout)}
+
+    return run
+
+
+def test_pinned_memory_fails(client):
+    """The lanes then allocate for themselves, without the shared block beside them."""
+    got = client("pinned")
+    assert got["held"] == 0
+    assert got["wide"] > 0 and got["narrow"] > 0
+    assert got["left"] == 0
