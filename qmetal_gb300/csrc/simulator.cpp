@@ -110,7 +110,7 @@ uint64_t Simulator::recommended_working_set() {
   return total_b;
 }
 
-Simulator::Simulator(uint32_t n) : n_(n), capacity_(n) {
+Simulator::Simulator(uint32_t n) : n_(n) {
   if (n == 0 || n > kMaxQubits)
     throw std::runtime_error("Simulator: num_qubits must be 1.." + std::to_string(kMaxQubits));
   const char *fault = std::getenv("QMETAL_FAULT");
@@ -181,7 +181,7 @@ size_t Simulator::lane_pinned_bytes() { return (kResultSlots + 1) * sizeof(doubl
 
 // A batch lane's simulator of up to n qubits: everything but its stream comes
 // from the batch's memory, so a lane allocates nothing and frees nothing.
-Simulator::Simulator(uint32_t n, const LaneMemory &m) : n_(n), capacity_(n), lane_(m) {
+Simulator::Simulator(uint32_t n, const LaneMemory &m) : n_(n), lane_(m) {
   if (n == 0 || n > kMaxQubits)
     throw std::runtime_error("Simulator: num_qubits must be 1.." + std::to_string(kMaxQubits));
   cuda_check(cudaGetDevice(&device_), "cudaGetDevice");
@@ -222,8 +222,11 @@ Simulator::Simulator(uint32_t n, const LaneMemory &m) : n_(n), capacity_(n), lan
   }
 }
 
+// Buffers that it takes from here on are of this width, and one that a wider
+// state found no room for is asked for again.
 void Simulator::narrow_to(uint32_t n) {
-  if (n == 0 || n > capacity_) throw std::runtime_error("Simulator: wider than its memory");
+  if (n == 0 || n > n_) throw std::runtime_error("Simulator: wider than its memory");
+  if (n < n_) scratch_failed_ = false;
   n_ = n;
   small_ws_bytes_ = qmk_small_workspace_bytes(n);
   invalidate_graphs();
@@ -293,7 +296,7 @@ void Simulator::synchronize() {
 bool Simulator::ensure_scratch() {
   if (scratch_) return true;
   if (scratch_failed_) return false;
-  const size_t bytes = size_t(8) << capacity_;
+  const size_t bytes = dim() * 8;
   size_t free_b = 0, total_b = 0;
   // Keep 2 GiB of headroom for other simulators and the runtime.
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < bytes + (2ull << 30) ||
@@ -320,7 +323,7 @@ float *Simulator::take_buffer() {
   size_t held = 0;
   for (const Checkpoint &c : ckpts_) held += c.buf != nullptr;
   if (held >= ck_limit_) return nullptr;
-  const size_t bytes = size_t(8) << capacity_;
+  const size_t bytes = dim() * 8;
   size_t free_b = 0, total_b = 0;
   float *b = nullptr;
   // Keep 4 GiB of headroom for other simulators and the runtime.

@@ -35,8 +35,8 @@ class Simulator {
   Simulator(uint32_t num_qubits, const LaneMemory &memory);
   static size_t lane_device_bytes(uint32_t num_qubits, size_t max_gates, size_t max_shots);
   static size_t lane_pinned_bytes();
-  // The next circuits have n qubits, at most the simulator's own number. The
-  // state is undefined until it is reset or set.
+  // From here on a simulator of n qubits, at most its present number. The state
+  // is undefined until it is reset or set.
   void narrow_to(uint32_t n);
   ~Simulator();
   Simulator(const Simulator &) = delete;
@@ -190,7 +190,6 @@ class Simulator {
   void invalidate_graphs();
 
   uint32_t n_ = 0;
-  uint32_t capacity_ = 0;               // qubits its buffers hold
   LaneMemory lane_;
   int device_ = 0;
   void *stream_ = nullptr;

@@ -39,3 +39,11 @@ def test_pinned_memory_fails(client):
     assert got["held"] == 0
     assert got["wide"] > 0 and got["narrow"] > 0
     assert got["left"] == 0
+
+
+def test_no_second_buffer_for_the_widest(client):
+    """Narrower requests that have room for theirs use the gather passes."""
+    got = client("scratch")
+    assert got["wide"] == 0
+    assert got["narrow"] > 0
+    assert got["left"] == 0
