@@ -300,13 +300,20 @@ namespace {
 // One way to issue a pending run of one-wire ops and the CX / SWAP gates that
 // follow it: passes of at most `cap` wires >= 6 each (at most four beside
 // wires 0..5), every pass with the gates, in order, that it holds both wires
-// of and that no gate left for later has a wire of.
+// of and that no gate left for later has a wire of. Empty where that takes
+// `most` passes or more.
 std::vector<ForwardStep> move_passes(const WireRun &held, const std::vector<PermGate> &run,
-                                     const std::vector<size_t> &run_ops, uint32_t cap) {
+                                     const std::vector<size_t> &run_ops, uint32_t cap,
+                                     size_t most) {
   std::vector<ForwardStep> out;
-  std::vector<bool> gate_done(run.size(), false), wire_done(held.wires.size(), false);
-  size_t left = run.size() + held.wires.size();
-  while (left) {
+  std::vector<size_t> todo(run.size());   // the run's gates not yet in a pass
+  for (size_t k = 0; k < todo.size(); k++) todo[k] = k;
+  std::vector<bool> wire_done(held.wires.size(), false);
+  size_t wires_left = held.wires.size();
+  uint64_t used = 0;   // by any gate
+  for (const PermGate &g : run) used |= (1ull << g.a) | (1ull << g.b);
+  while (!todo.empty() || wires_left) {
+    if (out.size() + 1 >= most) return {};
     uint64_t tile = 0, blocked = 0;
     uint32_t high = 0;
     bool low = false;
@@ -323,26 +330,39 @@ std::vector<ForwardStep> move_passes(const WireRun &held, const std::vector<Perm
       low = lo;
       return true;
     };
+    // Wires that a further gate of this pass could have: gates after the point
+    // where there are fewer than two need no look.
+    auto usable = [&]() {
+      uint64_t m = tile;
+      if (high < (low ? std::min(cap, 4u) : cap)) m |= ~63ull;
+      if (high <= std::min(cap, 4u)) m |= 63ull;
+      return m & ~blocked;
+    };
     ForwardStep s;
     s.kind = ForwardStep::Moves;
-    for (size_t k = 0; k < run.size(); k++) {
-      if (gate_done[k]) continue;
+    size_t at = 0, left = 0;
+    for (; at < todo.size(); at++) {
+      const size_t k = todo[at];
       const uint64_t w = (1ull << run[k].a) | (1ull << run[k].b);
       if ((w & blocked) || !admit(w)) {
         blocked |= w;
+        todo[left++] = k;
+        if (popc(usable() & used) < 2) {
+          at++;
+          break;
+        }
         continue;
       }
       s.moves.push_back(run[k]);
       s.ops.push_back(run_ops[k]);
-      gate_done[k] = true;
-      left--;
     }
+    todo.erase(todo.begin() + left, todo.begin() + at);
     std::vector<size_t> idx;
     for (size_t i = 0; i < held.wires.size(); i++) {
       if (wire_done[i] || !admit(1ull << held.wires[i])) continue;
       wire_done[i] = true;
       idx.push_back(i);
-      left--;
+      wires_left--;
     }
     std::sort(idx.begin(), idx.end(),
               [&](size_t a, size_t b) { return held.wires[a] < held.wires[b]; });
@@ -435,26 +455,35 @@ std::vector<ForwardStep> inplace_schedule(const Plan &p) {
   std::vector<PermGate> run;
   std::vector<size_t> run_ops;
   auto flush = [&]() {
-    const auto groups = split_run(n, held);
-    std::vector<ForwardStep> best;
-    if (!run.empty() && n >= kMovesMinQubits) {
-      for (uint32_t cap = 4; cap <= 7; cap++) {
-        std::vector<ForwardStep> t = move_passes(held, run, run_ops, cap);
-        if (best.empty() || t.size() < best.size()) best = std::move(t);
+    // A long run in pieces, which keeps the search for passes linear in it.
+    for (size_t from = 0; from < run.size() || !held.wires.empty(); from += kMovesPiece) {
+      const size_t to = std::min(run.size(), from + kMovesPiece);
+      const std::vector<PermGate> piece(run.begin() + from, run.begin() + to);
+      const std::vector<size_t> ops(run_ops.begin() + from, run_ops.begin() + to);
+      const auto groups = split_run(n, held);
+      // A pass reads and writes the state (2 S); a CX or SWAP of its own moves S.
+      std::vector<ForwardStep> best;
+      if (!piece.empty() && n >= kMovesMinQubits) {
+        size_t most = groups.size() + piece.size() / 2 + 1;
+        for (uint32_t cap = 4; cap <= 7; cap++) {
+          std::vector<ForwardStep> t = move_passes(held, piece, ops, cap, most);
+          if (t.empty()) continue;
+          most = t.size();
+          best = std::move(t);
+        }
       }
-    }
-    // A pass reads and writes the state (2 S); a CX or SWAP of its own moves S.
-    if (!best.empty() && 2 * best.size() <= 2 * groups.size() + run.size()) {
-      for (ForwardStep &s : best) out.push_back(std::move(s));
-    } else {
-      for (const auto &pass : groups) out.push_back(group_step(held, pass));
-      for (size_t i : run_ops) {
-        ForwardStep s;
-        s.ops = {i};
-        out.push_back(std::move(s));
+      if (!best.empty()) {
+        for (ForwardStep &s : best) out.push_back(std::move(s));
+      } else {
+        for (const auto &pass : groups) out.push_back(group_step(held, pass));
+        for (size_t i : ops) {
+          ForwardStep s;
+          s.ops = {i};
+          out.push_back(std::move(s));
+        }
       }
+      held.clear();
     }
-    held.clear();
     run.clear();
     run_ops.clear();
   };

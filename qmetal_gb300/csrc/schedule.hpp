@@ -89,6 +89,7 @@ std::vector<ForwardStep> merged_schedule(const Plan &p);
 // on: alone a stage costs 2 S for its gate and S for its fan, the pass 2 S to
 // 3 S in time.
 constexpr uint32_t kMovesMinQubits = 13;
+constexpr size_t kMovesPiece = 512;   // gates of a run shared out at once
 constexpr uint32_t kStagesMinQubits = 13;
 std::vector<ForwardStep> inplace_schedule(const Plan &p);
 
