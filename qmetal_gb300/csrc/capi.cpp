@@ -174,7 +174,6 @@ int qm_circuit_add_many(qm_circuit c, size_t count, const int *kinds, const uint
     return -1;
   }
   return guarded([&] {
-    c->c.ops.reserve(c->c.ops.size() + count);
     for (size_t k = 0; k < count; k++) {
       const uint32_t nq = num_qubits[k], np = num_params[k];
       c->c.add(gate_of(c->c.num_qubits, static_cast<qm_gate_kind>(kinds[k]), qubits, nq, params, np));
