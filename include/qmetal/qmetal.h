@@ -166,19 +166,24 @@ size_t qm_circuit_plan_export(qm_circuit c, int collapse_1q_windows,
 
 /* The executor's launch schedules, computed on the host only (no device
  * needed), in a flat double layout:
- *   which = 0: the merged forward pass of the default plan (gradients, and
- *              qm_run_merged unless which = 3 moves fewer bytes);
+ *   which = 0: the merged forward pass of the default plan, every diagonal
+ *              layer by itself;
  *   which = 1: the block-wise backward sweep (qm_energy_and_gradient) with
  *              `tile_high` wires >= 6 per window pass (1..6);
  *   which = 2: the co-state lambda = H psi of `h` for the circuit's width;
- *   which = 3: the default plan as qm_run launches it, in place;
- *   which = 4: the default plan as one launch runs it, up to 13 qubits (its
- *              groups hold up to three wires).
+ *   which = 3: the default plan as qm_run launches it from 14 qubits on, in place;
+ *   which = 4: the default plan as one launch runs it, qm_run up to 13 qubits and
+ *              gradients up to 12 (its groups hold up to three wires);
+ *   which = 5: which = 0 with diagonal layers that take wires >= 13 of the groups
+ *              after them along, as gradients launch it from 13 qubits on and
+ *              qm_run_merged from 14 on unless which = 3 moves fewer bytes.
  * Forward steps: 0 group (nw, then wire and a row-major 2x2 as re/im pairs per
  * wire), 1 gather (n, cols[n], off, nops, plan op indices), 2 plan op (index),
  * 3 group with CX / SWAP gates after it (nw and its matrices as 0, then ngates
  * and swap 0/1, a, b per gate), 4 stages (ns, then wire, has matrix, its 2x2, phase
- * 0 none / 1 after / 2 before the 2x2, and n angles per stage). Backward steps: 0 window tile (nops, then wire, inverse 2x2, generator 0-3,
+ * 0 none / 1 after / 2 before the 2x2, and n angles per stage), 5 diagonal layer
+ * and then a group in the same pass (the layer's plan op index, then as 0).
+ * Backward steps: 0 window tile (nops, then wire, inverse 2x2, generator 0-3,
  * gradient slot per op), 1 diagonal block (undo, nt, (mask, angle) x nt,
  * global phase, ng, (Z mask, slot) x ng), 2 gather undo (n, cols[n], off,
  * ngates, gate indices), 3 gate undo (index). Co-state steps: 0 Z strings

@@ -318,9 +318,11 @@ class Circuit:
         """The executor's launch schedule as the flat double list of
         qm_schedule_export: which is "forward" (merged forward pass),
         "backward" (block-wise adjoint sweep) or "costate" (lambda = H psi of
-        `hamiltonian`) or "inplace" / "small" (Simulator.run from 14 qubits / below).
-        Host only; needs no device."""
-        code = {"forward": 0, "backward": 1, "costate": 2, "inplace": 3, "small": 4}[which]
+        `hamiltonian`), "inplace" / "small" (Simulator.run from 14 qubits / below)
+        or "gradient" (the forward pass of gradients from 13 qubits). Host only;
+        needs no device."""
+        code = {"forward": 0, "backward": 1, "costate": 2, "inplace": 3, "small": 4,
+                "gradient": 5}[which]
         h = hamiltonian._c() if hamiltonian is not None else None
         hp = byref(h) if h is not None else None
         n = int(_schedule_export(self._h, hp, code, int(tile_high), None, 0))

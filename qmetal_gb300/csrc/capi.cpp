@@ -419,7 +419,12 @@ size_t qm_schedule_export(qm_circuit c, const qm_hamiltonian *h, int which, uint
       case 2: serialise_schedule(costate_schedule(hamiltonian_of(h), n), v); break;
       case 3: serialise_schedule(inplace_schedule(build_plan(c->c, FusionOptions{})), n, v); break;
       case 4: serialise_schedule(small_schedule(build_plan(c->c, FusionOptions{})), n, v); break;
-      default: throw std::runtime_error("schedule: which must be 0..4");
+      case 5: {
+        const Plan p = build_plan(c->c, FusionOptions{});
+        serialise_schedule(fold_diagonals(p, merged_schedule(p)), n, v);
+        break;
+      }
+      default: throw std::runtime_error("schedule: which must be 0..5");
     }
     if (out && cap) std::memcpy(out, v.data(), sizeof(double) * std::min(cap, v.size()));
     return v.size();
