@@ -117,7 +117,7 @@ int qmk_apply_diagonal(float *state, uint32_t n, uint32_t num_terms,
  *               invertible map: a run of CX / SWAP gates)
  *   LAYER       a diagonal layer (masks of any weight), as qmk_apply_diagonal;
  *               conj: its conjugate
- * and with `adjoint` also
+ * and with `adjoint` (up to QMK_SMALL_MAX_ADJOINT qubits) also
  *   both        the op on the state and the co-state
  *   save k      MAP: keep the state from before it as number k (from 1, up to
  *               qmk_small_saves(n)); with `both`: the state comes from number
@@ -134,6 +134,7 @@ int qmk_apply_diagonal(float *state, uint32_t n, uint32_t num_terms,
  * kept states. Serves the reference's dispatches gate by gate
  * (kernels.metal:48-218, 313-408). */
 #define QMK_SMALL_MAX_QUBITS 13
+#define QMK_SMALL_MAX_ADJOINT 12
 #define QMK_SMALL_MAX_TERMS 3000   /* per op */
 #define QMK_SMALL_MAX_WINDOW 24
 enum {

@@ -17,9 +17,9 @@
 //
 // Bound by latency: a barrier, shared-memory round trip and up to three
 // dependent 2x2s an op. The 9-qubit U3 circuit of depth 10 with its read-out:
-// 310 -> 80 us; gradients of four HEA layers, host work and read-out in, at 6, 10
-// and 12 qubits 213 -> 112, 233 -> 163 and 304 -> 254 us. At 13 qubits, where one
-// block took 369 us and the launches 334, a gradient goes by launches.
+// 310 -> 77 us; gradients of four HEA layers, host work and read-out in, at 6, 10
+// and 12 qubits 213 -> 108, 233 -> 157 and 304 -> 247 us. At 13 qubits, where one
+// block took 360 us and the launches take 297, a gradient goes by launches.
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -34,15 +34,15 @@ using qmk_host::launch_status;
 
 namespace {
 
-constexpr uint32_t kMaxN = QMK_SMALL_MAX_QUBITS;
+constexpr uint32_t kMaxN = QMK_SMALL_MAX_QUBITS, kMaxN2 = QMK_SMALL_MAX_ADJOINT;
 // Phase tables per launch and states kept: what fits with the rest of a
 // simulator's workspace in 2 MiB, the device's allocation unit (a second one
 // takes 35 us of a simulator's creation).
 constexpr uint32_t kMaxLayers = 32;
 constexpr uint32_t layers_of(uint32_t n) { return n >= 13 ? 16 : kMaxLayers; }
-constexpr uint32_t saves_of(uint32_t n) { return n >= 13 ? 8 : n >= 12 ? 16 : 32; }
-// Widest blocks: eight amplitudes a thread at 13 qubits, sixteen of each state
-// with the co-state.
+constexpr uint32_t saves_of(uint32_t n) { return n > kMaxN2 ? 0 : n >= 12 ? 16 : 32; }
+// Widest blocks: eight amplitudes a thread at 13 qubits, eight of each state at
+// 12 with the co-state.
 constexpr unsigned kSmallThreads = 1024, kSmallThreads2 = 512;
 // Warps beside a gradient's threads (while those are at most 256) that add up
 // the rows of partial sums, so that no working warp waits for them (6 qubits,
@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(TWO ? kSmallThreads2 : kSmallThreads)
 k_small(float2 *__restrict__ st, uint32_t n, uint32_t step,
         const __grid_constant__ Code<WORDS> code, const float2 *__restrict__ tables, SmallOut out) {
   extern __shared__ __align__(16) float2 amp[];
-  constexpr int E = TWO ? 16 : 8;   // most amplitudes a thread
+  constexpr int E = 8;   // most amplitudes a thread
   const uint32_t dim = 1u << n;
   // A helper warp's index is past every loop over amplitudes.
   const bool helper = TWO && threadIdx.x >= step;
@@ -532,7 +532,7 @@ k_small(float2 *__restrict__ st, uint32_t n, uint32_t step,
             if (TWO && kept && states == 1) kept[y] = x[slot(y)];
             uint32_t from = base;
 #pragma unroll
-            for (int j = 0; j < 4; j++)
+            for (int j = 0; j < 3; j++)
               if ((e >> j) & 1) from ^= high[j];
             r[e] = x[slot(from)];
           }
@@ -666,7 +666,7 @@ int launch_small(float *state, uint32_t n, const std::vector<uint32_t> &code, co
     if (!opted[dev]) {   // the opt-in above 48 KiB is per device
       const cudaError_t e =
           cudaFuncSetAttribute(k_small<WORDS, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(bytes(kMaxN, most)));
+                               static_cast<int>(bytes(TWO ? kMaxN2 : kMaxN, most)));
       if (e != cudaSuccess) return static_cast<int>(e);
       opted[dev] = true;
     }
@@ -805,7 +805,7 @@ extern "C" int qmk_run_small_counted(float *state, uint32_t n, size_t num_ops,
   if (!state || n < 1 || n > kMaxN || (num_ops && !ops) || !ws ||
       ws_bytes < qmk_small_workspace_bytes(n))
     return -1;
-  if (adjoint && (!adjoint->costate || !adjoint->grad || !adjoint->energy)) return -1;
+  if (adjoint && (n > kMaxN2 || !adjoint->costate || !adjoint->grad || !adjoint->energy)) return -1;
   // Everything is checked before anything is launched.
   for (size_t k = 0; k < num_ops; k++) {
     if (!small_op_ok(ops[k], n, adjoint != nullptr)) return -1;

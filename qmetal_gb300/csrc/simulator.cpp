@@ -30,8 +30,7 @@ constexpr uint32_t kTermsPerPass = 16;
 constexpr uint32_t kSmallExpect = 14;    // widest state whose strings go a block each
 constexpr size_t kSmallTerms = 64;       // strings per such launch
 constexpr size_t kZTermsPerPass = 32;
-constexpr uint32_t kSmallGradient = 12;  // widest gradient in one block (four HEA layers at 13
-                                         // qubits: 369 us there, 334 by launches)
+constexpr uint32_t kSmallGradient = QMK_SMALL_MAX_ADJOINT;   // widest gradient in one block
 
 cudaStream_t S(void *p) { return static_cast<cudaStream_t>(p); }
 
