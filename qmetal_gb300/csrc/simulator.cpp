@@ -161,9 +161,13 @@ namespace {
 
 size_t padded(size_t bytes) { return (bytes + 255) & ~size_t(255); }
 
-// The widest workspace for narrow states that a simulator of up to n qubits needs.
+// The largest workspace for narrow states that a simulator of up to n qubits
+// needs (12 qubits need more than 13, which keep no states).
 size_t small_bytes_up_to(uint32_t n) {
-  return qmk_small_workspace_bytes(std::min<uint32_t>(n, QMK_SMALL_MAX_QUBITS));
+  size_t most = 0;
+  for (uint32_t w = 1; w <= std::min<uint32_t>(n, QMK_SMALL_MAX_QUBITS); w++)
+    most = std::max(most, qmk_small_workspace_bytes(w));
+  return most;
 }
 
 }  // namespace

@@ -4,6 +4,8 @@
 // nothing, and copies to the host are zeros.
 #include "fake_device.hpp"
 
+#include "../../include/qmetal/qmetal_kernels.h"
+
 #include <cuda_runtime_api.h>
 
 #include <cstdlib>
@@ -15,7 +17,7 @@ namespace fake {
 
 std::mutex lock;
 size_t total = size_t(1) << 40, used = 0;
-int fail_pinned = 0;
+int fail_pinned = 0, small_runs = 0, overlaps = 0;
 size_t used_after_failed_pinned = 0;
 bool pinned_failed = false;
 std::map<uint32_t, int> permutations;
@@ -105,26 +107,31 @@ cudaError_t cudaGraphInstantiate(cudaGraphExec_t *e, cudaGraph_t, unsigned long 
 }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
 
-// The kernel layer; calls pass more arguments than are named here.
-size_t qmk_workspace_bytes() { return 1u << 20; }
-size_t qmk_sample_workspace_bytes() { return 1u << 20; }
-size_t qmk_small_workspace_bytes(uint32_t n) { return n <= 13 ? 1u << 20 : 0; }
-uint32_t qmk_small_saves() { return 0; }
-int qmk_apply_permutation(float *, const float *, uint32_t n) {
+// The kernel layer, but for the calls of fake_kernels.c.
+size_t qmk_workspace_bytes(uint32_t) { return 1u << 20; }
+size_t qmk_sample_workspace_bytes(uint32_t) { return 1u << 20; }
+uint32_t qmk_small_saves(uint32_t) { return 0; }
+// Not growing with the width, as the real one.
+size_t qmk_small_workspace_bytes(uint32_t n) { return n > 13 ? 0 : n == 12 ? 3u << 19 : 1u << 20; }
+int qmk_apply_permutation(float *, const float *, uint32_t n, const uint64_t *, uint64_t, void *) {
   std::lock_guard<std::mutex> g(lock);
   permutations[n]++;
   return 0;
 }
-void *qmk_wait_counter(void *ws) { return ws; }
-#define LAUNCH(name) int name() { return 0; }
-LAUNCH(qmk_abs2sum) LAUNCH(qmk_adjoint_1q) LAUNCH(qmk_adjoint_diagonal) LAUNCH(qmk_adjoint_group)
-LAUNCH(qmk_apply_1q) LAUNCH(qmk_apply_blocked) LAUNCH(qmk_apply_controlled)
-LAUNCH(qmk_apply_diagonal) LAUNCH(qmk_apply_diagonal_group) LAUNCH(qmk_apply_group)
-LAUNCH(qmk_apply_group_moves) LAUNCH(qmk_apply_phase64) LAUNCH(qmk_apply_stages)
-LAUNCH(qmk_apply_swap) LAUNCH(qmk_dot_re) LAUNCH(qmk_expect_small) LAUNCH(qmk_init_basis)
-LAUNCH(qmk_pauli_accum) LAUNCH(qmk_pauli_accum_local) LAUNCH(qmk_pauli_expect)
-LAUNCH(qmk_run_small_counted) LAUNCH(qmk_sample) LAUNCH(qmk_set_wait_poll_limit)
-LAUNCH(qmk_take_wait_timeouts) LAUNCH(qmk_workspace_init) LAUNCH(qmk_x_expect)
-LAUNCH(qmk_xfield_costate) LAUNCH(qmk_z_expect) LAUNCH(qmk_zdiag_costate)
-
+unsigned int *qmk_wait_counter(void *ws) { return static_cast<unsigned int *>(ws); }
+int qmk_run_small_counted(float *, uint32_t n, size_t, const qmk_small_op *,
+                          const qmk_small_adjoint *adj, void *ws, size_t bytes, void *,
+                          uint32_t *launches) {
+  std::lock_guard<std::mutex> g(lock);
+  small_runs++;
+  *launches = 1;
+  const char *from = static_cast<char *>(ws), *to = from + bytes;
+  const auto in = [&](const void *p, size_t size) {
+    const char *b = static_cast<const char *>(p);
+    return b < to && b + size > from;
+  };
+  if (adj && (in(adj->costate, size_t(8) << n) || in(adj->grad, 8 * adj->num_grad) || in(adj->energy, 8)))
+    overlaps++;
+  return 0;
+}
 }  // extern "C"

@@ -23,8 +23,8 @@ Circuit ladders(uint32_t n) {
 }  // namespace
 
 int main(int argc, char **argv) {
-  const bool pinned = argc > 1 && std::strcmp(argv[1], "pinned") == 0;
-  const Circuit wide = ladders(20), narrow = ladders(16);
+  const char *what = argc > 1 ? argv[1] : "";
+  const Circuit wide = ladders(20), narrow = ladders(std::strcmp(what, "narrow") ? 16 : 12);
   Hamiltonian h;
   h.add(1.0, PauliString::single('Z', 0));
   std::vector<double> g0(wide.size()), g1(narrow.size());
@@ -34,12 +34,14 @@ int main(int argc, char **argv) {
   items[1].circuit = &narrow;
   items[1].grad = g1.data();
   for (BatchItem &it : items) it.hamiltonian = &h;
-  if (pinned) fake::fail_pinned = 1;
+  if (!std::strcmp(what, "pinned")) fake::fail_pinned = 1;
   // The lane's memory, 2 GiB of headroom, and room for a second buffer of 16
   // qubits (512 KiB) but not of 20 (8 MiB).
-  else fake::total = Simulator::lane_device_bytes(20, wide.size(), 0) + (size_t(2) << 30) + (4u << 20);
+  if (!std::strcmp(what, "scratch"))
+    fake::total = Simulator::lane_device_bytes(20, wide.size(), 0) + (size_t(2) << 30) + (4u << 20);
   run_batch(items, BatchMode::Lanes, 1);
-  std::printf("wide %d narrow %d held %zu left %zu\n", fake::permutations[20],
-              fake::permutations[16], fake::used_after_failed_pinned, fake::used);
+  std::printf("wide %d narrow %d held %zu left %zu small %d overlaps %d\n",
+              fake::permutations[20], fake::permutations[16], fake::used_after_failed_pinned,
+              fake::used, fake::small_runs, fake::overlaps);
   return 0;
 }

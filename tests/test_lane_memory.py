@@ -19,9 +19,13 @@ def client(tmp_path_factory):
     if shutil.which("g++") is None:
         pytest.skip("no g++")
     exe = str(tmp_path_factory.mktemp("lanes") / "lanes")
+    r = subprocess.run(["gcc", "-w", "-c", os.path.join(HERE, "host_cuda", "fake_kernels.c"), "-o",
+                        exe + ".kernels.o"], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-3000:]
     cmd = ["g++", "-std=c++17", "-O1", "-w", "-pthread", "-I" + os.path.join(CUDA, "include")]
     cmd += [os.path.join(HERE, "host_cuda", f) for f in ("lanes.cpp", "fake_device.cpp")]
     cmd += [os.path.join(OBJ, f + ".cpp.o") for f in ("simulator", "batch", "schedule", "plan", "circuit")]
+    cmd.append(exe + ".kernels.o")
     r = subprocess.run(cmd + ["-o", exe], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-3000:]
 
@@ -46,4 +50,11 @@ def test_no_second_buffer_for_the_widest(client):
     got = client("scratch")
     assert got["wide"] == 0
     assert got["narrow"] > 0
+    assert got["left"] == 0
+
+
+def test_memory_of_a_narrow_request(client):
+    """A lane's one-launch workspace lies beside the rest of its memory at each width."""
+    got = client("narrow")
+    assert got["small"] > 0 and got["overlaps"] == 0
     assert got["left"] == 0
