@@ -30,6 +30,7 @@ constexpr uint32_t kTermsPerPass = 16;
 constexpr uint32_t kSmallExpect = 14;    // widest state whose strings go a block each
 constexpr size_t kSmallTerms = 64;       // strings per such launch
 constexpr size_t kZTermsPerPass = 32;
+constexpr size_t kFewSmallSteps = 5;     // three launches of 13 wires in the one-launch steps
 constexpr uint32_t kSmallGradient = QMK_SMALL_MAX_ADJOINT;   // widest gradient in one block
 
 cudaStream_t S(void *p) { return static_cast<cudaStream_t>(p); }
@@ -494,9 +495,9 @@ void Simulator::run(const Circuit &c) {
   run_inplace(build_plan(c, FusionOptions{}));
 }
 
-void Simulator::run_inplace(const Plan &p) {
+void Simulator::run_inplace(const Plan &p, bool replayed) {
   if (small()) {
-    run_small(p);
+    run_narrow(p, replayed);
     return;
   }
   for (const ForwardStep &st : inplace_schedule(p)) {
@@ -806,15 +807,51 @@ uint64_t Simulator::launch_program(const std::vector<qmk_small_op> &ops,
   return launches;
 }
 
+namespace {
+
+// A plan op by itself, in launches of the least kind: a diagonal layer of more
+// than one term takes the time of four (its table and its pass, against 10 us in
+// all in the one launch).
+size_t launches_alone(const PlanOp &op) {
+  return op.kind == PlanOp::Kind::DiagonalLayer && !(op.masks.size() == 1 && op.global_phase == 0.0)
+             ? 4 : 1;
+}
+
+// As many launches as are no slower than the one launch of k_small, whose
+// block loads and stores the state and takes its ops from shared memory: us by
+// launches and in one, 1 to 4 ops of a gate each: 8 qubits 9.8, 12.6, 15.5, 18.6
+// and 13.7, 15.0, 15.3, 16.2; 13 qubits 10.3, 13.9, 17.7, 21.5 and 15.1, 17.6,
+// 19.6, 20.3; 2 qubits 9.7, 12.3 and 11.4, 12.4. In a graph that is replayed a
+// launch is 1.2 us and the limits are higher (13 qubits, 3 and 8 ops: 12.5, 18.6
+// and 16.0, 22.8; 8 qubits, 2 to 4: 9.1, 10.9, 12.1 and 11.3, 11.9, 12.2).
+size_t few_launches(uint32_t n, bool replayed = false) {
+  if (replayed) return n >= 13 ? 8 : n >= 5 ? 3 : 2;
+  return n >= 13 ? 3 : n >= 5 ? 2 : 1;
+}
+
+}  // namespace
+
+// A plan on a narrow state: op by op if it is of a launch or two, else in one.
+void Simulator::run_narrow(const Plan &p, bool replayed) {
+  const size_t few = few_launches(n_, replayed);
+  size_t launches = 0;
+  for (const PlanOp &op : p.ops)
+    if ((launches += launches_alone(op)) > few) break;
+  if (launches > few) {
+    run_small(p, small_schedule(p));
+    return;
+  }
+  for (const PlanOp &op : p.ops) apply_op_to(state_, op);
+}
+
 // The plan on a narrow state, its ops in one launch. A dispatch is counted for
 // each plan op. An op the launch cannot take (malformed, or a layer of too
 // many terms) runs, or is refused, by itself in its place. Returns the number of
 // kernels launched.
-uint64_t Simulator::run_small(const Plan &p) {
+uint64_t Simulator::run_small(const Plan &p, const std::vector<ForwardStep> &steps) {
   SmallProgram prog(n_);
   const uint64_t start = dispatches_;
   uint64_t launched = 0, extra = 0;   // extra: launches of an op beyond one
-  const auto steps = small_schedule(p);
   for (const ForwardStep &st : steps) {
     if (st.kind == ForwardStep::Group) {
       prog.group(st.wires.data(), static_cast<uint32_t>(st.wires.size()), st.mats.data());
@@ -950,7 +987,7 @@ void Simulator::run(const Plan &p) {
   if (p.num_qubits != n_) throw std::runtime_error("plan/simulator size mismatch");
   activate();
   if (small()) {
-    run_small(p);
+    run_narrow(p);
     return;
   }
   for (const PlanOp &op : p.ops) apply_op_to(state_, op);
@@ -1008,7 +1045,7 @@ void Simulator::run_cached(const Circuit &c) {
   cuda_check(cudaStreamBeginCapture(S(stream_), cudaStreamCaptureModeThreadLocal), "graph capture");
   cudaGraph_t graph = nullptr;
   try {
-    run_inplace(plan);
+    run_inplace(plan, true);
   } catch (...) {
     cudaStreamEndCapture(S(stream_), &graph);
     if (graph) cudaGraphDestroy(graph);
@@ -1037,8 +1074,19 @@ void Simulator::run_merged(const Plan &p) {
   if (p.num_qubits != n_) throw std::runtime_error("plan/simulator size mismatch");
   activate();
   if (small()) {
+    const std::vector<ForwardStep> steps = small_schedule(p);
+    if (steps.size() <= kFewSmallSteps) {   // (which may be passes of more wires, or one gather)
+      const std::vector<ForwardStep> merged = merged_schedule(p);
+      size_t launches = 0;
+      for (const ForwardStep &st : merged)
+        launches += st.kind == ForwardStep::Op ? launches_alone(p.ops[st.ops[0]]) : 1;
+      if (launches <= few_launches(n_)) {
+        run_steps(p, merged);
+        return;
+      }
+    }
     const uint64_t own = dispatches_;
-    const uint64_t launched = run_small(p);
+    const uint64_t launched = run_small(p, steps);
     dispatches_ = own + launched;
     return;
   }

@@ -142,9 +142,10 @@ class Simulator {
   void apply_group_step(const ForwardStep &st);
   void apply_stages_step(const ForwardStep &st);
   void apply_diag_group_step(const Plan &p, const ForwardStep &st);
-  void run_inplace(const Plan &p);
+  void run_inplace(const Plan &p, bool replayed = false);   // replayed: under capture
   void run_steps(const Plan &p, const std::vector<ForwardStep> &steps);   // merged_schedule's
-  uint64_t run_small(const Plan &p);
+  void run_narrow(const Plan &p, bool replayed = false);
+  uint64_t run_small(const Plan &p, const std::vector<ForwardStep> &steps);
   bool small_gradient(const Circuit &c, const Hamiltonian &h, const Plan &plan, size_t shots,
                       uint64_t seed);
   void fused_gradient(const Circuit &c, const Hamiltonian &h, size_t shots, uint64_t seed);

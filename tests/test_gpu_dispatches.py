@@ -27,7 +27,8 @@ def test_counts():
     for c in (short, long, layers):
         assert _counted(sim, sim.run, c) == c.plan_size()
     rx = W.to_circuit(n, [(W.RX, (q,), (0.2,)) for q in range(n)])
-    assert _counted(sim, sim.run_merged, rx) == 1
+    assert _counted(sim, sim.run_merged, rx) <= 2          # by itself where that is a launch or two
+    assert _counted(sim, sim.run_merged, W.to_circuit(n, W.hea(n, 2))) == 1
     for c in (short, layers):                              # the layers' tables, then the circuit
         assert _counted(sim, sim.run_merged, c) == 2
     assert _counted(sim, sim.run_merged, long) >= 6
