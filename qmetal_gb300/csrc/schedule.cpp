@@ -448,9 +448,36 @@ size_t match_stages(const Plan &p, size_t first, ForwardStep &step) {
 
 }  // namespace
 
-std::vector<ForwardStep> inplace_schedule(const Plan &p) {
+namespace {
+
+double step_cost(const Plan &p, const ForwardStep &st) {
+  if (st.kind == ForwardStep::Stages) return 2.7;
+  if (st.kind != ForwardStep::Op) return 2.0;
+  const PlanOp &op = p.ops[st.ops[0]];
+  const bool half = op.kind == PlanOp::Kind::Controlled1q || op.kind == PlanOp::Kind::Swap ||
+                    fan_centres(op, p.num_qubits) != 0;
+  return op.kind == PlanOp::Kind::CCX ? 0.5 : half ? 1.0 : 2.0;
+}
+
+}  // namespace
+
+double schedule_cost(const Plan &p, const std::vector<ForwardStep> &steps) {
+  double cost = 0.0;
+  for (const ForwardStep &st : steps) cost += step_cost(p, st);
+  return cost;
+}
+
+namespace {
+
+// inplace_schedule() before diagonal layers take wires along; false, with `out`
+// unfinished, once it costs `most` or more.
+bool inplace_steps(const Plan &p, double most, std::vector<ForwardStep> &out) {
   const uint32_t n = p.num_qubits;
-  std::vector<ForwardStep> out;
+  double spent = 0.0;
+  auto emit = [&](ForwardStep &&s) {
+    spent += step_cost(p, s);
+    out.push_back(std::move(s));
+  };
   WireRun held;
   std::vector<PermGate> run;
   std::vector<size_t> run_ops;
@@ -464,28 +491,32 @@ std::vector<ForwardStep> inplace_schedule(const Plan &p) {
       // A pass reads and writes the state (2 S); a CX or SWAP of its own moves S.
       std::vector<ForwardStep> best;
       if (!piece.empty() && n >= kMovesMinQubits) {
-        size_t most = groups.size() + piece.size() / 2 + 1;
+        double passes = static_cast<double>(groups.size() + piece.size() / 2 + 1);
+        passes = std::min(passes, std::max(0.0, std::ceil((most - spent) / 2.0)));
+        size_t fewer = static_cast<size_t>(passes);   // than so many
         for (uint32_t cap = 4; cap <= 7; cap++) {
-          std::vector<ForwardStep> t = move_passes(held, piece, ops, cap, most);
+          std::vector<ForwardStep> t = move_passes(held, piece, ops, cap, fewer);
           if (t.empty()) continue;
-          most = t.size();
+          fewer = t.size();
           best = std::move(t);
         }
       }
       if (!best.empty()) {
-        for (ForwardStep &s : best) out.push_back(std::move(s));
+        for (ForwardStep &s : best) emit(std::move(s));
       } else {
-        for (const auto &pass : groups) out.push_back(group_step(held, pass));
+        if (spent + 2.0 * groups.size() + piece.size() >= most) return false;
+        for (const auto &pass : groups) emit(group_step(held, pass));
         for (size_t i : ops) {
           ForwardStep s;
           s.ops = {i};
-          out.push_back(std::move(s));
+          emit(std::move(s));
         }
       }
       held.clear();
     }
     run.clear();
     run_ops.clear();
+    return spent < most;
   };
   for (size_t i = 0; i < p.ops.size(); i++) {
     const PlanOp &op = p.ops[i];
@@ -493,8 +524,8 @@ std::vector<ForwardStep> inplace_schedule(const Plan &p) {
     if (n >= kStagesMinQubits && i + 1 < p.ops.size() &&
         (op.kind == PlanOp::Kind::Dense1q || op.kind == PlanOp::Kind::DiagonalLayer)) {
       if (const size_t taken = match_stages(p, i, stages)) {
-        flush();
-        out.push_back(std::move(stages));
+        if (!flush()) return false;
+        emit(std::move(stages));
         i += taken - 1;
         continue;
       }
@@ -508,20 +539,53 @@ std::vector<ForwardStep> inplace_schedule(const Plan &p) {
     const cdouble *m = nullptr;
     size_t count = 0;
     if (!one_wire_op(op, n, w, m, count)) {
-      flush();
+      if (!flush()) return false;
       ForwardStep s;
       s.ops = {i};
-      out.push_back(std::move(s));
+      emit(std::move(s));
       continue;
     }
     bool later = !run.empty();
     for (size_t j = 0; j < count; j++) later = later || held.holds(w[j]);
-    if (later) flush();
+    if (later && !flush()) return false;
     for (size_t j = 0; j < count; j++) held.add(w[j], m + 4 * j);
   }
-  flush();
+  return flush();
+}
+
+// Does inplace_schedule() do anything that merged_schedule() does not: carry
+// moves, or take single gates and fans as stages?
+bool inplace_differs(const Plan &p) {
+  bool before = false;   // a single gate or a fan was the last op
+  for (const PlanOp &op : p.ops) {
+    if (is_wire_move(op, p.num_qubits)) return true;
+    const bool stage = op.kind == PlanOp::Kind::Dense1q || fan_centres(op, p.num_qubits) != 0;
+    if (stage && before) return true;
+    before = stage;
+  }
+  return false;
+}
+
+}  // namespace
+
+std::vector<ForwardStep> inplace_schedule(const Plan &p) {
+  std::vector<ForwardStep> out;
+  inplace_steps(p, HUGE_VAL, out);
   return fold_diagonals(p, std::move(out));
 }
+
+std::vector<ForwardStep> run_merged_schedule(const Plan &p) {
+  std::vector<ForwardStep> steps = fold_diagonals(p, merged_schedule(p));
+  if (!inplace_differs(p)) return steps;
+  const double cost = schedule_cost(p, steps);
+  double folds = 0.0;   // what the folding of layers may still save
+  for (const PlanOp &op : p.ops) folds += op.kind == PlanOp::Kind::DiagonalLayer ? 4.0 : 0.0;
+  std::vector<ForwardStep> inplace;
+  if (!inplace_steps(p, cost + folds, inplace)) return steps;
+  inplace = fold_diagonals(p, std::move(inplace));
+  return schedule_cost(p, inplace) < cost ? inplace : steps;
+}
+
 
 std::vector<ForwardStep> fold_diagonals(const Plan &p, std::vector<ForwardStep> steps) {
   const uint32_t n = p.num_qubits;
@@ -583,23 +647,6 @@ std::vector<ForwardStep> fold_diagonals(const Plan &p, std::vector<ForwardStep> 
     i = j - 1;
   }
   return out;
-}
-
-double schedule_cost(const Plan &p, const std::vector<ForwardStep> &steps) {
-  double cost = 0.0;
-  for (const ForwardStep &st : steps) {
-    if (st.kind == ForwardStep::Stages) {
-      cost += 2.7;
-    } else if (st.kind != ForwardStep::Op) {
-      cost += 2.0;
-    } else {
-      const PlanOp &op = p.ops[st.ops[0]];
-      const bool half = op.kind == PlanOp::Kind::Controlled1q || op.kind == PlanOp::Kind::Swap ||
-                        fan_centres(op, p.num_qubits) != 0;
-      cost += op.kind == PlanOp::Kind::CCX ? 0.5 : half ? 1.0 : 2.0;
-    }
-  }
-  return cost;
 }
 
 // ---------------------------------------------------------------------------

@@ -104,6 +104,12 @@ std::vector<ForwardStep> fold_diagonals(const Plan &p, std::vector<ForwardStep> 
 // of stages counts 2.7 S for its multiply-adds).
 double schedule_cost(const Plan &p, const std::vector<ForwardStep> &steps);
 
+// qm_run_merged's steps from 14 qubits on: merged_schedule() folded, or
+// inplace_schedule() where that moves less. The second is given up where it
+// cannot be cheaper any more (200 random CX: one gather against dozens of passes,
+// whose search took 45 us of the call's 73).
+std::vector<ForwardStep> run_merged_schedule(const Plan &p);
+
 // The plan for a state that one block holds: one-qubit ops three wires a
 // step, every run of CX / SWAP ops as one gather, other ops as they are.
 std::vector<ForwardStep> small_schedule(const Plan &p);

@@ -1090,10 +1090,7 @@ void Simulator::run_merged(const Plan &p) {
     dispatches_ = own + launched;
     return;
   }
-  std::vector<ForwardStep> steps = fold_diagonals(p, merged_schedule(p));
-  std::vector<ForwardStep> inplace = inplace_schedule(p);
-  if (schedule_cost(p, inplace) < schedule_cost(p, steps)) steps = std::move(inplace);
-  run_steps(p, steps);
+  run_steps(p, run_merged_schedule(p));
 }
 
 void Simulator::run_steps(const Plan &p, const std::vector<ForwardStep> &steps) {

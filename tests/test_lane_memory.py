@@ -14,16 +14,16 @@ OBJ = os.path.join(os.path.dirname(qm.library_path()), "_build")
 CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 
 
-@pytest.fixture(scope="module")
-def client(tmp_path_factory):
+def build_client(name, where):
+    """tests/host_cuda/<name>.cpp with the host's objects and the device that is not there."""
     if shutil.which("g++") is None:
         pytest.skip("no g++")
-    exe = str(tmp_path_factory.mktemp("lanes") / "lanes")
+    exe = str(where / name)
     r = subprocess.run(["gcc", "-w", "-c", os.path.join(HERE, "host_cuda", "fake_kernels.c"), "-o",
                         exe + ".kernels.o"], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-3000:]
     cmd = ["g++", "-std=c++17", "-O1", "-w", "-pthread", "-I" + os.path.join(CUDA, "include")]
-    cmd += [os.path.join(HERE, "host_cuda", f) for f in ("lanes.cpp", "fake_device.cpp")]
+    cmd += [os.path.join(HERE, "host_cuda", f) for f in (name + ".cpp", "fake_device.cpp")]
     cmd += [os.path.join(OBJ, f + ".cpp.o") for f in ("simulator", "batch", "schedule", "plan", "circuit")]
     cmd.append(exe + ".kernels.o")
     r = subprocess.run(cmd + ["-o", exe], capture_output=True, text=True, timeout=300)
@@ -35,6 +35,11 @@ def client(tmp_path_factory):
         return {k: int(v) for k, v in re.findall(r"(\w+) (\d+)", out.stdout)}
 
     return run
+
+
+@pytest.fixture(scope="module")
+def client(tmp_path_factory):
+    return build_client("lanes", tmp_path_factory.mktemp("lanes"))
 
 
 def test_pinned_memory_fails(client):
