@@ -100,6 +100,9 @@ size_t qmk_workspace_bytes(uint32_t n);
 /* Zero the workspace bookkeeping (call once after allocating it). */
 int qmk_workspace_init(void *workspace, size_t bytes, void *stream);
 
+/* The first so many bytes of a workspace hold nothing from one call to the next. */
+size_t qmk_workspace_scratch_bytes(uint32_t n);
+
 /* amplitude i *= exp(i (global_phase + sum of angles[t] over terms whose mask
  * is fully set in i)), one pass. Phase sums are formed in FP64.
  * Replaces apply_diagonal_layer (kernels.metal:203-218; simulator.mm:559-592). */
@@ -177,11 +180,17 @@ uint32_t qmk_small_saves(uint32_t n);
 int qmk_run_small(float *state, uint32_t n, size_t num_ops,
                   const qmk_small_op *ops, const qmk_small_adjoint *adjoint,
                   void *workspace, size_t workspace_bytes, void *stream);
-/* The same; *launches receives the number of kernels launched. */
+/* The same with the phase tables and the kept states apart: `tables` of at least
+ * one table (8 * 2^n bytes) if any op has a layer's terms, which are tabulated as
+ * many at a time as it holds (beyond qmk_small_tables(n) there is no use for
+ * more); `saves` of num_saves states (up to qmk_small_saves(n)), for ops that
+ * name them. Neither holds anything between calls. *launches receives the number
+ * of kernels launched. */
+uint32_t qmk_small_tables(uint32_t n);
 int qmk_run_small_counted(float *state, uint32_t n, size_t num_ops,
                           const qmk_small_op *ops, const qmk_small_adjoint *adjoint,
-                          void *workspace, size_t workspace_bytes, void *stream,
-                          uint32_t *launches);
+                          void *tables, size_t tables_bytes, float *saves,
+                          uint32_t num_saves, void *stream, uint32_t *launches);
 
 /* Stages in one in-place pass, in order, n >= 13. A stage is a 2x2 on its wire
  * (has_matrix) and a fan of controlled phases from it (phase 1: after the 2x2,

@@ -238,6 +238,10 @@ extern "C" size_t qmk_workspace_bytes(uint32_t n) {
   return kDescBytes + kTableBytes + 1024 * 32 * sizeof(double) + 256;
 }
 
+extern "C" size_t qmk_workspace_scratch_bytes(uint32_t n) {
+  return n >= 1 ? qmk_workspace_bytes(n) - 256 : 0;   // all but the counters of the reductions
+}
+
 extern "C" int qmk_workspace_init(void *ws, size_t bytes, void *stream) {
   if (!ws || bytes < qmk_workspace_bytes(0)) return -1;
   cudaError_t e = cudaMemsetAsync(ws, 0, bytes, (cudaStream_t)stream);

@@ -35,9 +35,7 @@ using qmk_host::launch_status;
 namespace {
 
 constexpr uint32_t kMaxN = QMK_SMALL_MAX_QUBITS, kMaxN2 = QMK_SMALL_MAX_ADJOINT;
-// Phase tables per launch and states kept: what fits with the rest of a
-// simulator's workspace in 2 MiB, the device's allocation unit (a second one
-// takes 35 us of a simulator's creation).
+// Most phase tables per launch, and states kept.
 constexpr uint32_t kMaxLayers = 32;
 constexpr uint32_t layers_of(uint32_t n) { return n >= 13 ? 16 : kMaxLayers; }
 constexpr uint32_t saves_of(uint32_t n) { return n > kMaxN2 ? 0 : n >= 12 ? 16 : 32; }
@@ -732,10 +730,18 @@ extern "C" size_t qmk_small_workspace_bytes(uint32_t n) {
 
 extern "C" uint32_t qmk_small_saves(uint32_t n) { return n >= 1 && n <= kMaxN ? saves_of(n) : 0; }
 
-// Checks of one op; two: the ops that need the co-state are allowed.
-static bool small_op_ok(const qmk_small_op &o, uint32_t n, bool two) {
+extern "C" uint32_t qmk_small_tables(uint32_t n) { return n >= 1 && n <= kMaxN ? layers_of(n) : 0; }
+
+static bool needs_table(const qmk_small_op &o) {
+  return o.kind == QMK_SMALL_LAYER || (o.kind == QMK_SMALL_COSTATE && o.layer.num_terms);
+}
+
+// Checks of one op; two: the ops that need the co-state are allowed; room for so
+// many phase tables and kept states.
+static bool small_op_ok(const qmk_small_op &o, uint32_t n, bool two, uint32_t tables,
+                        uint32_t saves) {
   auto layer_ok = [&]() {
-    if (o.layer.num_terms > QMK_SMALL_MAX_TERMS ||
+    if (o.layer.num_terms > QMK_SMALL_MAX_TERMS || (!tables && needs_table(o)) ||
         (o.layer.num_terms && (!o.layer.masks || !o.layer.angles)))
       return false;
     for (uint32_t t = 0; t < o.layer.num_terms; t++)
@@ -754,7 +760,7 @@ static bool small_op_ok(const qmk_small_op &o, uint32_t n, bool two) {
     case QMK_SMALL_CONTROLLED:
       return o.q[0] < n && !(o.mask >> n) && !((o.mask >> o.q[0]) & 1ull) && o.mats;
     case QMK_SMALL_MAP:
-      if (!o.cols || o.save > saves_of(n)) return false;
+      if (!o.cols || o.save > saves) return false;
       for (uint32_t j = 0; j < n; j++)
         if (o.cols[j] >> n) return false;
       return true;
@@ -792,23 +798,30 @@ static bool small_op_ok(const qmk_small_op &o, uint32_t n, bool two) {
 extern "C" int qmk_run_small(float *state, uint32_t n, size_t num_ops, const qmk_small_op *ops,
                              const qmk_small_adjoint *adjoint, void *ws, size_t ws_bytes,
                              void *stream) {
+  if (!ws || n < 1 || n > kMaxN || ws_bytes < qmk_small_workspace_bytes(n)) return -1;
+  const size_t table = sizeof(float2) << n;
   uint32_t launches = 0;
-  return qmk_run_small_counted(state, n, num_ops, ops, adjoint, ws, ws_bytes, stream, &launches);
+  return qmk_run_small_counted(state, n, num_ops, ops, adjoint, ws, table * layers_of(n),
+                               reinterpret_cast<float *>(static_cast<uint8_t *>(ws) +
+                                                         table * layers_of(n)),
+                               saves_of(n), stream, &launches);
 }
 
 extern "C" int qmk_run_small_counted(float *state, uint32_t n, size_t num_ops,
                                      const qmk_small_op *ops, const qmk_small_adjoint *adjoint,
-                                     void *ws, size_t ws_bytes, void *stream,
-                                     uint32_t *launches) {
+                                     void *table_area, size_t table_bytes, float *saves,
+                                     uint32_t num_saves, void *stream, uint32_t *launches) {
   if (!launches) return -1;
   *launches = 0;
-  if (!state || n < 1 || n > kMaxN || (num_ops && !ops) || !ws ||
-      ws_bytes < qmk_small_workspace_bytes(n))
+  if (!state || n < 1 || n > kMaxN || (num_ops && !ops) ||
+      (num_saves && (!saves || num_saves > saves_of(n))))
     return -1;
+  const uint32_t most = static_cast<uint32_t>(std::min<size_t>(
+      layers_of(n), table_area ? table_bytes / (sizeof(float2) << n) : 0));
   if (adjoint && (n > kMaxN2 || !adjoint->costate || !adjoint->grad || !adjoint->energy)) return -1;
   // Everything is checked before anything is launched.
   for (size_t k = 0; k < num_ops; k++) {
-    if (!small_op_ok(ops[k], n, adjoint != nullptr)) return -1;
+    if (!small_op_ok(ops[k], n, adjoint != nullptr, most, num_saves)) return -1;
     if (ops[k].kind == QMK_SMALL_WINDOW)
       for (uint32_t i = 0; i < ops[k].num_items; i++)
         if (ops[k].items[3 * i + 1] && ops[k].items[3 * i + 2] >= adjoint->num_grad) return -1;
@@ -817,11 +830,11 @@ extern "C" int qmk_run_small_counted(float *state, uint32_t n, size_t num_ops,
         if (ops[k].items[2 * i + 1] >= adjoint->num_grad) return -1;
   }
   cudaStream_t s = (cudaStream_t)stream;
-  float2 *tables = static_cast<float2 *>(ws);
+  float2 *tables = static_cast<float2 *>(table_area);
   SmallOut out{};
   if (adjoint)
     out = {reinterpret_cast<float2 *>(adjoint->costate), adjoint->grad, adjoint->energy,
-           tables + (static_cast<size_t>(layers_of(n)) << n)};
+           reinterpret_cast<float2 *>(saves)};
   std::vector<uint32_t> code;
   std::vector<qmk_phase_layer> layers;
   uint32_t terms = 0, real = 0;
@@ -848,7 +861,7 @@ extern "C" int qmk_run_small_counted(float *state, uint32_t n, size_t num_ops,
            !(((real >> l) & 1u) == (is_real ? 1u : 0u) && same_layer(layers[l], layer)))
       l++;
     if (l == layers.size()) {
-      if (l == layers_of(n) || terms + layer.num_terms > static_cast<uint32_t>(kLongTerms)) {
+      if (l == most || terms + layer.num_terms > static_cast<uint32_t>(kLongTerms)) {
         if (const int rc = flush()) return rc;
         l = 0;
       }

@@ -122,7 +122,6 @@ Simulator::Simulator(uint32_t n) : n_(n) {
   cuda_check(cudaGetDevice(&device_), "cudaGetDevice");
   const uint64_t bytes = (uint64_t(1) << n) * 8ull;
   ws_bytes_ = qmk_workspace_bytes(n);
-  small_ws_bytes_ = qmk_small_workspace_bytes(n);   // behind ws_
   size_t free_b = 0, total_b = 0;
   cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
   if (bytes + ws_bytes_ > free_b)
@@ -133,8 +132,7 @@ Simulator::Simulator(uint32_t n) : n_(n) {
   stream_ = s;
   try {
     cuda_check(cudaMalloc(&state_, bytes), "Simulator: state allocation failed");
-    cuda_check(cudaMalloc(&ws_, ws_bytes_ + small_ws_bytes_),
-               "Simulator: workspace allocation failed");
+    cuda_check(cudaMalloc(&ws_, ws_bytes_), "Simulator: workspace allocation failed");
     cuda_check(cudaMalloc(&d_results_, kResultSlots * sizeof(double)), "cudaMalloc results");
     cuda_check(cudaMallocHost(&h_results_, (kResultSlots + 1) * sizeof(double)), "cudaMallocHost");
     h_waits_ = reinterpret_cast<unsigned *>(h_results_ + kResultSlots);
@@ -162,19 +160,26 @@ namespace {
 
 size_t padded(size_t bytes) { return (bytes + 255) & ~size_t(255); }
 
-// The largest workspace for narrow states that a simulator of up to n qubits
-// needs (12 qubits need more than 13, which keep no states).
-size_t small_bytes_up_to(uint32_t n) {
+// Bytes of the phase tables and of the kept states of one-launch programs, for
+// every width up to n.
+size_t tables_up_to(uint32_t n) {
   size_t most = 0;
   for (uint32_t w = 1; w <= std::min<uint32_t>(n, QMK_SMALL_MAX_QUBITS); w++)
-    most = std::max(most, qmk_small_workspace_bytes(w));
+    most = std::max(most, qmk_small_tables(w) * (size_t(8) << w));
+  return most;
+}
+size_t saves_up_to(uint32_t n) {
+  size_t most = 0;
+  for (uint32_t w = 1; w <= std::min<uint32_t>(n, QMK_SMALL_MAX_QUBITS); w++)
+    most = std::max(most, qmk_small_saves(w) * (size_t(8) << w));
   return most;
 }
 
 }  // namespace
 
 size_t Simulator::lane_device_bytes(uint32_t n, size_t max_gates, size_t max_shots) {
-  return 2 * padded((size_t(8) << n)) + padded(qmk_workspace_bytes(n) + small_bytes_up_to(n)) +
+  return 2 * padded((size_t(8) << n)) + padded(qmk_workspace_bytes(n)) +
+         padded(tables_up_to(n)) + padded(saves_up_to(n)) +
          padded(kResultSlots * sizeof(double)) +
          padded(std::max<size_t>(max_gates, 1) * sizeof(double)) +
          (max_shots ? padded(qmk_sample_workspace_bytes(n)) + padded(max_shots * sizeof(uint64_t))
@@ -190,7 +195,6 @@ Simulator::Simulator(uint32_t n, const LaneMemory &m) : n_(n), lane_(m) {
     throw std::runtime_error("Simulator: num_qubits must be 1.." + std::to_string(kMaxQubits));
   cuda_check(cudaGetDevice(&device_), "cudaGetDevice");
   ws_bytes_ = qmk_workspace_bytes(n);
-  small_ws_bytes_ = qmk_small_workspace_bytes(n);
   uint8_t *at = static_cast<uint8_t *>(m.device);
   auto take = [&](size_t bytes) {
     uint8_t *p = at;
@@ -199,7 +203,9 @@ Simulator::Simulator(uint32_t n, const LaneMemory &m) : n_(n), lane_(m) {
   };
   state_ = reinterpret_cast<float *>(take(size_t(8) << n));
   costate_ = reinterpret_cast<float *>(take(size_t(8) << n));
-  ws_ = take(ws_bytes_ + small_bytes_up_to(n));
+  ws_ = take(ws_bytes_);
+  tables_ = take(tables_up_to(n));
+  saves_ = reinterpret_cast<float *>(take(saves_up_to(n)));
   d_results_ = reinterpret_cast<double *>(take(kResultSlots * sizeof(double)));
   d_grad_cap_ = std::max<size_t>(m.max_gates, 1);
   d_grad_ = reinterpret_cast<double *>(take(d_grad_cap_ * sizeof(double)));
@@ -232,7 +238,6 @@ void Simulator::narrow_to(uint32_t n) {
   if (n == 0 || n > n_) throw std::runtime_error("Simulator: wider than its memory");
   if (n < n_) scratch_failed_ = false;
   n_ = n;
-  small_ws_bytes_ = qmk_small_workspace_bytes(n);
   invalidate_graphs();
 }
 
@@ -257,6 +262,8 @@ void Simulator::release() {
   for (float *b : ck_free_) free_device(b);
   ck_free_.clear();
   free_device(ws_);
+  free_device(tables_);
+  free_device(saves_);
   free_device(sample_ws_);
   free_device(d_shots_);
   free_device(d_results_);
@@ -270,7 +277,8 @@ void Simulator::release() {
   if (ev_stop_) cudaEventDestroy(static_cast<cudaEvent_t>(ev_stop_));
   if (stream_) cudaStreamDestroy(S(stream_));
   state_ = costate_ = nullptr;
-  ws_ = sample_ws_ = nullptr;
+  ws_ = sample_ws_ = tables_ = nullptr;
+  saves_ = nullptr;
   d_shots_ = nullptr;
   d_results_ = h_results_ = d_grad_ = nullptr;
   h_waits_ = nullptr;
@@ -795,16 +803,67 @@ class SmallProgram {
 
 }  // namespace
 
-// Returns the number of kernels launched.
+namespace {
+
+// Are there more than `most` different phase layers among the ops?
+bool more_layers(const std::vector<qmk_small_op> &ops, size_t most) {
+  std::vector<const qmk_small_op *> layers, seen;
+  for (const qmk_small_op &o : ops)
+    if (o.kind == QMK_SMALL_LAYER || (o.kind == QMK_SMALL_COSTATE && o.layer.num_terms))
+      layers.push_back(&o);
+  if (layers.size() <= most) return false;
+  for (const qmk_small_op *o : layers) {
+    const qmk_phase_layer &a = o->layer;
+    bool again = false;
+    for (const qmk_small_op *s : seen) {
+      const qmk_phase_layer &b = s->layer;
+      again = again || (s->kind == o->kind && a.num_terms == b.num_terms &&
+                        a.global_phase == b.global_phase &&
+                        std::equal(a.angles, a.angles + a.num_terms, b.angles) &&
+                        std::equal(a.masks, a.masks + a.num_terms, b.masks));
+    }
+    if (again) continue;
+    seen.push_back(o);
+    if (seen.size() > most) return true;
+  }
+  return false;
+}
+
+}  // namespace
+
+// The phase tables lie in the workspace, where 5 of 13 qubits fit, 10 of 12 and so
+// on. A circuit of more layers has them tabulated in several goes; from the second
+// one on it takes memory for as many as a launch can have (13 qubits: 10 us a go
+// against 130 us once. A simulator that held it from the start took 117 us to
+// create at 11 and 12 qubits, 42 without: its allocations needed a second 2 MiB of
+// the device). Returns the number of kernels launched.
 uint64_t Simulator::launch_program(const std::vector<qmk_small_op> &ops,
                                    const qmk_small_adjoint *adj) {
   if (ops.empty()) return 0;
+  const size_t table = size_t(8) << n_, room = qmk_workspace_scratch_bytes(n_);
+  if (!tables_ && !capturing_ && more_layers(ops, room / table)) {
+    if (many_layers_ && cudaMalloc(&tables_, qmk_small_tables(n_) * table) != cudaSuccess) {
+      cudaGetLastError();
+      tables_ = nullptr;
+    }
+    many_layers_ = true;
+  }
   uint32_t launches = 0;
-  check(qmk_run_small_counted(state_, n_, ops.size(), ops.data(), adj,
-                              static_cast<uint8_t *>(ws_) + ws_bytes_, small_ws_bytes_, stream_,
-                              &launches),
+  check(qmk_run_small_counted(state_, n_, ops.size(), ops.data(), adj, tables_ ? tables_ : ws_,
+                              tables_ ? qmk_small_tables(n_) * table : room, saves_,
+                              saves_ ? qmk_small_saves(n_) : 0, stream_, &launches),
         "circuit");
   return launches;
+}
+
+// Memory for the states that a narrow gradient keeps.
+bool Simulator::ensure_saves() {
+  const size_t bytes = qmk_small_saves(n_) * (size_t(8) << n_);
+  if (!saves_ && bytes && !capturing_ && cudaMalloc(&saves_, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    saves_ = nullptr;
+  }
+  return saves_ != nullptr;
 }
 
 namespace {
@@ -926,7 +985,8 @@ bool Simulator::small_gradient(const Circuit &c, const Hamiltonian &h, const Pla
     pair = undone_by(plan, *kept[kept.size() - 1 - i], undone[i]->gates);
 
   // The last maps' states are kept, as many as there is room for.
-  const size_t room = pair ? std::min<size_t>(kept.size(), qmk_small_saves(n_)) : 0;
+  const size_t room = pair && !kept.empty() && ensure_saves()
+                          ? std::min<size_t>(kept.size(), qmk_small_saves(n_)) : 0;
   size_t ahead = kept.size();   // maps of the forward pass still to come
   SmallProgram prog(n_);
   for (const ForwardStep &st : fwd) {
@@ -1044,9 +1104,12 @@ void Simulator::run_cached(const Circuit &c) {
   const uint64_t before = dispatches_;
   cuda_check(cudaStreamBeginCapture(S(stream_), cudaStreamCaptureModeThreadLocal), "graph capture");
   cudaGraph_t graph = nullptr;
+  capturing_ = true;
   try {
     run_inplace(plan, true);
+    capturing_ = false;
   } catch (...) {
+    capturing_ = false;
     cudaStreamEndCapture(S(stream_), &graph);
     if (graph) cudaGraphDestroy(graph);
     dispatches_ = before;
@@ -1857,6 +1920,7 @@ void Simulator::reserve(size_t max_gates, size_t max_shots) {
     d_shots_cap_ = max_shots;
   }
   ensure_scratch();
+  ensure_saves();
 }
 
 void Simulator::serve_enqueue(const Circuit &c, const Hamiltonian &h, size_t shots, uint64_t seed,
@@ -1868,6 +1932,11 @@ void Simulator::serve_enqueue(const Circuit &c, const Hamiltonian &h, size_t sho
   prepare_adjoint(c, h);
   reset();
   const Plan plan = build_plan(c, FusionOptions{});
+  struct Capturing {   // (the caller's graph records what follows)
+    bool &flag;
+    explicit Capturing(bool &f) : flag(f) { flag = true; }
+    ~Capturing() { flag = false; }
+  } capturing(capturing_);
   if (n_ > kSmallGradient || !small_gradient(c, h, plan, shots, seed)) {
     run_steps(plan, fold_diagonals(plan, merged_schedule(plan)));
     if (shots) launch_sample(shots, seed);

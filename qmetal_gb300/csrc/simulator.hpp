@@ -151,7 +151,8 @@ class Simulator {
   void fused_gradient(const Circuit &c, const Hamiltonian &h, size_t shots, uint64_t seed);
   uint64_t launch_program(const std::vector<qmk_small_op> &ops, const qmk_small_adjoint *adj);
   // The state fits one block: circuits run in one launch.
-  bool small() const { return small_ws_bytes_ != 0; }
+  bool small() const { return n_ <= QMK_SMALL_MAX_QUBITS; }
+  bool ensure_saves();
   void pauli_values(const float *state, const Hamiltonian &h, std::vector<double> &vals);
   void costate(const Hamiltonian &h);
   void prepare_adjoint(const Circuit &c, const Hamiltonian &h);
@@ -200,7 +201,11 @@ class Simulator {
   bool scratch_failed_ = false;
   void *ws_ = nullptr;
   size_t ws_bytes_ = 0;
-  size_t small_ws_bytes_ = 0;           // behind ws_bytes_ in ws_ (0: the state is too wide)
+  void *tables_ = nullptr;              // one-launch programs: phase tables that ws_ has no room
+                                        // for, and kept states
+  bool many_layers_ = false;            // a program had more of them than that
+  float *saves_ = nullptr;
+  bool capturing_ = false;              // a graph is being recorded: nothing may be allocated
   void *sample_ws_ = nullptr;
   size_t sample_ws_bytes_ = 0;
   uint64_t *d_shots_ = nullptr;

@@ -12,6 +12,8 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <utility>
+#include <vector>
 
 namespace fake {
 
@@ -110,28 +112,44 @@ cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess;
 // The kernel layer, but for the calls of fake_kernels.c.
 size_t qmk_workspace_bytes(uint32_t) { return 1u << 20; }
 size_t qmk_sample_workspace_bytes(uint32_t) { return 1u << 20; }
-uint32_t qmk_small_saves(uint32_t) { return 0; }
-// Not growing with the width, as the real one.
-size_t qmk_small_workspace_bytes(uint32_t n) { return n > 13 ? 0 : n == 12 ? 3u << 19 : 1u << 20; }
+size_t qmk_workspace_scratch_bytes(uint32_t) { return 1u << 18; }
+// Neither grows with the width, as the real ones.
+uint32_t qmk_small_saves(uint32_t n) { return n > 12 ? 0 : n == 12 ? 16 : 32; }
+uint32_t qmk_small_tables(uint32_t n) { return n > 13 ? 0 : n == 13 ? 4 : 32; }
 int qmk_apply_permutation(float *, const float *, uint32_t n, const uint64_t *, uint64_t, void *) {
   std::lock_guard<std::mutex> g(lock);
   permutations[n]++;
   return 0;
 }
 unsigned int *qmk_wait_counter(void *ws) { return static_cast<unsigned int *>(ws); }
-int qmk_run_small_counted(float *, uint32_t n, size_t, const qmk_small_op *,
-                          const qmk_small_adjoint *adj, void *ws, size_t bytes, void *,
-                          uint32_t *launches) {
+int qmk_run_small_counted(float *state, uint32_t n, size_t, const qmk_small_op *,
+                          const qmk_small_adjoint *adj, void *tables, size_t bytes, float *saves,
+                          uint32_t num_saves, void *, uint32_t *launches) {
   std::lock_guard<std::mutex> g(lock);
   small_runs++;
   *launches = 1;
-  const char *from = static_cast<char *>(ws), *to = from + bytes;
-  const auto in = [&](const void *p, size_t size) {
-    const char *b = static_cast<const char *>(p);
-    return b < to && b + size > from;
+  const size_t amps = size_t(8) << n;
+  std::vector<std::pair<const char *, size_t>> held;
+  auto hold = [&](const void *p, size_t size) {
+    if (p && size) held.push_back({static_cast<const char *>(p), size});
   };
-  if (adj && (in(adj->costate, size_t(8) << n) || in(adj->grad, 8 * adj->num_grad) || in(adj->energy, 8)))
-    overlaps++;
+  hold(state, amps);
+  hold(tables, bytes);
+  hold(saves, num_saves * amps);
+  if (adj) {
+    hold(adj->costate, amps);
+    hold(adj->grad, 8 * adj->num_grad);
+    hold(adj->energy, 8);
+  }
+  for (size_t i = 0; i < held.size(); i++)
+    for (size_t j = 0; j < i; j++)
+      if (held[i].first < held[j].first + held[j].second &&
+          held[j].first < held[i].first + held[i].second)
+        overlaps++;
+  for (const auto &h : held) {   // inside one allocation
+    auto it = blocks.upper_bound(const_cast<char *>(h.first));
+    if (it == blocks.begin() || (--it)->first + it->second < h.first + h.second) overlaps++;
+  }
   return 0;
 }
 }  // extern "C"

@@ -24,21 +24,39 @@ Circuit ladders(uint32_t n) {
 
 int main(int argc, char **argv) {
   const char *what = argc > 1 ? argv[1] : "";
-  const Circuit wide = ladders(20), narrow = ladders(std::strcmp(what, "narrow") ? 16 : 12);
+  auto mode = [&](const char *m) { return std::strcmp(what, m) == 0; };
+  if (mode("create")) {   // device memory of a simulator of 12 qubits, and after a run and a gradient
+    Simulator sim(12);
+    const size_t made = fake::used;
+    const Circuit c = ladders(12);
+    Hamiltonian h;
+    h.add(1.0, PauliString::single('Z', 0));
+    sim.run(c);
+    const size_t ran = fake::used;
+    sim.energy_and_gradient(c, h);
+    std::printf("made %zu ran %zu gradient %zu small %d overlaps %d\n", made, ran, fake::used,
+                fake::small_runs, fake::overlaps);
+    return 0;
+  }
+  std::vector<uint32_t> widths = {20, 16};
+  if (mode("narrow")) widths = {20, 13, 12, 12, 11, 6, 1};
+  std::vector<Circuit> circuits;
+  for (uint32_t n : widths) circuits.push_back(ladders(n));
   Hamiltonian h;
   h.add(1.0, PauliString::single('Z', 0));
-  std::vector<double> g0(wide.size()), g1(narrow.size());
-  std::vector<BatchItem> items(2);
-  items[0].circuit = &wide;
-  items[0].grad = g0.data();
-  items[1].circuit = &narrow;
-  items[1].grad = g1.data();
-  for (BatchItem &it : items) it.hamiltonian = &h;
-  if (!std::strcmp(what, "pinned")) fake::fail_pinned = 1;
+  std::vector<std::vector<double>> grads;
+  std::vector<BatchItem> items(widths.size());
+  for (const Circuit &c : circuits) grads.emplace_back(c.size());
+  for (size_t k = 0; k < items.size(); k++) {
+    items[k].circuit = &circuits[k];
+    items[k].hamiltonian = &h;
+    items[k].grad = grads[k].data();
+  }
+  if (mode("pinned")) fake::fail_pinned = 1;
   // The lane's memory, 2 GiB of headroom, and room for a second buffer of 16
   // qubits (512 KiB) but not of 20 (8 MiB).
-  if (!std::strcmp(what, "scratch"))
-    fake::total = Simulator::lane_device_bytes(20, wide.size(), 0) + (size_t(2) << 30) + (4u << 20);
+  if (mode("scratch"))
+    fake::total = Simulator::lane_device_bytes(20, circuits[0].size(), 0) + (size_t(2) << 30) + (4u << 20);
   run_batch(items, BatchMode::Lanes, 1);
   std::printf("wide %d narrow %d held %zu left %zu small %d overlaps %d\n",
               fake::permutations[20], fake::permutations[16], fake::used_after_failed_pinned,

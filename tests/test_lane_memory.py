@@ -59,7 +59,18 @@ def test_no_second_buffer_for_the_widest(client):
 
 
 def test_memory_of_a_narrow_request(client):
-    """A lane's one-launch workspace lies beside the rest of its memory at each width."""
+    """A lane's phase tables and kept states lie beside the rest of its memory at each width."""
     got = client("narrow")
-    assert got["small"] > 0 and got["overlaps"] == 0
+    assert got["small"] > 4 and got["overlaps"] == 0
     assert got["left"] == 0
+
+
+def test_memory_of_a_simulator(client):
+    """A narrow simulator holds its state, workspace and results, and what a gradient
+    keeps from the first one on."""
+    got = client("create")
+    fixed = (8 << 12) + (1 << 20) + 8 * 4096
+    assert got["made"] <= fixed and got["ran"] == got["made"]
+    # the co-state, sixteen kept states and the gradient of 69 gates
+    assert got["gradient"] <= fixed + 17 * (8 << 12) + 8 * 69
+    assert got["small"] >= 2 and got["overlaps"] == 0
