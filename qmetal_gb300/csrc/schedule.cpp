@@ -237,6 +237,7 @@ std::vector<ForwardStep> merged_schedule(const Plan &p) {
   std::vector<ForwardStep> out;
   WireRun held;
   auto flush = [&]() {
+    if (held.wires.empty()) return;
     for (const auto &pass : split_run(n, held)) out.push_back(group_step(held, pass));
     held.clear();
   };
@@ -574,10 +575,39 @@ std::vector<ForwardStep> inplace_schedule(const Plan &p) {
   return fold_diagonals(p, std::move(out));
 }
 
+size_t plan_runs(const Plan &p, size_t most) {
+  enum { None, Single, Move } last = None;
+  size_t runs = 0;
+  for (const PlanOp &op : p.ops) {
+    if (runs > most) break;
+    if (is_wire_move(op, p.num_qubits)) {
+      runs += last == None;
+      last = Move;
+    } else if (op.kind == PlanOp::Kind::Dense1q || op.kind == PlanOp::Kind::Dense1qGroup) {
+      runs += last != Single;
+      last = Single;
+    } else {
+      runs++;
+      last = None;
+    }
+  }
+  return runs;
+}
+
 std::vector<ForwardStep> run_merged_schedule(const Plan &p) {
   std::vector<ForwardStep> steps = fold_diagonals(p, merged_schedule(p));
   if (!inplace_differs(p)) return steps;
   const double cost = schedule_cost(p, steps);
+  // One run of single gates and moves goes in passes of up to seven wires >= 6.
+  if (plan_runs(p, 1) == 1) {
+    uint64_t wires = 0;
+    for (const PlanOp &op : p.ops) {
+      if (is_wire_move(op, p.num_qubits)) wires |= (1ull << op.qubits[0]) | (1ull << op.qubits[1]);
+      else if (op.kind == PlanOp::Kind::Dense1q) wires |= 1ull << op.qubits[0];
+      else for (uint32_t w : op.group_qubits) wires |= 1ull << w;
+    }
+    if (2.0 * std::max(1u, (popc(wires >> 6) + 6) / 7) >= cost) return steps;
+  }
   double folds = 0.0;   // what the folding of layers may still save
   for (const PlanOp &op : p.ops) folds += op.kind == PlanOp::Kind::DiagonalLayer ? 4.0 : 0.0;
   std::vector<ForwardStep> inplace;

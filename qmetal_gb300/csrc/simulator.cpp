@@ -30,7 +30,7 @@ constexpr uint32_t kTermsPerPass = 16;
 constexpr uint32_t kSmallExpect = 14;    // widest state whose strings go a block each
 constexpr size_t kSmallTerms = 64;       // strings per such launch
 constexpr size_t kZTermsPerPass = 32;
-constexpr size_t kFewSmallSteps = 5;     // three launches of 13 wires in the one-launch steps
+constexpr size_t kFewRuns = 2;           // of a plan that may be few launches merged
 constexpr uint32_t kSmallGradient = QMK_SMALL_MAX_ADJOINT;   // widest gradient in one block
 
 cudaStream_t S(void *p) { return static_cast<cudaStream_t>(p); }
@@ -1137,8 +1137,7 @@ void Simulator::run_merged(const Plan &p) {
   if (p.num_qubits != n_) throw std::runtime_error("plan/simulator size mismatch");
   activate();
   if (small()) {
-    const std::vector<ForwardStep> steps = small_schedule(p);
-    if (steps.size() <= kFewSmallSteps) {   // (which may be passes of more wires, or one gather)
+    if (plan_runs(p, kFewRuns) <= kFewRuns) {   // (which may be a pass and a gather)
       const std::vector<ForwardStep> merged = merged_schedule(p);
       size_t launches = 0;
       for (const ForwardStep &st : merged)
@@ -1149,7 +1148,7 @@ void Simulator::run_merged(const Plan &p) {
       }
     }
     const uint64_t own = dispatches_;
-    const uint64_t launched = run_small(p, steps);
+    const uint64_t launched = run_small(p, small_schedule(p));
     dispatches_ = own + launched;
     return;
   }
