@@ -1,7 +1,7 @@
 // kreduce.cuh -- the deterministic device-wide reduction used by every
 // kernel that returns numbers (norms, expectations, energies, gradients).
 //
-// Each block reduces its FP64 accumulators (warp shuffles, then shared
+// Each block reduces its accumulators, FP64 or FP32 pairs (warp shuffles, then shared
 // memory) into per-block partials in the workspace; the last block to finish
 // (atomic ticket) sums the partials in a fixed order and hands each total to
 // an output functor. A result depends only on the grid size, never on timing.
