@@ -575,6 +575,10 @@ std::vector<ForwardStep> inplace_schedule(const Plan &p) {
   return fold_diagonals(p, std::move(out));
 }
 
+namespace {
+
+// The runs that a plan falls into, each of single gates and then CX / SWAP moves,
+// or one other op; counted as far as most + 1.
 size_t plan_runs(const Plan &p, size_t most) {
   enum { None, Single, Move } last = None;
   size_t runs = 0;
@@ -593,6 +597,8 @@ size_t plan_runs(const Plan &p, size_t most) {
   }
   return runs;
 }
+
+}  // namespace
 
 std::vector<ForwardStep> run_merged_schedule(const Plan &p) {
   std::vector<ForwardStep> steps = fold_diagonals(p, merged_schedule(p));

@@ -104,10 +104,6 @@ std::vector<ForwardStep> fold_diagonals(const Plan &p, std::vector<ForwardStep> 
 // of stages counts 2.7 S for its multiply-adds).
 double schedule_cost(const Plan &p, const std::vector<ForwardStep> &steps);
 
-// The runs that a plan falls into, each of single gates and then CX / SWAP moves,
-// or one other op; counted as far as most + 1.
-size_t plan_runs(const Plan &p, size_t most);
-
 // qm_run_merged's steps from 14 qubits on: merged_schedule() folded, or
 // inplace_schedule() where that moves less. The second is given up where it
 // cannot be cheaper any more (200 random CX: one gather against dozens of passes,

@@ -30,7 +30,6 @@ constexpr uint32_t kTermsPerPass = 16;
 constexpr uint32_t kSmallExpect = 14;    // widest state whose strings go a block each
 constexpr size_t kSmallTerms = 64;       // strings per such launch
 constexpr size_t kZTermsPerPass = 32;
-constexpr size_t kFewRuns = 2;           // of a plan that may be few launches merged
 constexpr uint32_t kSmallGradient = QMK_SMALL_MAX_ADJOINT;   // widest gradient in one block
 
 cudaStream_t S(void *p) { return static_cast<cudaStream_t>(p); }
@@ -876,6 +875,26 @@ size_t launches_alone(const PlanOp &op) {
              ? 4 : 1;
 }
 
+// The fewest launches that the merged plan can be, counted as far as most + 1: a
+// pass for single gates that follow each other, one for moves.
+size_t merged_least(const Plan &p, size_t most) {
+  enum { None, Single, Move } last = None;
+  size_t least = 0;
+  for (const PlanOp &op : p.ops) {
+    if (least > most) break;
+    const bool single = op.kind == PlanOp::Kind::Dense1q || op.kind == PlanOp::Kind::Dense1qGroup;
+    const bool move = op.kind == PlanOp::Kind::Swap || op.kind == PlanOp::Kind::Controlled1q;
+    if (single || move) {
+      least += last != (single ? Single : Move);
+      last = single ? Single : Move;
+    } else {
+      least += launches_alone(op);
+      last = None;
+    }
+  }
+  return least;
+}
+
 // As many launches as are no slower than the one launch of k_small, whose
 // block loads and stores the state and takes its ops from shared memory: us by
 // launches and in one, 1 to 4 ops of a gate each: 8 qubits 9.8, 12.6, 15.5, 18.6
@@ -1137,7 +1156,7 @@ void Simulator::run_merged(const Plan &p) {
   if (p.num_qubits != n_) throw std::runtime_error("plan/simulator size mismatch");
   activate();
   if (small()) {
-    if (plan_runs(p, kFewRuns) <= kFewRuns) {   // (which may be a pass and a gather)
+    if (merged_least(p, few_launches(n_)) <= few_launches(n_)) {
       const std::vector<ForwardStep> merged = merged_schedule(p);
       size_t launches = 0;
       for (const ForwardStep &st : merged)
